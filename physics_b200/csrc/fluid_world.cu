@@ -410,10 +410,10 @@ SphParams SphParams::from_c(const PhySphParams& c) {
 FluidWorld::FluidWorld(const SphParams& p, Precision prec) : params(p), prec_(prec), h0_(p.h) {
   cuda_check(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
   stream_ = own_stream_;
-  dalloc(b_.flags, 1);
+  dalloc(b_.flags, kStepWords);
+  b_.order_count = b_.flags + 2;
   dalloc(b_.counters, 2);
-  dalloc(b_.order_count, 1);
-  cuda_check(cudaMemsetAsync(b_.flags, 0, sizeof(uint32_t), stream_), "memset");
+  cuda_check(cudaMemsetAsync(b_.flags, 0, kStepWords * sizeof(uint32_t), stream_), "memset");
   cuda_check(cudaMemsetAsync(b_.counters, 0, 2 * sizeof(unsigned long long), stream_), "memset");
 }
 
@@ -457,6 +457,8 @@ void FluidWorld::free_all() {
   }
   dfree(b_.mu);
   dfree(b_.cpos);
+  dfree(b_.rec);
+  dfree(b_.search);
   dfree(b_.cvel);
   dfree(b_.cmr);
   dfree(b_.nbr);
@@ -492,7 +494,7 @@ void FluidWorld::free_all() {
   dfree(b_.stage);
   dfree(b_.flags);
   dfree(b_.counters);
-  dfree(b_.order_count);
+  b_.order_count = nullptr;
 }
 
 void FluidWorld::set_stream(cudaStream_t s) {
@@ -541,6 +543,9 @@ void FluidWorld::ensure_capacity(size_t n) {
   }
   dgrow(b_.nbr_count, 0, cap, s);
   dfree(b_.nbr);
+  dfree(b_.rec);
+  dfree(b_.search);
+  if (prec_ == Precision::F64Plain) dfree(b_.cpos);
   dfree(b_.nbr16);
   dfree(b_.sorted_cell);
   dfree(b_.tile_of);
@@ -568,11 +573,17 @@ void FluidWorld::ensure_mode_buffers() {
   if (cap == 0) return;
   const bool tiled = prec_ == Precision::F32Comp && comp_tile_ > 0;
   if (!tiled && !b_.nbr) dalloc(b_.nbr, (size_t)kMaxNeighbors * cap);
+  if (prec_ == Precision::F64Plain) {
+    if (!b_.rec) dalloc(b_.rec, (size_t)kPlainRec * cap);
+    if (!b_.cpos) dalloc(b_.cpos, cap);
+    if (!b_.sorted_cell) dalloc(b_.sorted_cell, cap);
+    if (!b_.search) dalloc(b_.search, (cap + 31) / 32 * (size_t)kSearchRecord);
+  }
   if (tiled) {
     if (!b_.nbr16) dalloc(b_.nbr16, (size_t)kMaxNeighbors * cap);
     if (!b_.sorted_cell) dalloc(b_.sorted_cell, cap);
     if (!b_.tile_of) dalloc(b_.tile_of, cap + 1);
-    if (!b_.large_cells) dalloc(b_.large_cells, cap / 64 + 64);  // cells of more than 64 particles
+    if (!b_.large_cells) dalloc(b_.large_cells, cap / 16 + 64);  // cells of more than 16 particles
     if (!b_.tile_slot) dalloc(b_.tile_slot, cap + 1);
     if (!b_.tile_crowd) dalloc(b_.tile_crowd, cap + 1);
     if (!b_.num_tiles) dalloc(b_.num_tiles, 1);
@@ -787,7 +798,8 @@ void FluidWorld::ensure_cells() {
     ++alloc_gen_;
   }
   // The scan's tile sums serve the cell scan and the tile scan alike.
-  const int sums = (int)std::max(scan_block_sums_needed(b_.cell_capacity), tile_scan_sums_needed(b_.cell_capacity));
+  const int sums =
+      (int)std::max(2 * scan_block_sums_needed(b_.cell_capacity), tile_scan_sums_needed(b_.cell_capacity));
   if (sums > b_.block_sums_capacity) {
     cuda_check(cudaStreamSynchronize(stream_), "sums sync");
     dalloc(b_.block_sums, (size_t)sums);
@@ -839,6 +851,7 @@ StepConsts FluidWorld::make_consts(double dt) const {
   c.ncz = nc_[2];
   c.ncells = ncells_;
   c.tile = tile_;
+  c.plain = prec_ == Precision::F64Plain ? 1 : 0;
   c.tile_log2 = tile_ == 4 ? 2 : (tile_ == 2 ? 1 : 0);
   c.halo_cap = halo_cap_;
   c.dense_mean = dense_mean_;
@@ -1218,7 +1231,7 @@ void FluidWorld::ensure_masks() {
 
 // The device work of one step on the world's stream.
 void FluidWorld::enqueue_step(const StepConsts& c, const PassEvents& pe, const cudaEvent_t* ev) {
-  cuda_check(cudaMemsetAsync(b_.flags, 0, sizeof(uint32_t), stream_), "flags reset");
+  cuda_check(cudaMemsetAsync(b_.flags, 0, kStepWords * sizeof(uint32_t), stream_), "flags reset");
   if (counting_) cuda_check(cudaMemsetAsync(b_.counters, 0, 2 * sizeof(unsigned long long), stream_), "memset");
   unsigned long long* saved = b_.counters;
   if (!counting_) b_.counters = nullptr;
@@ -1828,6 +1841,7 @@ void FluidWorld::couple_bodies(PhyCoupleBody* bodies, uint32_t nb, const double*
 int FluidSubsystem::validate() {
   if (world->is_empty()) return 0;
   uint32_t f = world->last_step_flags();
+  if (f & kFlagSortLost) return -1;
   if (f & kFlagNonFinite) return 2;
   if (f & kFlagOutOfBox) return 5;
   return 0;

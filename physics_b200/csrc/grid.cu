@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "sph_buffers.h"
 
@@ -24,6 +25,23 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kThreads * kScanItems;  // 4096 cells per scan block
+
+// Particles and buckets below which the sort is one cooperative launch.  The
+// separate kernels take ~40 us up to 100,000 particles (launches), the fused
+// one 22 us at 343, 21 us at 4,275, 32 us at 65,536 and 46 us at 111,777 (its
+// grid of resident blocks moves less at once); tiled, 30 against 41 us at
+// 8,303 and 66 against 59 us at 379,603.
+constexpr int kFusedBelow = 80000;
+constexpr int kFusedBuckets = 1 << 22;
+
+// Cells up to kOrderSmall particles are ordered by counting the smaller keys;
+// larger ones, up to kOrderLarge, in shared memory by a block of kOrderThreads.
+constexpr uint32_t kOrderSmall = 64;
+constexpr uint32_t kOrderLarge = 4096;
+constexpr int kOrderThreads = 512;
+// Tiles too crowded for shared memory leave cells above this to the blocks of
+// order_large (counting 60 keys through global memory took 60 us).
+constexpr uint32_t kOrderTile = 16;
 
 int grid_for(int n, int threads = kThreads) {
   int b = (n + threads - 1) / threads;
@@ -50,21 +68,33 @@ __device__ __forceinline__ uint32_t quantise_local(double x, long long k, double
 
 // Cell of every particle plus its arrival rank inside its bucket: the cell
 // (bucket_shift 0), or the tile of 2^bucket_shift consecutive cells (the
-// overflow cell's bucket follows the last tile's).  Lanes of a warp that
-// share a bucket (the common case: the previous order is already sorted by
-// cell) are aggregated into one atomic.
-__global__ void __launch_bounds__(kThreads) k_cell_hist(StepConsts c, int bucket_shift,
-                                                        const double* __restrict__ px,
-                                                        const double* __restrict__ py,
-                                                        const double* __restrict__ pz,
-                                                        uint32_t* __restrict__ cell_of,
-                                                        uint32_t* __restrict__ rank,
-                                                        uint32_t* __restrict__ count,
-                                                        uint32_t* __restrict__ flags,
-                                                        const uint16_t* __restrict__ scene,
-                                                        const uint32_t* __restrict__ id,
-                                                        unsigned long long* __restrict__ okey) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// overflow cell's bucket follows the last tile's).  Every thread of the block
+// calls it.
+struct HistArgs {
+  int bucket_shift;
+  const double* __restrict__ px;
+  const double* __restrict__ py;
+  const double* __restrict__ pz;
+  uint32_t* __restrict__ cell_of;
+  uint32_t* __restrict__ rank;
+  uint32_t* __restrict__ count;
+  uint32_t* __restrict__ flags;
+  const uint16_t* __restrict__ scene;
+  const uint32_t* __restrict__ id;
+  unsigned long long* __restrict__ okey;
+  // Fused x-major sort (nullable): per scan tile the particles, and a word set
+  // when a bucket below `buckets` passes kOrderSmall.
+  uint2* sums;
+  uint32_t buckets;
+  uint32_t* crowded;
+};
+__device__ __forceinline__ void cell_hist(const StepConsts& c, const HistArgs& h, int i) {
+  const double *px = h.px, *py = h.py, *pz = h.pz;
+  uint32_t *cell_of = h.cell_of, *rank = h.rank, *count = h.count, *flags = h.flags;
+  const uint16_t* scene = h.scene;
+  const uint32_t* id = h.id;
+  unsigned long long* okey = h.okey;
+  const int bucket_shift = h.bucket_shift;
   bool active = i < c.n;
   uint32_t cell = 0;
   if (active) {
@@ -97,22 +127,51 @@ __global__ void __launch_bounds__(kThreads) k_cell_hist(StepConsts c, int bucket
       okey[i] = ((unsigned long long)m << 32) | id[i];
     }
   }
-  unsigned mask = __ballot_sync(0xffffffffu, active);
-  if (!active) return;
-  const uint32_t bucket = cell >> bucket_shift;
-  unsigned peers = __match_any_sync(mask, bucket);
-  int lane = threadIdx.x & 31;
-  int leader = __ffs(peers) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(&count[bucket], (uint32_t)__popc(peers));
-  base = __shfl_sync(peers, base, leader);
-  rank[i] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  // Runs of consecutive particles of one bucket inside the block (the previous
+  // order is nearly sorted by cell, so a crowded bucket is a few long runs)
+  // take one atomic each: counters of crowded buckets are contended.
+  __shared__ uint32_t s_bucket[kThreads + 1], s_base[kThreads];
+  __shared__ int s_last[kThreads / 32], s_first[kThreads / 32];
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)blockDim.x >> 5;
+  const uint32_t bucket = active ? cell >> bucket_shift : 0xffffffffu;
+  __syncthreads();  // a previous call's arrays are free
+  s_bucket[tid + 1] = bucket;
+  if (tid == 0) s_bucket[0] = ~bucket;
+  __syncthreads();
+  const unsigned heads = __ballot_sync(0xffffffffu, s_bucket[tid] != bucket);
+  if (lane == 0) {
+    s_last[warp] = heads ? warp * 32 + 31 - __clz(heads) : -1;
+    s_first[warp] = heads ? warp * 32 + __ffs(heads) - 1 : -1;
+  }
+  __syncthreads();
+  const unsigned below = heads & (0xffffffffu >> (31 - lane));
+  int head = below ? warp * 32 + 31 - __clz(below) : -1;
+  for (int w = warp - 1; head < 0; --w) head = s_last[w];  // thread 0 is a head
+  if (active && head == tid) {
+    const unsigned above = lane < 31 ? heads >> (lane + 1) : 0u;
+    int end = above ? tid + __ffs(above) : -1;
+    for (int w = warp + 1; end < 0 && w < nw; ++w) end = s_first[w];
+    if (end < 0) end = (int)blockDim.x;
+    const uint32_t count_run = (uint32_t)(end - tid);
+    const uint32_t base = atomicAdd(&count[bucket], count_run);
+    s_base[tid] = base;
+    if (h.sums) {
+      uint2* sum = h.sums + bucket / (uint32_t)kScanTile;
+      atomicAdd(&sum->x, count_run);
+      if (base + count_run > kOrderSmall && bucket < h.buckets) *h.crowded = 1u;
+    }
+  }
+  __syncthreads();
+  if (active) rank[i] = s_base[head] + (uint32_t)(tid - head);
+}
+__global__ void __launch_bounds__(kThreads) k_cell_hist(StepConsts c, HistArgs h) {
+  cell_hist(c, h, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Sum of each 4096-cell tile.
-__global__ void __launch_bounds__(kThreads) k_scan_reduce(const uint32_t* __restrict__ v,
-                                                          uint32_t* __restrict__ block_sums) {
-  const uint4* t = reinterpret_cast<const uint4*>(v + (size_t)blockIdx.x * kScanTile) + threadIdx.x * 4;
+__device__ __forceinline__ void scan_reduce(const uint32_t* __restrict__ v, uint32_t* __restrict__ block_sums,
+                                            uint32_t blk) {
+  const uint4* t = reinterpret_cast<const uint4*>(v + (size_t)blk * kScanTile) + threadIdx.x * 4;
   uint32_t s = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -126,8 +185,12 @@ __global__ void __launch_bounds__(kThreads) k_scan_reduce(const uint32_t* __rest
   if (threadIdx.x == 0) {
     uint32_t tot = 0;
     for (int w = 0; w < kThreads / 32; ++w) tot += ws[w];
-    block_sums[blockIdx.x] = tot;
+    block_sums[blk] = tot;
   }
+}
+__global__ void __launch_bounds__(kThreads) k_scan_reduce(const uint32_t* __restrict__ v,
+                                                          uint32_t* __restrict__ block_sums) {
+  scan_reduce(v, block_sums, blockIdx.x);
 }
 
 // Block-wide exclusive scan of one value per thread; returns the block total.
@@ -171,9 +234,8 @@ __global__ void __launch_bounds__(1024) k_scan_top(uint32_t* __restrict__ block_
 }
 
 // In-place exclusive scan of each tile plus its tile offset.
-__global__ void __launch_bounds__(kThreads) k_scan_apply(uint32_t* __restrict__ v,
-                                                         const uint32_t* __restrict__ block_sums) {
-  uint4* t = reinterpret_cast<uint4*>(v + (size_t)blockIdx.x * kScanTile) + threadIdx.x * 4;
+__device__ __forceinline__ void scan_apply(uint32_t* __restrict__ v, uint32_t before, uint32_t blk) {
+  uint4* t = reinterpret_cast<uint4*>(v + (size_t)blk * kScanTile) + threadIdx.x * 4;
   uint32_t a[kScanItems];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -191,29 +253,33 @@ __global__ void __launch_bounds__(kThreads) k_scan_apply(uint32_t* __restrict__ 
     s += x;
   }
   uint32_t total;
-  uint32_t off = block_exclusive_scan(s, total) + block_sums[blockIdx.x];
+  uint32_t off = block_exclusive_scan(s, total) + before;
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     t[q] = make_uint4(a[4 * q] + off, a[4 * q + 1] + off, a[4 * q + 2] + off, a[4 * q + 3] + off);
 }
+__global__ void __launch_bounds__(kThreads) k_scan_apply(uint32_t* __restrict__ v,
+                                                         const uint32_t* __restrict__ block_sums) {
+  scan_apply(v, block_sums[blockIdx.x], blockIdx.x);
+}
 
 // Every particle to its bucket's range (start = the scanned bucket counts),
 // in arrival order inside the bucket.
+__device__ __forceinline__ void scatter(int n, int bucket_shift, const uint32_t* __restrict__ cell_of,
+                                        const uint32_t* __restrict__ rank, const uint32_t* __restrict__ start,
+                                        uint32_t* __restrict__ tmp, int i) {
+  if (i < n) tmp[start[cell_of[i] >> bucket_shift] + rank[i]] = (uint32_t)i;
+}
 __global__ void __launch_bounds__(kThreads) k_scatter(int n, int bucket_shift, const uint32_t* __restrict__ cell_of,
                                                       const uint32_t* __restrict__ rank,
                                                       const uint32_t* __restrict__ start,
                                                       uint32_t* __restrict__ tmp) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  tmp[start[cell_of[i] >> bucket_shift] + rank[i]] = (uint32_t)i;
+  scatter(n, bucket_shift, cell_of, rank, start, tmp, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Cells up to kOrderSmall particles are ordered by k_order (each particle
 // counts the smaller keys of its cell); cells up to kOrderLarge by a bitonic
 // sort in shared memory (k_order_large); larger cells fall back to counting.
-constexpr uint32_t kOrderSmall = 64;
-constexpr uint32_t kOrderLarge = 4096;
-constexpr int kOrderThreads = 512;
 
 // Final slot of every particle: its rank by insertion index (or by in-cell
 // order key) among the particles of its cell.  The overflow cell keeps
@@ -221,20 +287,16 @@ constexpr int kOrderThreads = 512;
 // count <= kOrderLarge particles are left to k_order_large: the thread of
 // their first slot appends them to `large` (a list in any order; each cell's
 // result does not depend on it).
-__global__ void __launch_bounds__(kThreads) k_order(int n, int ncells, const uint32_t* __restrict__ cell_of,
-                                                    const uint32_t* __restrict__ cell_start,
-                                                    const uint32_t* __restrict__ tmp,
-                                                    const uint32_t* __restrict__ id,
-                                                    const unsigned long long* __restrict__ okey,
-                                                    uint32_t* __restrict__ perm,
-                                                    uint32_t* __restrict__ large,
-                                                    uint32_t* __restrict__ large_count) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
+template <class Place>
+__device__ __forceinline__ void order(
+    int n, int ncells, const uint32_t* __restrict__ cell_of, const uint32_t* __restrict__ cell_start,
+    const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ id, const unsigned long long* __restrict__ okey,
+    uint32_t* __restrict__ large, uint32_t* __restrict__ large_count, int s, Place place) {
   if (s >= n) return;
   uint32_t i = tmp[s];
   uint32_t cell = cell_of[i];
   if ((int)cell == ncells) {
-    perm[s] = i;
+    place((uint32_t)s, i);
     return;
   }
   uint32_t cs = cell_start[cell], ce = cell_start[cell + 1];
@@ -245,12 +307,21 @@ __global__ void __launch_bounds__(kThreads) k_order(int n, int ncells, const uin
   uint32_t r = 0;
   if (okey) {
     const unsigned long long mine = okey[i];
+#pragma unroll 8
     for (uint32_t k = cs; k < ce; ++k) r += okey[tmp[k]] < mine ? 1u : 0u;
   } else {
     const uint32_t mine = id[i];
+#pragma unroll 8
     for (uint32_t k = cs; k < ce; ++k) r += id[tmp[k]] < mine ? 1u : 0u;
   }
-  perm[cs + r] = i;
+  place(cs + r, i);
+}
+__global__ void __launch_bounds__(kThreads) k_order(
+    int n, int ncells, const uint32_t* __restrict__ cell_of, const uint32_t* __restrict__ cell_start,
+    const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ id, const unsigned long long* __restrict__ okey,
+    uint32_t* __restrict__ perm, uint32_t* __restrict__ large, uint32_t* __restrict__ large_count) {
+  order(n, ncells, cell_of, cell_start, tmp, id, okey, large, large_count, blockIdx.x * blockDim.x + threadIdx.x,
+        [&](uint32_t slot, uint32_t i) { perm[slot] = i; });
 }
 
 // Order key of particle i: the in-cell order key (tiled form) or the
@@ -267,15 +338,19 @@ __device__ __forceinline__ unsigned long long order_key(const unsigned long long
 // barrier between steps); a larger one is sorted with a bitonic network
 // padded to a power of two.  Either way each particle goes to its final slot.
 constexpr uint32_t kRankCount = 256;
-__global__ void __launch_bounds__(kOrderThreads) k_order_large(const uint32_t* __restrict__ cell_start,
-                                                              const uint32_t* __restrict__ tmp,
-                                                              const uint32_t* __restrict__ id,
-                                                              const unsigned long long* __restrict__ okey,
-                                                              const uint32_t* __restrict__ large,
-                                                              const uint32_t* __restrict__ large_count,
-                                                              uint32_t* __restrict__ perm) {
-  __shared__ unsigned long long s_key[kOrderLarge];
-  __shared__ uint32_t s_val[kOrderLarge];
+struct LargeStage {
+  unsigned long long key[kOrderLarge];
+  uint32_t val[kOrderLarge];
+};
+template <int kBlock, class Place>
+__device__ __forceinline__ void order_large(const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ tmp,
+                                            const uint32_t* __restrict__ id,
+                                            const unsigned long long* __restrict__ okey,
+                                            const uint32_t* __restrict__ large,
+                                            const uint32_t* __restrict__ large_count, LargeStage& stage,
+                                            Place place) {
+  unsigned long long* s_key = stage.key;
+  uint32_t* s_val = stage.val;
   const uint32_t nl = *large_count;
   for (uint32_t w = blockIdx.x; w < nl; w += gridDim.x) {
     const uint32_t cell = large[w];
@@ -283,7 +358,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_large(const uint32_t* _
     uint32_t m = 1;
     while (m < cnt) m <<= 1;
     __syncthreads();  // the previous cell's pairs are written out
-    for (uint32_t k = threadIdx.x; k < m; k += kOrderThreads) {
+    for (uint32_t k = threadIdx.x; k < m; k += kBlock) {
       if (k < cnt) {
         const uint32_t i = tmp[cs + k];
         s_key[k] = order_key(okey, id, i);
@@ -295,17 +370,17 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_large(const uint32_t* _
     }
     __syncthreads();
     if (cnt <= kRankCount) {
-      for (uint32_t k = threadIdx.x; k < cnt; k += kOrderThreads) {
+      for (uint32_t k = threadIdx.x; k < cnt; k += kBlock) {
         const unsigned long long mine = s_key[k];
         uint32_t r = 0;
         for (uint32_t q = 0; q < cnt; ++q) r += s_key[q] < mine ? 1u : 0u;
-        perm[cs + r] = s_val[k];
+        place(cs + r, s_val[k]);
       }
       continue;  // uniform; the next cell's staging waits at the loop's first barrier
     }
     for (uint32_t size = 2; size <= m; size <<= 1) {
       for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-        for (uint32_t k = threadIdx.x; k < m / 2; k += kOrderThreads) {
+        for (uint32_t k = threadIdx.x; k < m / 2; k += kBlock) {
           // Element pair (lo, lo + stride) of compare step k.
           const uint32_t lo = 2 * k - (k & (stride - 1));
           const uint32_t hi = lo + stride;
@@ -322,8 +397,19 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_large(const uint32_t* _
         __syncthreads();
       }
     }
-    for (uint32_t k = threadIdx.x; k < cnt; k += kOrderThreads) perm[cs + k] = s_val[k];
+    for (uint32_t k = threadIdx.x; k < cnt; k += kBlock) place(cs + k, s_val[k]);
   }
+}
+__global__ void __launch_bounds__(kOrderThreads) k_order_large(const uint32_t* __restrict__ cell_start,
+                                                              const uint32_t* __restrict__ tmp,
+                                                              const uint32_t* __restrict__ id,
+                                                              const unsigned long long* __restrict__ okey,
+                                                              const uint32_t* __restrict__ large,
+                                                              const uint32_t* __restrict__ large_count,
+                                                              uint32_t* __restrict__ perm) {
+  __shared__ LargeStage stage;
+  order_large<kOrderThreads>(cell_start, tmp, id, okey, large, large_count, stage,
+                             [&](uint32_t slot, uint32_t i) { perm[slot] = i; });
 }
 
 // ---- Tiled sort: counts per tile, cells per occupied tile ------------------
@@ -339,9 +425,9 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_large(const uint32_t* _
 // Per scan tile of the tile counts (kScanTile entries, kScanItems per
 // thread): the sum of the counts and the number of occupied tiles (index
 // below ntiles, count above zero).
-__global__ void __launch_bounds__(kThreads) k_tile_reduce(uint32_t ntiles, const uint32_t* __restrict__ cnt,
-                                                          uint2* __restrict__ sums) {
-  const uint32_t e0 = blockIdx.x * (uint32_t)kScanTile + threadIdx.x * (uint32_t)kScanItems;
+__device__ __forceinline__ void tile_reduce(uint32_t ntiles, const uint32_t* __restrict__ cnt,
+                                            uint2* __restrict__ sums, uint32_t blk) {
+  const uint32_t e0 = blk * (uint32_t)kScanTile + threadIdx.x * (uint32_t)kScanItems;
   const uint4* t = reinterpret_cast<const uint4*>(cnt + e0);
   uint32_t s = 0, o = 0;
 #pragma unroll
@@ -365,8 +451,12 @@ __global__ void __launch_bounds__(kThreads) k_tile_reduce(uint32_t ntiles, const
       tot.x += ws[w].x;
       tot.y += ws[w].y;
     }
-    sums[blockIdx.x] = tot;
+    sums[blk] = tot;
   }
+}
+__global__ void __launch_bounds__(kThreads) k_tile_reduce(uint32_t ntiles, const uint32_t* __restrict__ cnt,
+                                                          uint2* __restrict__ sums) {
+  tile_reduce(ntiles, cnt, sums, blockIdx.x);
 }
 
 // Exclusive scans of the tile counts (in place: the tile starts) and of the
@@ -375,14 +465,12 @@ __global__ void __launch_bounds__(kThreads) k_tile_reduce(uint32_t ntiles, const
 // before its own.  The thread holding entry ntiles (the overflow bucket)
 // writes the overflow cell's range, the number of occupied tiles and the end
 // of the last tile.
-__global__ void __launch_bounds__(kThreads) k_tile_scan(int n, int ncells, uint32_t ntiles, uint32_t* __restrict__ cnt,
-                                                        const uint2* __restrict__ sums,
-                                                        uint32_t* __restrict__ cell_start,
-                                                        uint32_t* __restrict__ tile_of,
-                                                        uint32_t* __restrict__ tile_slot,
-                                                        uint32_t* __restrict__ num_tiles) {
+__device__ __forceinline__ void tile_scan(
+    int n, int ncells, uint32_t ntiles, uint32_t* __restrict__ cnt, const uint2* __restrict__ sums,
+    uint32_t* __restrict__ cell_start, uint32_t* __restrict__ tile_of, uint32_t* __restrict__ tile_slot,
+    uint32_t* __restrict__ num_tiles, uint32_t blk) {
   uint32_t ps = 0, po = 0, total = 0;
-  for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) {
+  for (uint32_t k = threadIdx.x; k < blk; k += blockDim.x) {
     const uint2 v = sums[k];
     ps += v.x;
     po += v.y;
@@ -391,7 +479,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(int n, int ncells, uint3
   const uint32_t carry_s = total;
   (void)block_exclusive_scan(po, total);
   const uint32_t carry_o = total;
-  const uint32_t e0 = blockIdx.x * (uint32_t)kScanTile + threadIdx.x * (uint32_t)kScanItems;
+  const uint32_t e0 = blk * (uint32_t)kScanTile + threadIdx.x * (uint32_t)kScanItems;
   uint4* t = reinterpret_cast<uint4*>(cnt + e0);
   uint32_t a[kScanItems];
 #pragma unroll
@@ -432,6 +520,12 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(int n, int ncells, uint3
     tile_slot[count] = of;  // the end of the last tile
   }
 }
+__global__ void __launch_bounds__(kThreads) k_tile_scan(
+    int n, int ncells, uint32_t ntiles, uint32_t* __restrict__ cnt, const uint2* __restrict__ sums,
+    uint32_t* __restrict__ cell_start, uint32_t* __restrict__ tile_of, uint32_t* __restrict__ tile_slot,
+    uint32_t* __restrict__ num_tiles) {
+  tile_scan(n, ncells, ntiles, cnt, sums, cell_start, tile_of, tile_slot, num_tiles, blockIdx.x);
+}
 
 // One CTA per occupied tile (persistent over the tile list).  The tile's
 // particles (`tmp`, grouped by tile) are counted per cell in shared memory;
@@ -441,31 +535,32 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(int n, int ncells, uint3
 // particles to the dense-cell passes.  Then every particle goes to its final
 // slot in `perm`: its rank among its cell's particles by in-cell order key
 // (the keys are unique).  A tile of at most kTileOrder particles whose cells
-// hold at most kOrderSmall each counts the smaller keys in shared memory;
+// hold at most kRankCount each counts the smaller keys in shared memory;
 // other tiles scatter their particles by cell into `out` and count in global
-// memory, except in cells of kOrderSmall < count <= kOrderLarge particles,
+// memory, except in cells of kOrderTile < count <= kOrderLarge particles,
 // which go to `large` for k_order_large (the thread of the cell's first slot
 // appends it).  Particles of the overflow cell keep their slots.
 constexpr int kTileCache = 4;                         // particles per thread held in registers
 constexpr int kTileOrder = kTileCache * kThreads;     // 1024
 template <int kCells>
-__global__ void __launch_bounds__(kThreads) k_tile_cells(int n, int ncells, const uint32_t* __restrict__ tstart,
-                                                         const uint32_t* __restrict__ tile_of,
-                                                         const uint32_t* __restrict__ num_tiles,
-                                                         const uint32_t* __restrict__ tmp,
-                                                         const uint32_t* __restrict__ cell_of,
-                                                         const unsigned long long* __restrict__ okey,
-                                                         uint32_t* __restrict__ rank, uint32_t* __restrict__ perm,
-                                                         uint32_t* __restrict__ out, uint32_t* __restrict__ cell_start,
-                                                         uint32_t* __restrict__ tile_slot,
-                                                         uint8_t* __restrict__ tile_crowd, int dense_mean,
-                                                         uint32_t* __restrict__ large,
-                                                         uint32_t* __restrict__ large_count) {
+struct TileStage {
+  uint32_t cnt[kCells];
+  uint32_t off[kCells + 1];
+  int small;  // every cell of the tile holds at most kRankCount particles
+  unsigned long long key[kTileOrder];
+};
+template <int kCells, class Place>
+__device__ __forceinline__ void tile_cells(
+    int n, int ncells, const uint32_t* __restrict__ tstart, const uint32_t* __restrict__ tile_of,
+    const uint32_t* __restrict__ num_tiles, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ cell_of,
+    const unsigned long long* __restrict__ okey, uint32_t* __restrict__ rank,
+    uint32_t* __restrict__ out, uint32_t* __restrict__ cell_start, uint32_t* __restrict__ tile_slot,
+    uint8_t* __restrict__ tile_crowd, int dense_mean, uint32_t* __restrict__ large,
+    uint32_t* __restrict__ large_count, TileStage<kCells>& stage, Place place) {
   static_assert(kCells == 8 || kCells == 64, "tile of 2x2x2 or 4x4x4 cells");
-  __shared__ uint32_t s_cnt[kCells];
-  __shared__ uint32_t s_off[kCells + 1];
-  __shared__ unsigned long long s_key[kTileOrder];
-  __shared__ int s_small;  // every cell of the tile holds at most kOrderSmall particles
+  uint32_t *s_cnt = stage.cnt, *s_off = stage.off;
+  unsigned long long* s_key = stage.key;
+  int& s_small = stage.small;
   const uint32_t count = *num_tiles;
   const int lane = threadIdx.x & 31;
   for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) {
@@ -519,7 +614,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_cells(int n, int ncells, cons
       }
       const uint32_t total0 = __shfl_sync(0xffffffffu, x0, 31);
       const uint32_t occ = __popc(__ballot_sync(0xffffffffu, a0 > 0u)) + __popc(__ballot_sync(0xffffffffu, a1 > 0u));
-      const bool big = __any_sync(0xffffffffu, a0 > kOrderSmall || a1 > kOrderSmall);
+      const bool big = __any_sync(0xffffffffu, a0 > kRankCount || a1 > kRankCount);
       if (lane < kCells) {
         s_off[lane] = x0 - a0;
         cell_start[cell0 + lane] = ts + x0 - a0;
@@ -549,7 +644,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_cells(int n, int ncells, cons
           const unsigned long long mine = s_key[c0 + cr[j]];
           uint32_t r = 0;
           for (uint32_t q = c0; q < c1; ++q) r += s_key[q] < mine ? 1u : 0u;
-          perm[ts + c0 + r] = ci[j];
+          place(ts + c0 + r, ci[j]);
         }
     } else {
       if (cached) {
@@ -580,23 +675,37 @@ __global__ void __launch_bounds__(kThreads) k_tile_cells(int n, int ncells, cons
         const uint32_t i = out[e];
         const uint32_t l = cell_of[i] - cell0;
         const uint32_t c0 = ts + s_off[l], c1 = ts + s_off[l + 1];
-        if (c1 - c0 > kOrderSmall && c1 - c0 <= kOrderLarge) {
+        if (c1 - c0 > kOrderTile && c1 - c0 <= kOrderLarge) {
           if (e == c0) large[atomicAdd(large_count, 1u)] = cell0 + l;
           continue;
         }
         const unsigned long long mine = okey[i];
         uint32_t r = 0;
+#pragma unroll 8
         for (uint32_t q = c0; q < c1; ++q) r += okey[out[q]] < mine ? 1u : 0u;
-        perm[c0 + r] = i;
+        place(c0 + r, i);
       }
     }
     __syncthreads();  // the counters and keys are free for the next tile
   }
   const uint32_t of = cell_start[ncells];
   for (uint32_t e = of + blockIdx.x * blockDim.x + threadIdx.x; e < (uint32_t)n; e += gridDim.x * blockDim.x) {
-    out[e] = tmp[e];
-    perm[e] = tmp[e];
+    place(e, tmp[e]);
   }
+}
+
+template <int kCells>
+__global__ void __launch_bounds__(kThreads) k_tile_cells(
+    int n, int ncells, const uint32_t* __restrict__ tstart, const uint32_t* __restrict__ tile_of,
+    const uint32_t* __restrict__ num_tiles, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ cell_of,
+    const unsigned long long* __restrict__ okey, uint32_t* __restrict__ rank, uint32_t* __restrict__ perm,
+    uint32_t* __restrict__ out, uint32_t* __restrict__ cell_start, uint32_t* __restrict__ tile_slot,
+    uint8_t* __restrict__ tile_crowd, int dense_mean, uint32_t* __restrict__ large,
+    uint32_t* __restrict__ large_count) {
+  __shared__ TileStage<kCells> stage;
+  tile_cells<kCells>(n, ncells, tstart, tile_of, num_tiles, tmp, cell_of, okey, rank, out, cell_start, tile_slot,
+                     tile_crowd, dense_mean, large, large_count, stage,
+                     [&](uint32_t slot, uint32_t i) { perm[slot] = i; });
 }
 
 struct GatherArgs {
@@ -613,12 +722,26 @@ struct GatherArgs {
   float4* cvel;
   uint32_t* queue;
   double inv_cell, h0;
+  // f64 plain form (nullable): box-relative f32 coordinates with the z cell
+  // key, the first part of the packed pair operands, and the word that sends
+  // the force pass to plain divisions when a coordinate or mass leaves the
+  // range where its reciprocals are exact.
+  float4* fpos;
+  double* rec;
+  uint32_t* unsafe;
+  double origin[3];
+  long long bz0;
 };
 
-__global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __restrict__ perm, GatherArgs g) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  uint32_t i = perm[s];
+// Zero, or far enough from the ends of the f64 range that differences and
+// products of such values keep exact remainders.
+__device__ __forceinline__ bool plain_safe(double x, double least, double most) {
+  const double m = fabs(x);
+  return x == 0.0 || (m > least && m < most);
+}
+
+// Moves the state of particle i to sorted slot s.
+__device__ __forceinline__ void move_particle(const GatherArgs& g, uint32_t s, uint32_t i) {
 #pragma unroll
   for (int k = 0; k < 6; ++k) g.dst_pv[k][s] = g.src_pv[k][i];
   g.dst.mass[s] = g.src.mass[i];
@@ -630,6 +753,18 @@ __global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __re
   }
   if (g.src.scene) g.dst.scene[s] = g.src.scene[i];
   if (g.sorted_cell) g.sorted_cell[s] = g.cell_of[i];
+  if (g.rec) {
+    const double x = g.dst_pv[0][s], y = g.dst_pv[1][s], z = g.dst_pv[2][s], m = g.dst.mass[s];
+    const long long kz = key_axis(z, g.inv_cell) - g.bz0;
+    g.fpos[s] = make_float4((float)(x - g.origin[0]), (float)(y - g.origin[1]), (float)(z - g.origin[2]),
+                            __int_as_float((int)kz));
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(g.rec + (size_t)s * 4), "d"(x), "d"(y),
+                 "d"(z), "d"(m)
+                 : "memory");
+    if (!(plain_safe(x, 1e-200, 1e100) && plain_safe(y, 1e-200, 1e100) && plain_safe(z, 1e-200, 1e100) &&
+          plain_safe(m, 1e-60, 1e60)))
+      atomicOr(g.unsafe, 1u);
+  }
   if (g.cpos) {
     // Cell-local f32 coordinates (the cell is that of the f64 cell key).
     const double x = g.dst_pv[0][s], y = g.dst_pv[1][s], z = g.dst_pv[2][s];
@@ -645,6 +780,130 @@ __global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __re
       g.queue[4] = 0;
     }
   }
+}
+
+__global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __restrict__ perm, GatherArgs g) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < n) move_particle(g, (uint32_t)s, perm[s]);
+}
+
+// ---- The whole sort in one launch ------------------------------------------------
+//
+// A step of a small world is bound by its launches: the sort's eight kernels
+// and their memsets take ~3 us each whatever the particle count.  Below
+// kFusedBelow particles the sort is one cooperative launch instead (every
+// block resident), whose phases are the kernels' bodies over grid strides,
+// separated by a grid barrier of ~1.5 us: zero the counts | histogram, with
+// the scan tiles' sums | scan | scatter by bucket | order | gather.  Where no
+// cell is crowded the x-major form moves each particle's state as soon as its
+// slot is known (a tile's particles share a block, too few threads to move
+// them).
+struct SortArgs {
+  HistArgs h;
+  int ncells, dense_mean;
+  uint32_t len;           // scanned entries (whole scan tiles)
+  uint2* sums;            // per scan tile: particles, occupied tiles
+  uint32_t* cell_start;
+  uint32_t* tmp;
+  uint32_t* perm;
+  uint32_t* large;
+  uint32_t* large_count;
+  uint32_t* barrier;      // arrivals, zeroed before the launch
+  uint32_t* tile_of;
+  uint32_t* tile_slot;
+  uint32_t* num_tiles;
+  uint32_t* out;          // tiled: by-cell list of the tiles ordered in global memory
+  uint8_t* tile_crowd;
+  GatherArgs g;
+};
+
+// Waits until every block has arrived for the `phase`-th time; false (and the
+// error bit set) when the others do not arrive within the poll limit, which a
+// cooperative launch never lets happen.
+__device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t phase, uint32_t* flags) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(counter, 1u);
+    const uint32_t want = phase * gridDim.x;
+    uint32_t seen = 0;
+    int polls = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+    } while (seen < want && ++polls < (1 << 22));
+    s_ok = seen >= want;
+    if (seen < want) atomicOr(flags, kFlagSortLost);
+    __threadfence();
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// kCells: cells per tile (8 or 64), or 0 for the x-major form.
+template <int kCells>
+__global__ void __launch_bounds__(kThreads) k_sort_fused(StepConsts c, SortArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];  // sizeof(LargeStage), the larger of the two
+  LargeStage& large_stage = *reinterpret_cast<LargeStage*>(smem);
+  auto& tile_stage = *reinterpret_cast<TileStage<kCells == 0 ? 8 : kCells>*>(smem);
+  static_assert(sizeof(tile_stage) <= sizeof(LargeStage), "one staging area");
+  const int n = c.n;
+  const int first = (int)(blockIdx.x * blockDim.x), step = (int)(gridDim.x * blockDim.x);
+  const uint32_t blocks = a.len / (uint32_t)kScanTile;
+  uint32_t phase = 0;
+  uint4* zero = reinterpret_cast<uint4*>(a.h.count);
+  for (uint32_t k = (uint32_t)first + threadIdx.x; k < a.len / 4u; k += (uint32_t)step) zero[k] = make_uint4(0, 0, 0, 0);
+  if (kCells == 0)
+    for (uint32_t k = (uint32_t)first + threadIdx.x; k < blocks; k += (uint32_t)step) a.sums[k] = make_uint2(0u, 0u);
+  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  for (int i0 = first; i0 < n; i0 += step) cell_hist(c, a.h, i0 + (int)threadIdx.x);  // whole blocks
+  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (kCells != 0) {
+    // (A tile's few counters would be contended if the histogram summed them.)
+    for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+      tile_reduce(a.h.buckets, a.h.count, a.sums, b);
+      __syncthreads();
+    }
+    if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  }
+  for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+    if (kCells == 0) {
+      uint32_t before = 0, total = 0;
+      for (uint32_t k = threadIdx.x; k < b; k += blockDim.x) before += a.sums[k].x;
+      (void)block_exclusive_scan(before, total);
+      scan_apply(a.h.count, total, b);
+    } else {
+      tile_scan(n, a.ncells, a.h.buckets, a.h.count, a.sums, a.cell_start, a.tile_of, a.tile_slot, a.num_tiles, b);
+    }
+  }
+  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  for (int i0 = first; i0 < n; i0 += step)
+    scatter(n, a.h.bucket_shift, a.h.cell_of, a.h.rank, a.h.count, a.tmp, i0 + (int)threadIdx.x);
+  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  auto list = [&](uint32_t slot, uint32_t i) { a.perm[slot] = i; };
+  if (kCells == 0 && *a.h.crowded == 0u) {  // settled by the histogram: uniform across the grid
+    for (int s0 = first; s0 < n; s0 += step)
+      order(n, a.ncells, a.h.cell_of, a.cell_start, a.tmp, a.h.id, a.h.okey, a.large, a.large_count,
+            s0 + (int)threadIdx.x, [&](uint32_t slot, uint32_t i) { move_particle(a.g, slot, i); });
+    return;
+  }
+  if (kCells == 0) {
+    for (int s0 = first; s0 < n; s0 += step)
+      order(n, a.ncells, a.h.cell_of, a.cell_start, a.tmp, a.h.id, a.h.okey, a.large, a.large_count,
+            s0 + (int)threadIdx.x, list);
+  } else {
+    tile_cells<kCells == 0 ? 8 : kCells>(n, a.ncells, a.h.count, a.tile_of, a.num_tiles, a.tmp, a.h.cell_of, a.h.okey,
+                                         a.h.rank, a.out, a.cell_start, a.tile_slot, a.tile_crowd, a.dense_mean,
+                                         a.large, a.large_count, tile_stage, list);
+  }
+  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (*a.large_count != 0u) {  // uniform
+    order_large<kThreads>(a.cell_start, kCells == 0 ? a.tmp : a.out, a.h.id, a.h.okey, a.large, a.large_count,
+                          large_stage, list);
+    if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  }
+  for (int s0 = first; s0 < n; s0 += step)
+    if (s0 + (int)threadIdx.x < n) move_particle(a.g, (uint32_t)(s0 + (int)threadIdx.x), a.perm[s0 + (int)threadIdx.x]);
 }
 
 __global__ void k_unsort_f64(int n, const uint32_t* __restrict__ id, const double* __restrict__ src,
@@ -732,57 +991,121 @@ static void scan_in_place(uint32_t* v, int len, uint32_t* block_sums, cudaStream
   k_scan_apply<<<nb, kThreads, 0, s>>>(v, block_sums);
 }
 
+static HistArgs hist_args(const StepConsts& c, DevBuffers& b, unsigned long long* okey, uint32_t* flags) {
+  const ParticleConsts& src = b.pc[b.cur];
+  HistArgs h;
+  h.bucket_shift = c.tile ? 3 * c.tile_log2 : 0;
+  h.px = b.pv1[0];
+  h.py = b.pv1[1];
+  h.pz = b.pv1[2];
+  h.cell_of = b.cell_of;
+  h.rank = b.rank;
+  h.count = c.tile ? b.tile_head : b.cell_start;
+  h.flags = flags;
+  h.scene = src.scene;
+  h.id = src.id;
+  h.okey = okey;
+  h.sums = nullptr;
+  h.buckets = 0;
+  h.crowded = nullptr;
+  return h;
+}
+
+// (order_count is zero when the launches start.)
 static void build_cells(const StepConsts& c, DevBuffers& b, cudaStream_t s, int bs, unsigned long long* okey,
                         uint32_t* flags) {
   const int n = c.n;
-  const ParticleConsts& src = b.pc[b.cur];
-  cudaMemsetAsync(b.order_count, 0, sizeof(uint32_t), s);
+  const HistArgs h = hist_args(c, b, okey, flags);
   if (c.tile) {
     // Tiled: counts per tile, their scan with the occupied-tile list, then
     // cells and in-cell order per occupied tile (the tile-count array is
     // tile_head; the by-cell list of the tiles ordered in global memory goes
     // to sorted_cell, which the gather rewrites).
-    const int shift = 3 * c.tile_log2;
-    const int ntiles = c.ncells >> shift;
+    const int ntiles = c.ncells >> h.bucket_shift;
     const int tlen = scan_length(ntiles);
     uint2* sums = reinterpret_cast<uint2*>(b.block_sums);  // 2 x tlen / kScanTile entries
     cudaMemsetAsync(b.tile_head, 0, (size_t)tlen * sizeof(uint32_t), s);
-    k_cell_hist<<<grid_for(n, bs), bs, 0, s>>>(c, shift, b.pv1[0], b.pv1[1], b.pv1[2], b.cell_of, b.rank,
-                                                 b.tile_head, flags, src.scene, src.id, okey);
+    k_cell_hist<<<grid_for(n, bs), bs, 0, s>>>(c, h);
     k_tile_reduce<<<tlen / kScanTile, kThreads, 0, s>>>((uint32_t)ntiles, b.tile_head, sums);
     k_tile_scan<<<tlen / kScanTile, kThreads, 0, s>>>(n, c.ncells, (uint32_t)ntiles, b.tile_head, sums,
                                                       b.cell_start, b.tile_of, b.tile_slot, b.num_tiles);
-    k_scatter<<<grid_for(n, bs), bs, 0, s>>>(n, shift, b.cell_of, b.rank, b.tile_head, b.tmp);
+    k_scatter<<<grid_for(n, bs), bs, 0, s>>>(n, h.bucket_shift, b.cell_of, b.rank, b.tile_head, b.tmp);
     auto cells = c.tile == 4 ? k_tile_cells<64> : k_tile_cells<8>;
     cells<<<tile_cells_blocks(), kThreads, 0, s>>>(n, c.ncells, b.tile_head, b.tile_of, b.num_tiles, b.tmp, b.cell_of,
                                                   okey, b.rank, b.perm, b.sorted_cell, b.cell_start, b.tile_slot,
                                                   b.tile_crowd, c.dense_mean, b.large_cells, b.order_count);
-    k_order_large<<<order_large_blocks(), kOrderThreads, 0, s>>>(b.cell_start, b.sorted_cell, src.id, okey,
+    k_order_large<<<order_large_blocks(), kOrderThreads, 0, s>>>(b.cell_start, b.sorted_cell, h.id, okey,
                                                                  b.large_cells, b.order_count, b.perm);
     return;
   }
   const int len = scan_length(c.ncells);
   cudaMemsetAsync(b.cell_start, 0, (size_t)len * sizeof(uint32_t), s);
-  k_cell_hist<<<grid_for(n, bs), bs, 0, s>>>(c, 0, b.pv1[0], b.pv1[1], b.pv1[2], b.cell_of, b.rank, b.cell_start,
-                                               flags, src.scene, src.id, okey);
+  k_cell_hist<<<grid_for(n, bs), bs, 0, s>>>(c, h);
   scan_in_place(b.cell_start, len, b.block_sums, s);
   k_scatter<<<grid_for(n, bs), bs, 0, s>>>(n, 0, b.cell_of, b.rank, b.cell_start, b.tmp);
   // `rank` is free after the scatter: it holds the list of large cells.
-  k_order<<<grid_for(n, bs), bs, 0, s>>>(n, c.ncells, b.cell_of, b.cell_start, b.tmp, src.id, okey, b.perm, b.rank,
+  k_order<<<grid_for(n, bs), bs, 0, s>>>(n, c.ncells, b.cell_of, b.cell_start, b.tmp, h.id, okey, b.perm, b.rank,
                                          b.order_count);
-  k_order_large<<<order_large_blocks(), kOrderThreads, 0, s>>>(b.cell_start, b.tmp, src.id, okey, b.rank,
+  k_order_large<<<order_large_blocks(), kOrderThreads, 0, s>>>(b.cell_start, b.tmp, h.id, okey, b.rank,
                                                                b.order_count, b.perm);
 }
 
 void launch_cell_index(const StepConsts& c, DevBuffers& b, uint32_t* flags, cudaStream_t s) {
+  cudaMemsetAsync(b.order_count, 0, sizeof(uint32_t), s);
   build_cells(c, b, s, kThreads, nullptr, flags);
+}
+
+// Blocks of the fused sort: resident, at most four per SM (the barrier takes
+// 1.3 us with 35 blocks and 1.6 us with 296).
+template <int kCells>
+static int fused_blocks() {
+  static const int blocks = [] {
+    int dev = 0, sms = 1, per = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(k_sort_fused<kCells>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LargeStage));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sort_fused<kCells>, kThreads, sizeof(LargeStage));
+    return std::max(sms, 1) * std::min(std::max(per, 1), 4);
+  }();
+  return blocks;
+}
+
+template <int kCells>
+static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g, cudaStream_t s) {
+  SortArgs a;
+  a.h = hist_args(c, b, c.tile ? b.okey : nullptr, b.flags);
+  a.ncells = c.ncells;
+  a.dense_mean = c.dense_mean;
+  a.h.buckets = (uint32_t)(c.ncells >> a.h.bucket_shift);
+  a.len = (uint32_t)scan_length((int)a.h.buckets);
+  a.sums = reinterpret_cast<uint2*>(b.block_sums);
+  a.h.sums = c.tile ? nullptr : a.sums;
+  a.h.crowded = b.order_count + 2;
+  a.cell_start = b.cell_start;
+  a.tmp = b.tmp;
+  a.perm = b.perm;
+  a.large = c.tile ? b.large_cells : b.rank;
+  a.large_count = b.order_count;
+  a.barrier = b.order_count + 1;
+  a.tile_of = b.tile_of;
+  a.tile_slot = b.tile_slot;
+  a.num_tiles = b.num_tiles;
+  a.out = b.sorted_cell;
+  a.tile_crowd = b.tile_crowd;
+  a.g = g;
+  // Enough blocks for the particles and the scanned entries, at most the resident ones
+  // (all of those when tiled: crowded cells are ordered a block each).
+  const int want = c.tile ? INT_MAX : std::max(grid_for(c.n), (int)(a.len / kScanTile));
+  StepConsts cc = c;
+  void* args[] = {&cc, &a};
+  cudaLaunchCooperativeKernel((const void*)k_sort_fused<kCells>, dim3((unsigned)std::min(want, fused_blocks<kCells>())),
+                              dim3(kThreads), args, sizeof(LargeStage), s);
 }
 
 void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, int block) {
   // Per-particle kernels take any warp multiple up to kThreads.
   const int bs = block >= 32 && block <= kThreads ? block / 32 * 32 : kThreads;
   const int n = c.n;
-  build_cells(c, b, s, bs, c.tile ? b.okey : nullptr, b.flags);
   const ParticleConsts& src = b.pc[b.cur];
   const ParticleConsts& dst = b.pc[b.cur ^ 1];
   GatherArgs g;
@@ -794,13 +1117,31 @@ void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, int block) 
   g.dst = dst;
   g.has_ba = b.has_ba ? 1 : 0;
   g.cell_of = b.cell_of;
-  g.sorted_cell = c.tile ? b.sorted_cell : nullptr;
+  g.sorted_cell = c.tile || c.plain ? b.sorted_cell : nullptr;
   g.cpos = c.tile ? b.cpos : nullptr;
   g.cvel = c.tile ? b.cvel : nullptr;
   g.queue = c.tile ? b.queue : nullptr;
   g.inv_cell = c.inv_cell;
   g.h0 = c.h0;
-  k_gather<<<grid_for(n, bs), bs, 0, s>>>(n, b.perm, g);
+  g.fpos = c.plain ? b.cpos : nullptr;
+  g.rec = c.plain ? b.rec : nullptr;
+  g.unsafe = b.flags + 1;
+  g.origin[0] = (double)c.bx0 * c.h0;
+  g.origin[1] = (double)c.by0 * c.h0;
+  g.origin[2] = (double)c.bz0 * c.h0;
+  g.bz0 = c.bz0;
+  const int buckets = c.tile ? c.ncells >> (3 * c.tile_log2) : c.ncells;
+  if (n < kFusedBelow && buckets < kFusedBuckets) {
+    if (c.tile == 4)
+      launch_fused<64>(c, b, g, s);
+    else if (c.tile == 2)
+      launch_fused<8>(c, b, g, s);
+    else
+      launch_fused<0>(c, b, g, s);
+  } else {
+    build_cells(c, b, s, bs, c.tile ? b.okey : nullptr, b.flags);
+    k_gather<<<grid_for(n, bs), bs, 0, s>>>(n, b.perm, g);
+  }
   b.cur ^= 1;
 }
 

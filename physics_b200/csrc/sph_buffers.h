@@ -38,7 +38,14 @@ struct DevBuffers {
   double* acc[3] = {};
   double* xsph[3] = {};
   double* mu = nullptr;
-  // f32-compensated form: per-particle packed operands.
+  // f64 plain form: packed pair operands in three arrays of `capacity`
+  // records: x y z mass | vx vy vz rho | p/rho^2 1/rho.
+  double* rec = nullptr;
+  // f64 plain form: the neighbour search's records (kSearchRecord words per
+  // group of 32 slots).
+  uint32_t* search = nullptr;
+  // f32-compensated form: per-particle packed operands.  (The f64 plain form
+  // keeps box-relative f32 x, y, z and the z cell key in cpos.)
   float4* cpos = nullptr;  // cell-local x, y, z (f32) and mass
   float4* cvel = nullptr;  // vx, vy, vz (f32) and p/rho^2 (f32)
   float* cmr = nullptr;    // mass/rho (f32)
@@ -62,7 +69,7 @@ struct DevBuffers {
   size_t tile_scan_entries = 0;
   uint32_t* tile_of = nullptr;
   uint32_t* tile_slot = nullptr;
-  uint32_t* large_cells = nullptr;  // cells of more than kOrderSmall particles (capacity / 64 + 64)
+  uint32_t* large_cells = nullptr;  // cells left to order_large (capacity / 16 + 64)
   uint8_t* tile_crowd = nullptr;  // 1: tile above kDenseMean per occupied cell
   uint32_t* num_tiles = nullptr;
   // Scene boxes of the tiled linearisation (one entry for a single world),
@@ -99,8 +106,11 @@ struct DevBuffers {
   int block_sums_capacity = 0;
   // Insertion-order staging for uploads and downloads (f64 and u32 views).
   double* stage = nullptr;   // 8 * capacity doubles
-  uint32_t* flags = nullptr; // error bits, device
-  uint32_t* order_count = nullptr;  // sort: cells of more than kOrderSmall particles (device count)
+  // [0] error bits, [1] f64 plain step outside the reciprocals' safe range,
+  // [2] the sort's large-cell count, [3] its barrier arrivals, [4] whether a
+  // bucket is crowded; zeroed by one memset per step (device).
+  uint32_t* flags = nullptr;
+  uint32_t* order_count = nullptr;  // sort: cells of more than kOrderSmall particles (flags + 2)
   unsigned long long* counters = nullptr;  // candidates, pairs (device)
   // Optional outputs of the f64 plain force pass for the adjoint's tape: the
   // raw viscous force and the strain-rate proxy of every sorted slot.

@@ -28,6 +28,15 @@ constexpr int kCodeBits = 5;
 // and written out coalesced; further entries go straight to global memory.
 constexpr int kStagedNeighbors = 40;
 
+// f64 plain form: doubles per particle of the packed pair operands (parts
+// of 4, 4 and 2).
+constexpr int kPlainRec = 10;
+// f64 plain form: 32-candidate words the neighbour search keeps per group of
+// 32 slots (512 candidates; a group of a column at rest density has ~215), and
+// the u32 words of a group's record.
+constexpr int kSearchWords = 16;
+constexpr int kSearchRecord = 2 * kSearchWords * 32 + 2;
+
 // Tiled form: by default a tile whose occupied cells hold more than this many
 // particles on average goes to the dense-cell passes even when its halo could
 // be staged (StepConsts::dense_mean, a tuning knob); from about this density
@@ -35,10 +44,14 @@ constexpr int kStagedNeighbors = 40;
 // every query.
 constexpr uint32_t kDenseMean = 32;
 
+// Words of DevBuffers::flags.
+constexpr int kStepWords = 8;
+
 // Error bits written by device code into the per-world flag word.
 enum : uint32_t {
   kFlagOutOfBox = 1u,    // a cell key fell outside the grid box
   kFlagNonFinite = 2u,   // a new position or velocity is NaN/Inf
+  kFlagSortLost = 8u,   // a grid barrier of the fused sort ran out of polls: the step did not happen
   kFlagMaskTable = 4u,   // a dense-cell task's kept masks lie outside the mask buffer (filtered again)
 };
 
@@ -79,6 +92,7 @@ struct StepConsts {
   // x-major, so a tile's particles are contiguous (ncx, ncy, ncz are then
   // multiples of B and ntx, nty, ntz count tiles).
   int tile, tile_log2;
+  int plain;  // 1: f64 plain step (the sort writes its packed operands)
   int ntx, nty, ntz;
   // Tiles whose halo holds more particles than this are computed from
   // global memory instead of shared memory (<= the kernels' capacity).

@@ -170,6 +170,15 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* ws, uint32_
   return off + x - v;
 }
 
+// Tiles of the list: none when the sort did not finish.
+__device__ __forceinline__ uint32_t occupied_tiles(const TiledArgs& a) {
+  return (a.flags[0] & kFlagSortLost) ? 0u : *a.num_tiles;
+}
+// First slot of the overflow cell when no tile is occupied.
+__device__ __forceinline__ uint32_t first_outside(const TiledArgs& a) {
+  return (a.flags[0] & kFlagSortLost) ? 0u : a.tile_slot[0];
+}
+
 struct TileGeom {
   int tx, ty, tz;  // tile coordinates inside the scene box
   int sc;          // scene
@@ -450,7 +459,7 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2), H0SQ = f2_pack(c.h0sqf, c.h0sqf);
   __shared__ uint32_t s_next;
-  const uint32_t ntiles = *a.num_tiles;
+  const uint32_t ntiles = occupied_tiles(a);
   unsigned cand = 0, pairs = 0;
   for (uint32_t k = next_tile(a.queue, 0, blockIdx.x, &s_next); k < ntiles;
        k = next_tile(a.queue, 0, k + gridDim.x, &s_next)) {
@@ -511,7 +520,7 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
     }  // slabs
   }
   // Particles of the overflow cell (outside the grid box): no neighbours.
-  const uint32_t end = a.tile_slot[ntiles];
+  const uint32_t end = ntiles ? a.tile_slot[ntiles] : first_outside(a);
   for (uint32_t qi = end + blockIdx.x * kTT + threadIdx.x; qi < (uint32_t)c.n; qi += gridDim.x * kTT) {
     write_density(c, a, (int)qi, 0.0);
     a.nbr_count[qi] = 0;
@@ -787,7 +796,7 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
   uint32_t* ws = s_off + T::NH + 1;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   __shared__ uint32_t s_next;
-  const uint32_t ntiles = *a.num_tiles;
+  const uint32_t ntiles = occupied_tiles(a);
   for (uint32_t k = next_tile(a.queue, 1, blockIdx.x, &s_next); k < ntiles;
        k = next_tile(a.queue, 1, k + gridDim.x, &s_next)) {
     const TileGeom g = tile_geom<TB>(c, a, k);
@@ -858,7 +867,7 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
     __syncthreads();
     }  // slabs
   }
-  const uint32_t end = a.tile_slot[ntiles];
+  const uint32_t end = ntiles ? a.tile_slot[ntiles] : first_outside(a);
   for (uint32_t qi = end + blockIdx.x * kTT + threadIdx.x; qi < (uint32_t)c.n; qi += gridDim.x * kTT) {
     CompAcc q;
     finish_particle(c, a, (int)qi, q, c.boxes[a.scene ? (int)a.scene[qi] : 0], load_own(a, (int)qi));
