@@ -92,42 +92,111 @@ __global__ void k_append(int n0, int m, const double* __restrict__ st, double* p
   id[s] = (uint32_t)s;
 }
 
-// Cell-key bounding box of n interleaved positions: out[0..2] min, out[3..5]
-// max over finite coordinates, out[6] = 1 when a coordinate is not finite.
-// out must be preset to (LLONG_MAX x3, LLONG_MIN x3, 0).
-__global__ void k_key_bbox(int n, const double* __restrict__ pos3, double inv, long long* out) {
+// Cell-key bounding box of positions in a launch's own order: min and max
+// keys of the finite coordinates and a non-finite flag.
+struct KeyBox {
   long long mn[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, mx[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
   int bad = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      double x = pos3[3 * (size_t)i + a];
-      if (!isfinite(x)) {
-        bad = 1;
-        continue;
-      }
-      long long k = key_axis(x, inv);
-      mn[a] = k < mn[a] ? k : mn[a];
-      mx[a] = k > mx[a] ? k : mx[a];
+  __device__ __forceinline__ void add(int a, double x, double inv) {
+    if (!isfinite(x)) {
+      bad = 1;
+      return;
     }
+    const long long k = key_axis(x, inv);
+    mn[a] = k < mn[a] ? k : mn[a];
+    mx[a] = k > mx[a] ? k : mx[a];
   }
+};
+
+// Blocks' partial boxes (7 values each: min xyz, max xyz, non-finite) and
+// the arrival count that ends at zero again.
+constexpr int kBoxBlocks = 148 * 8;
+struct BoxScratch {
+  long long part[kBoxBlocks][7];
+  unsigned arrived;
+};
+
+int box_blocks(size_t n) { return (int)std::min<size_t>(kBoxBlocks, std::max<size_t>(1, (n + kThreads - 1) / kThreads)); }
+
+// Block reduction of a KeyBox into r[7] (thread 0).
+__device__ __forceinline__ void block_box(KeyBox& b, long long* r) {
+  __shared__ long long s_mn[3][kThreads / 32], s_mx[3][kThreads / 32];
+  __shared__ int s_bad[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     for (int o = 16; o > 0; o >>= 1) {
-      long long y = __shfl_xor_sync(0xffffffffu, mn[a], o);
-      long long z = __shfl_xor_sync(0xffffffffu, mx[a], o);
-      mn[a] = y < mn[a] ? y : mn[a];
-      mx[a] = z > mx[a] ? z : mx[a];
+      const long long y = __shfl_xor_sync(0xffffffffu, b.mn[a], o);
+      const long long z = __shfl_xor_sync(0xffffffffu, b.mx[a], o);
+      b.mn[a] = y < b.mn[a] ? y : b.mn[a];
+      b.mx[a] = z > b.mx[a] ? z : b.mx[a];
+    }
+    if (lane == 0) {
+      s_mn[a][warp] = b.mn[a];
+      s_mx[a][warp] = b.mx[a];
     }
   }
-  bad = __any_sync(0xffffffffu, bad);
-  if ((threadIdx.x & 31) == 0) {
+  b.bad = __any_sync(0xffffffffu, b.bad);
+  if (lane == 0) s_bad[warp] = b.bad;
+  __syncthreads();
+  if (threadIdx.x == 0) {
     for (int a = 0; a < 3; ++a) {
-      if (mn[a] != LLONG_MAX) atomicMin(&out[a], mn[a]);
-      if (mx[a] != LLONG_MIN) atomicMax(&out[3 + a], mx[a]);
+      r[a] = LLONG_MAX;
+      r[3 + a] = LLONG_MIN;
     }
-    if (bad) atomicMax(&out[6], 1ll);
+    r[6] = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      for (int a = 0; a < 3; ++a) {
+        r[a] = s_mn[a][w] < r[a] ? s_mn[a][w] : r[a];
+        r[3 + a] = s_mx[a][w] > r[3 + a] ? s_mx[a][w] : r[3 + a];
+      }
+      r[6] |= s_bad[w];
+    }
   }
+}
+
+// Every block's box into the scratch; the last block to arrive combines them
+// into host memory (mapped), so a launch and a stream wait give the box (one
+// atomic per block: warps adding to seven words with 64-bit atomics took 40 us
+// at a million particles).
+__device__ __forceinline__ void finish_box(KeyBox& b, BoxScratch* sc, long long* out) {
+  __shared__ unsigned s_last;
+  long long r[7];
+  block_box(b, r);
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 7; ++k) sc->part[blockIdx.x][k] = r[k];
+    __threadfence();
+    s_last = atomicAdd(&sc->arrived, 1u) == gridDim.x - 1u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  KeyBox t;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
+    const volatile long long* v = sc->part[q];
+    for (int a = 0; a < 3; ++a) {
+      t.mn[a] = v[a] < t.mn[a] ? v[a] : t.mn[a];
+      t.mx[a] = v[3 + a] > t.mx[a] ? v[3 + a] : t.mx[a];
+    }
+    t.bad |= (int)v[6];
+  }
+  block_box(t, r);
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 7; ++k) out[k] = r[k];
+    sc->arrived = 0;
+    __threadfence_system();
+  }
+}
+
+// The box of n interleaved positions (kThreads threads, at most kBoxBlocks blocks).
+__global__ void __launch_bounds__(kThreads) k_key_bbox(int n, const double* __restrict__ pos3, double inv,
+                                                       BoxScratch* sc, long long* out) {
+  KeyBox b;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) b.add(a, pos3[3 * (size_t)i + a], inv);
+  }
+  finish_box(b, sc, out);
 }
 
 // Scene of every slot from its insertion index: the scene whose insertion
@@ -145,58 +214,22 @@ __global__ void k_scene_of_id(int n, const uint32_t* __restrict__ id, const uint
   scene[s] = (uint16_t)lo;
 }
 
-// Cell-key bounding box of each scene's finite positions (interleaved xyz,
-// insertion order): one block per scene, out[7 s ..] = min xyz, max xyz,
-// non-finite flag.
+// Cell-key bounding box of a slice of each scene's finite positions
+// (interleaved xyz, insertion order): block (scene, slice) writes
+// out[7 (slices scene + slice) ..] = min xyz, max xyz, non-finite flag.
 __global__ void __launch_bounds__(kThreads) k_scene_bbox(const double* __restrict__ pos3,
                                                          const uint32_t* __restrict__ pbase, double inv,
                                                          long long* __restrict__ out) {
   const int sc = blockIdx.x;
-  long long mn[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, mx[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
-  int bad = 0;
-  for (uint32_t i = pbase[sc] + threadIdx.x; i < pbase[sc + 1]; i += kThreads) {
+  KeyBox b;
+  for (uint32_t i = pbase[sc] + blockIdx.y * kThreads + threadIdx.x; i < pbase[sc + 1]; i += gridDim.y * kThreads) {
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double x = pos3[3 * (size_t)i + a];
-      if (!isfinite(x)) {
-        bad = 1;
-        continue;
-      }
-      const long long k = key_axis(x, inv);
-      mn[a] = k < mn[a] ? k : mn[a];
-      mx[a] = k > mx[a] ? k : mx[a];
-    }
+    for (int a = 0; a < 3; ++a) b.add(a, pos3[3 * (size_t)i + a], inv);
   }
-  __shared__ long long s_mn[3][kThreads / 32], s_mx[3][kThreads / 32];
-  __shared__ int s_bad[kThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long y = __shfl_xor_sync(0xffffffffu, mn[a], o);
-      const long long z = __shfl_xor_sync(0xffffffffu, mx[a], o);
-      mn[a] = y < mn[a] ? y : mn[a];
-      mx[a] = z > mx[a] ? z : mx[a];
-    }
-    if (lane == 0) {
-      s_mn[a][warp] = mn[a];
-      s_mx[a][warp] = mx[a];
-    }
-  }
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) s_bad[warp] = bad;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    long long r[7] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MIN, LLONG_MIN, LLONG_MIN, 0};
-    for (int w = 0; w < kThreads / 32; ++w) {
-      for (int a = 0; a < 3; ++a) {
-        r[a] = s_mn[a][w] < r[a] ? s_mn[a][w] : r[a];
-        r[3 + a] = s_mx[a][w] > r[3 + a] ? s_mx[a][w] : r[3 + a];
-      }
-      r[6] |= s_bad[w];
-    }
-    for (int k = 0; k < 7; ++k) out[7 * sc + k] = r[k];
-  }
+  long long r[7];
+  block_box(b, r);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 7; ++k) out[7 * ((size_t)sc * gridDim.y + blockIdx.y) + k] = r[k];
 }
 
 // One recorded step of the adjoint tape: every per-particle array of the
@@ -421,7 +454,8 @@ FluidWorld::~FluidWorld() {
   if (stream_) cudaStreamSynchronize(stream_);
   drop_graphs();
   free_all();
-  dfree(d_bbox_);
+  if (d_bbox_) cudaFree(d_bbox_);
+  if (h_bbox_) cudaFreeHost(h_bbox_);
   dfree(d_couple_);
   couple_scratch_.release();
   dfree(d_heat_);
@@ -655,16 +689,19 @@ void FluidWorld::grow_box_with_positions(size_t n, const double* pos3) {
 // (interleaved xyz), through a reduction kernel and one small readback.
 void FluidWorld::grow_box_with_device_positions(size_t n, const double* d_pos3) {
   if (n == 0) return;
-  if (!d_bbox_) dalloc(d_bbox_, 7);
-  long long init[7] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MIN, LLONG_MIN, LLONG_MIN, 0};
-  long long res[7];
-  cuda_check(cudaMemcpyAsync(d_bbox_, init, sizeof(init), cudaMemcpyHostToDevice, stream_), "bbox init");
-  int blocks = (int)std::min<size_t>(148 * 8, (n + kThreads - 1) / kThreads);
-  k_key_bbox<<<std::max(blocks, 1), kThreads, 0, stream_>>>((int)n, d_pos3, 1.0 / h0_, d_bbox_);
+  ensure_box_scratch();
+  k_key_bbox<<<box_blocks(n), kThreads, 0, stream_>>>((int)n, d_pos3, 1.0 / h0_, static_cast<BoxScratch*>(d_bbox_),
+                                                      h_bbox_);
   cuda_check(cudaGetLastError(), "bbox kernel");
-  cuda_check(cudaMemcpyAsync(res, d_bbox_, sizeof(res), cudaMemcpyDeviceToHost, stream_), "bbox read");
   cuda_check(cudaStreamSynchronize(stream_), "bbox sync");
-  merge_box(res, res + 3, res[6] != 0);
+  merge_box(h_bbox_, h_bbox_ + 3, h_bbox_[6] != 0);
+}
+
+void FluidWorld::ensure_box_scratch() {
+  if (d_bbox_) return;
+  cuda_check(cudaMallocHost((void**)&h_bbox_, 7 * sizeof(long long)), "cudaMallocHost");
+  cuda_check(cudaMalloc(&d_bbox_, sizeof(BoxScratch)), "cudaMalloc");
+  cuda_check(cudaMemsetAsync(&static_cast<BoxScratch*>(d_bbox_)->arrived, 0, sizeof(unsigned), stream_), "memset");
 }
 
 // Merges a key range into the box (throws, leaving the box unchanged, when
@@ -951,22 +988,39 @@ void FluidWorld::add_particles(size_t m, const double* pos, const double* vel, c
   cuda_check(cudaStreamSynchronize(stream_), "append sync");
 }
 
-// Device-side twin of k_append for set_particles_device: material as u32.
-__global__ void k_load_dev(int m, const double* __restrict__ pos, const double* __restrict__ vel,
-                           const double* __restrict__ mass, const uint32_t* __restrict__ material, double* px,
-                           double* py, double* pz, double* vx, double* vy, double* vz, double* ms, uint32_t* mat,
-                           uint32_t* id) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  px[k] = pos[3 * (size_t)k];
-  py[k] = pos[3 * (size_t)k + 1];
-  pz[k] = pos[3 * (size_t)k + 2];
-  vx[k] = vel ? vel[3 * (size_t)k] : 0.0;
-  vy[k] = vel ? vel[3 * (size_t)k + 1] : 0.0;
-  vz[k] = vel ? vel[3 * (size_t)k + 2] : 0.0;
-  ms[k] = mass[k];
-  mat[k] = material ? material[k] : 0u;
-  id[k] = (uint32_t)k;
+// Loads a caller's device particles (set_particles_device) in one pass: the
+// state with insertion indices, Particle::new's zero outputs (acc, rho, p,
+// mu_eff, xsph, body_acc; particle.rs:50-63), and the positions' cell-key box.
+struct LoadArgs {
+  const double* pos;
+  const double* vel;  // nullable
+  const double* mass;
+  const uint32_t* material;  // nullable
+  double* pv[6];
+  double* ms;
+  uint32_t* mat;
+  uint32_t* id;
+  double* zero[12];
+  int n_zero;
+};
+__global__ void __launch_bounds__(kThreads) k_load_dev(int m, LoadArgs l, double inv, BoxScratch* sc, long long* out) {
+  KeyBox b;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double x = l.pos[3 * (size_t)k + a];
+      b.add(a, x, inv);
+      l.pv[a][k] = x;
+      l.pv[3 + a][k] = l.vel ? l.vel[3 * (size_t)k + a] : 0.0;
+    }
+    l.ms[k] = l.mass[k];
+    l.mat[k] = l.material ? l.material[k] : 0u;
+    l.id[k] = (uint32_t)k;
+#pragma unroll
+    for (int q = 0; q < 12; ++q)
+      if (q < l.n_zero) l.zero[q][k] = 0.0;
+  }
+  finish_box(b, sc, out);
 }
 
 void FluidWorld::set_particles_device(size_t m, const double* pos, const double* vel, const double* mass,
@@ -978,27 +1032,27 @@ void FluidWorld::set_particles_device(size_t m, const double* pos, const double*
   n_ = 0;
   if (m == 0) return;
   ensure_capacity(m);
-  // The positions, read from the caller's device buffer, may widen the grid box.
-  cuda_check(cudaMemcpyAsync(b_.stage, pos, 3 * m * sizeof(double), cudaMemcpyDeviceToDevice, stream_),
-             "set_particles_device positions");
-  grow_box_with_device_positions(m, b_.stage);
+  ensure_box_scratch();
   ParticleConsts& pc = b_.pc[b_.cur];
-  k_load_dev<<<grid_for(m), kThreads, 0, stream_>>>((int)m, pos, vel, mass, material, b_.pv1[0], b_.pv1[1],
-                                                    b_.pv1[2], b_.pv1[3], b_.pv1[4], b_.pv1[5], pc.mass, pc.mat,
-                                                    pc.id);
-  // Particle::new: acc, rho, p, mu_eff, xsph, body_acc start at zero (particle.rs:50-63).
-  const size_t bytes = m * sizeof(double);
-  cuda_check(cudaMemsetAsync(b_.rho, 0, bytes, stream_), "memset");
-  cuda_check(cudaMemsetAsync(b_.p, 0, bytes, stream_), "memset");
-  cuda_check(cudaMemsetAsync(b_.mu, 0, bytes, stream_), "memset");
-  for (int k = 0; k < 3; ++k) {
-    cuda_check(cudaMemsetAsync(b_.acc[k], 0, bytes, stream_), "memset");
-    cuda_check(cudaMemsetAsync(b_.xsph[k], 0, bytes, stream_), "memset");
-    if (b_.has_ba) cuda_check(cudaMemsetAsync(pc.ba[k], 0, bytes, stream_), "memset");
-  }
+  LoadArgs l{};
+  l.pos = pos;
+  l.vel = vel;
+  l.mass = mass;
+  l.material = material;
+  for (int k = 0; k < 6; ++k) l.pv[k] = b_.pv1[k];
+  l.ms = pc.mass;
+  l.mat = pc.mat;
+  l.id = pc.id;
+  for (double* z : {b_.rho, b_.p, b_.mu, b_.acc[0], b_.acc[1], b_.acc[2], b_.xsph[0], b_.xsph[1], b_.xsph[2]})
+    l.zero[l.n_zero++] = z;
+  if (b_.has_ba)
+    for (int k = 0; k < 3; ++k) l.zero[l.n_zero++] = pc.ba[k];
+  k_load_dev<<<box_blocks(m), kThreads, 0, stream_>>>((int)m, l, 1.0 / h0_, static_cast<BoxScratch*>(d_bbox_), h_bbox_);
   cuda_check(cudaGetLastError(), "set_particles_device kernel");
-  n_ = m;
   cuda_check(cudaStreamSynchronize(stream_), "set_particles_device sync");
+  // The positions may widen the grid box (a failure leaves the world empty).
+  merge_box(h_bbox_, h_bbox_ + 3, h_bbox_[6] != 0);
+  n_ = m;
 }
 
 void FluidWorld::get_field_device(int field, double* out) {
@@ -1395,13 +1449,29 @@ void FluidWorld::set_scenes(const std::vector<uint64_t>& counts, const std::vect
 // when the boxes would exceed the cell cap.
 void FluidWorld::grow_scene_boxes(const double* d_pos3) {
   const int ns = (int)scenes_.size();
-  dalloc(d_scene_bbox_, 7 * (size_t)ns);
-  k_scene_bbox<<<ns, kThreads, 0, stream_>>>(d_pos3, d_pbase_, 1.0 / h0_, d_scene_bbox_);
+  // A few slices per scene keep every SM busy with few scenes.
+  const int slices = std::max(1, std::min(32, 1184 / ns));
+  const size_t words = 7 * (size_t)ns * slices;
+  if (words > scene_bbox_cap_) {
+    dalloc(d_scene_bbox_, words);
+    scene_bbox_cap_ = words;
+  }
+  k_scene_bbox<<<dim3((unsigned)ns, (unsigned)slices), kThreads, 0, stream_>>>(d_pos3, d_pbase_, 1.0 / h0_,
+                                                                               d_scene_bbox_);
   cuda_check(cudaGetLastError(), "scene bbox");
-  std::vector<long long> r(7 * (size_t)ns);
-  cuda_check(cudaMemcpyAsync(r.data(), d_scene_bbox_, r.size() * sizeof(long long), cudaMemcpyDeviceToHost, stream_),
+  std::vector<long long> part(words), r(7 * (size_t)ns);
+  cuda_check(cudaMemcpyAsync(part.data(), d_scene_bbox_, words * sizeof(long long), cudaMemcpyDeviceToHost, stream_),
              "scene bbox read");
   cuda_check(cudaStreamSynchronize(stream_), "scene bbox sync");
+  for (int s = 0; s < ns; ++s)
+    for (int k = 0; k < 7; ++k) {
+      long long v = part[7 * (size_t)s * slices + k];
+      for (int q = 1; q < slices; ++q) {
+        const long long u = part[7 * ((size_t)s * slices + q) + k];
+        v = k < 3 ? std::min(v, u) : k < 6 ? std::max(v, u) : (v | u);
+      }
+      r[7 * (size_t)s + k] = v;
+    }
   std::vector<Scene> sc = scenes_;
   long double total = 0;
   for (int s = 0; s < ns; ++s) {

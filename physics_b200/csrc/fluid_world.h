@@ -253,7 +253,9 @@ class FluidWorld {
   void collect_phase_times();
   double phase_ms_[4] = {0, 0, 0, 0};
   double timed_steps_ = 0;
-  long long* d_bbox_ = nullptr;  // 7 values: min xyz, max xyz, non-finite flag
+  void* d_bbox_ = nullptr;       // partial key boxes (BoxScratch)
+  long long* h_bbox_ = nullptr;  // mapped host memory: min xyz, max xyz, non-finite flag
+  void ensure_box_scratch();
   // Point records of couple_points (10 doubles each) plus one word of flags.
   double* d_couple_ = nullptr;
   CouplePointsScratch couple_scratch_;
@@ -276,6 +278,7 @@ class FluidWorld {
   int boxes_capacity_ = 0;
   uint32_t* d_pbase_ = nullptr;
   long long* d_scene_bbox_ = nullptr;
+  size_t scene_bbox_cap_ = 0;
   LaunchTuning tuning_;
   // CUDA graphs of step chunks, keyed by everything a captured launch bakes in.
   struct GraphEntry {
