@@ -463,7 +463,7 @@ FluidWorld::~FluidWorld() {
   dfree(d_pbase_);
   dfree(d_scene_bbox_);
   release_snapshot();
-  tape_clear();
+  tape_free();
   for (auto& set : ev_pool_)
     for (auto& e : set) cudaEventDestroy(e);
   if (own_stream_) cudaStreamDestroy(own_stream_);
@@ -479,6 +479,7 @@ void FluidWorld::free_all() {
     dfree(b_.pc[q].mat);
     dfree(b_.pc[q].id);
     dfree(b_.pc[q].scene);
+    dfree(scene_keep_[q]);
     for (int k = 0; k < 3; ++k) dfree(b_.pc[q].ba[k]);
   }
   dfree(b_.rho);
@@ -544,6 +545,8 @@ void FluidWorld::ensure_capacity(size_t n) {
   if (n >= (1ull << (32 - kCodeBits)))
     throw std::invalid_argument("FluidWorld: more than 2^27 particles in one subsystem");
   if ((int)n <= b_.capacity) return;
+  if (!tape_.on && tape_.n) tape_free();
+  for (auto& p : scene_keep_) dfree(p);
   size_t cap = std::max<size_t>(n, (size_t)b_.capacity + b_.capacity / 2);
   cudaStream_t s = stream_;
   for (int k = 0; k < 6; ++k) {
@@ -1030,6 +1033,7 @@ void FluidWorld::set_particles_device(size_t m, const double* pos, const double*
   if (tape_.on) throw std::invalid_argument("set_particles_device: the adjoint tape is recording");
   if (m > (size_t)INT32_MAX) throw std::invalid_argument("set_particles_device: too many particles");
   n_ = 0;
+  if (tape_.n && tape_.n != m) tape_free();
   if (m == 0) return;
   ensure_capacity(m);
   ensure_box_scratch();
@@ -1424,11 +1428,19 @@ void FluidWorld::set_scenes(const std::vector<uint64_t>& counts, const std::vect
   }
   pbase[counts.size()] = (uint32_t)first;
   cuda_check(cudaStreamSynchronize(stream_), "scenes sync");
-  dalloc(d_pbase_, pbase.size());
+  if (pbase.size() > pbase_cap_) {
+    dalloc(d_pbase_, pbase.size());
+    pbase_cap_ = pbase.size();
+  }
   cuda_check(cudaMemcpy(d_pbase_, pbase.data(), pbase.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
              "pbase upload");
   for (int q = 0; q < 2; ++q)
-    if (!b_.pc[q].scene) dalloc(b_.pc[q].scene, (size_t)std::max(b_.capacity, 1));
+    if (!b_.pc[q].scene) {
+      if (scene_keep_[q])
+        std::swap(scene_keep_[q], b_.pc[q].scene);
+      else
+        dalloc(b_.pc[q].scene, (size_t)std::max(b_.capacity, 1));
+    }
   ++alloc_gen_;
   if (n_ > 0)
     k_scene_of_id<<<grid_for(n_), kThreads, 0, stream_>>>((int)n_, b_.pc[b_.cur].id, d_pbase_, (int)counts.size(),
@@ -1493,7 +1505,13 @@ void FluidWorld::grow_scene_boxes(const double* d_pos3) {
 void FluidWorld::clear_scenes() {
   scenes_.clear();
   host_boxes_.clear();
-  for (int q = 0; q < 2; ++q) dfree(b_.pc[q].scene);
+  // The arrays stay for the next set of scenes (a null pointer in the
+  // constants means a single scene).
+  for (int q = 0; q < 2; ++q)
+    if (b_.pc[q].scene) {
+      dfree(scene_keep_[q]);
+      std::swap(scene_keep_[q], b_.pc[q].scene);
+    }
   ++alloc_gen_;
 }
 
@@ -1961,7 +1979,24 @@ void FluidWorld::save_checkpoint() {
   ++tape_.nckpt;
 }
 
+// Ends the tape.  Its buffers stay for the next tape of the same size while
+// they are small (an optimisation loop clears and begins a tape every
+// iteration; allocating and freeing them took two thirds of it at 65,536
+// particles); they go with the world or when its particle count changes.
 void FluidWorld::tape_clear() {
+  constexpr size_t kKeepBytes = size_t(1) << 30;
+  tape_.nckpt = 0;
+  tape_.dts.clear();
+  tape_.on = false;
+  size_t bytes = (6 * tape_.ckpt.size() + 22 * adj_slot_f_.size() + (adj_work_ ? 30 : 0)) * tape_.n * sizeof(double) +
+                 comp_rec_cap_ * sizeof(uint32_t);
+  for (size_t u : adj_slot_ucount_) bytes += u * sizeof(uint32_t);
+  for (size_t q : snap_bytes_) bytes += q;
+  if (bytes > kKeepBytes) tape_free();
+  for (auto& c : snap_count_) c = 0;  // the saved states are void
+}
+
+void FluidWorld::tape_free() {
   for (auto& p : tape_.ckpt) dfree(p);
   tape_.ckpt.clear();
   tape_.nckpt = 0;
@@ -1987,7 +2022,7 @@ void FluidWorld::tape_begin(int every) {
   if (every < 1) throw std::invalid_argument("tape_begin: checkpoint interval must be >= 1");
   if (n_ == 0) throw std::invalid_argument("tape_begin: empty world");
   // Checkpoint and sweep buffers are kept for the next tape of the same size.
-  if (tape_.n != n_) tape_clear();
+  if (tape_.n != n_) tape_free();
   tape_.n = n_;
   tape_.nckpt = 0;
   tape_.dts.clear();

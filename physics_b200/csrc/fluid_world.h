@@ -278,7 +278,8 @@ class FluidWorld {
   int boxes_capacity_ = 0;
   uint32_t* d_pbase_ = nullptr;
   long long* d_scene_bbox_ = nullptr;
-  size_t scene_bbox_cap_ = 0;
+  size_t scene_bbox_cap_ = 0, pbase_cap_ = 0;
+  uint16_t* scene_keep_[2] = {};  // scene arrays of cleared scenes
   LaunchTuning tuning_;
   // CUDA graphs of step chunks, keyed by everything a captured launch bakes in.
   struct GraphEntry {
@@ -299,7 +300,8 @@ class FluidWorld {
     size_t nckpt = 0;
     PhySphParams params;
   } tape_;
-  // Reverse-sweep buffers kept between sweeps (freed by tape_clear).
+  void tape_free();
+  // Reverse-sweep buffers kept between sweeps and tapes (tape_clear).
   double* adj_work_ = nullptr;
   uint32_t* comp_rec_ = nullptr;  // compensated adjoint: insertion index -> recorded slot
   size_t comp_rec_cap_ = 0;
