@@ -179,6 +179,17 @@ __device__ __forceinline__ uint32_t first_outside(const TiledArgs& a) {
   return (a.flags[0] & kFlagSortLost) ? 0u : a.tile_slot[0];
 }
 
+// Work items per tile: a world of few tiles splits each into x-slabs (the
+// slabs a tile with a large halo runs in), so that its queries spread over
+// more SMs; one CTA took 31 us for a tile's ~512 queries however few tiles
+// there were.  Both passes use the same split: list entries are slots of the
+// slab's staging.
+constexpr uint32_t kSplitItems = 2 * 148;
+template <int TB>
+__device__ __forceinline__ uint32_t tile_parts(uint32_t ntiles) {
+  return TB * ntiles <= kSplitItems ? (uint32_t)TB : (TB == 4 && 2u * ntiles <= kSplitItems) ? 2u : 1u;
+}
+
 struct TileGeom {
   int tx, ty, tz;  // tile coordinates inside the scene box
   int sc;          // scene
@@ -461,16 +472,22 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
   __shared__ uint32_t s_next;
   const uint32_t ntiles = occupied_tiles(a);
   unsigned cand = 0, pairs = 0;
-  for (uint32_t k = next_tile(a.queue, 0, blockIdx.x, &s_next); k < ntiles;
-       k = next_tile(a.queue, 0, k + gridDim.x, &s_next)) {
+  const uint32_t parts = tile_parts<TB>(ntiles);
+  const int layers = T::B / (int)parts;
+  for (uint32_t item = next_tile(a.queue, 0, blockIdx.x, &s_next); item < ntiles * parts;
+       item = next_tile(a.queue, 0, item + gridDim.x, &s_next)) {
+    const uint32_t k = item / parts;
+    const int xa = (int)(item % parts) * layers;
     const TileGeom g = tile_geom<TB>(c, a, k);
     halo_table<TB>(c, a, g, s_src, s_end, s_off, ws);
-    const int slab = a.tile_crowd[k] ? 0 : pick_slab<TB>(s_off, (uint32_t)min(c.halo_cap, kHaloCap));
-    if (slab == 0) {
-      queue_dense_tasks<TB>(a, g, ws, s_src, &s_next);
+    const int fit = a.tile_crowd[k] ? 0 : pick_slab<TB>(s_off, (uint32_t)min(c.halo_cap, kHaloCap));
+    if (fit == 0) {
+      if (xa == 0) queue_dense_tasks<TB>(a, g, ws, s_src, &s_next);
+      else __syncthreads();  // the table is read before the next one is built
       continue;  // uniform across the CTA
     }
-    for (int x0 = 0; x0 < T::B; x0 += slab) {
+    const int slab = min(fit, layers);
+    for (int x0 = xa; x0 < xa + layers; x0 += slab) {
     const uint32_t base = s_off[x0 * T::H * T::H];
     stage_halo<TB>(
         s_src, s_end, s_off, x0 * T::H, (x0 + slab + 2) * T::H, base,
@@ -797,13 +814,21 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
   const float hc2 = fminf(c.h2f, c.h0sqf);
   __shared__ uint32_t s_next;
   const uint32_t ntiles = occupied_tiles(a);
-  for (uint32_t k = next_tile(a.queue, 1, blockIdx.x, &s_next); k < ntiles;
-       k = next_tile(a.queue, 1, k + gridDim.x, &s_next)) {
+  const uint32_t parts = tile_parts<TB>(ntiles);
+  const int layers = T::B / (int)parts;
+  for (uint32_t item = next_tile(a.queue, 1, blockIdx.x, &s_next); item < ntiles * parts;
+       item = next_tile(a.queue, 1, item + gridDim.x, &s_next)) {
+    const uint32_t k = item / parts;
+    const int xa = (int)(item % parts) * layers;
     const TileGeom g = tile_geom<TB>(c, a, k);
     halo_table<TB>(c, a, g, s_src, s_end, s_off, ws);
-    const int slab = a.tile_crowd[k] ? 0 : pick_slab<TB>(s_off, (uint32_t)min(c.halo_cap, kHaloCap));
-    if (slab == 0) continue;  // the dense-cell pass computes this tile
-    for (int x0 = 0; x0 < T::B; x0 += slab) {
+    const int fit = a.tile_crowd[k] ? 0 : pick_slab<TB>(s_off, (uint32_t)min(c.halo_cap, kHaloCap));
+    if (fit == 0) {
+      __syncthreads();  // the table is read before the next one is built
+      continue;  // the dense-cell pass computes this tile
+    }
+    const int slab = min(fit, layers);
+    for (int x0 = xa; x0 < xa + layers; x0 += slab) {
     const uint32_t base = s_off[x0 * T::H * T::H];
     stage_halo<TB>(
         s_src, s_end, s_off, x0 * T::H, (x0 + slab + 2) * T::H, base,
