@@ -13,16 +13,15 @@
 //     samples (world.rs:702-751);
 //   * a point outside the bounds is skipped and its force left unwritten.
 //
-// One CTA walks the points in order.  Per point, its candidates are staged
-// through shared memory and summed in visit order by one thread (the
-// reference's sequential sums); the reaction is then applied in parallel
-// (every fluid particle lies in one cell, so the updates are disjoint).
-// Consecutive points whose neighbourhoods are pairwise disjoint run at once,
-// one warp each (k_couple_points_grouped); k_couple_points is the one-point-
-// at-a-time form, used when the grouped walk's shared memory is unavailable.
+// Per point, its candidates are staged through shared memory and summed in
+// visit order by one lane (the reference's sequential sums); the reaction is
+// then applied in parallel (every fluid particle lies in one cell, so the
+// updates are disjoint).  Points whose neighbourhoods overlap keep their
+// order, the others run at once (k_couple_points_flow).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <stdexcept>
 #include <vector>
 
 #include "sph_buffers.h"
@@ -31,8 +30,7 @@ namespace phy {
 
 namespace {
 
-constexpr int kCT = 256;        // threads of the coupling CTA
-constexpr int kCChunk = 1024;   // candidates staged per chunk
+constexpr int kCT = 256;        // threads per block
 
 struct CoupleArgs {
   const uint32_t* cell_start;
@@ -81,109 +79,33 @@ __device__ __forceinline__ void point_force(const StepConsts& c, const CoupleArg
   r[3] = sw;
 }
 
-__global__ void __launch_bounds__(kCT) k_couple_points(StepConsts c, CoupleArgs a) {
-  __shared__ uint32_t s_beg[27];
-  __shared__ uint32_t s_pre[28];
-  __shared__ double s_v[3][kCChunk];
-  __shared__ double s_m[kCChunk];
-  __shared__ double s_r[4];  // reaction xyz, sum of masses
-  __shared__ int s_in;
-  const int t = threadIdx.x;
-  for (int k = 0; k < a.np; ++k) {
-    double* q = a.pts + 10 * (size_t)k;
-    if (t < 32) {
-      // Warp 0: lane u < 27 reads cell u of the visit order (u = 9 (di+1) +
-      // 3 (dj+1) + (dk+1)); a shuffle scan gives the cells' first candidates.
-      const double x = q[0], y = q[1], z = q[2];
-      // world.rs:704-711 (a NaN coordinate passes, as there).
-      const bool in = !(x < c.lo[0] || x > c.hi[0] || y < c.lo[1] || y > c.hi[1] || z < c.lo[2] || z > c.hi[2]);
-      if (t == 0) s_in = in ? 1 : 0;
-      if (in) {
-        const long long kx = key_axis(x, c.inv_cell), ky = key_axis(y, c.inv_cell), kz = key_axis(z, c.inv_cell);
-        uint32_t beg = 0, cnt = 0;
-        if (t < 27) {
-          const int lin = cell_linear(c, kx + t / 9 - 1, ky + (t / 3) % 3 - 1, kz + t % 3 - 1);
-          if (lin >= 0) {
-            beg = a.cell_start[lin];
-            cnt = a.cell_start[lin + 1] - beg;
-          }
-        }
-        uint32_t incl = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (t >= o) incl += y;
-        }
-        if (t < 27) {
-          s_beg[t] = beg;
-          s_pre[t] = incl - cnt;
-        }
-        if (t == 26) s_pre[27] = incl;
-      }
-    }
-    __syncthreads();
-    if (!s_in) {
-      __syncthreads();  // every thread has read s_in before thread 0 rewrites it
-      continue;
-    }
-    const uint32_t total = s_pre[27];
-    double sx = 0.0, sy = 0.0, sz = 0.0, sw = 0.0;  // thread 0's sums
-    for (uint32_t base = 0; base < total; base += kCChunk) {
-      const uint32_t m = min((uint32_t)kCChunk, total - base);
-      for (uint32_t e = t; e < m; e += kCT) {
-        const uint32_t i = candidate(a, s_beg, s_pre, base + e);
-        s_v[0][e] = a.vx[i];
-        s_v[1][e] = a.vy[i];
-        s_v[2][e] = a.vz[i];
-        s_m[e] = a.mass[i];
-      }
-      __syncthreads();
-      if (t == 0)
-        for (uint32_t e = 0; e < m; ++e) {
-          const double w = s_m[e];
-          sx = sx + s_v[0][e] * w;
-          sy = sy + s_v[1][e] * w;
-          sz = sz + s_v[2][e] * w;
-          sw = sw + w;
-        }
-      __syncthreads();
-    }
-    if (t == 0) point_force(c, a, q, sx, sy, sz, sw, s_r);
-    __syncthreads();
-    const double msum = s_r[3];
-    if (msum > 0.0)
-      for (uint32_t flat = t; flat < total; flat += kCT) {
-        const uint32_t i = candidate(a, s_beg, s_pre, flat);
-        const double frac = a.mass[i] / msum;
-        a.vx[i] = a.vx[i] + s_r[0] * frac;
-        a.vy[i] = a.vy[i] + s_r[1] * frac;
-        a.vz[i] = a.vz[i] + s_r[2] * frac;
-      }
-    __syncthreads();
-  }
-}
-
-// Grouped form of the same walk.  Only velocities change from one point to
-// the next, so everything else is prepared in parallel first: one warp per
-// point finds its 27 cell ranges and whether its neighbourhood overlaps those
-// of the kGW - 1 points before it (k_point_tables), and, after a prefix sum
-// of the candidate counts, writes its candidates' particle indices and masses
-// in visit order (k_point_candidates).  Two points whose centre cells are
-// more than 2 apart on some axis have disjoint 27-cell neighbourhoods, so
-// they read and write disjoint particles: a run of consecutive points that
-// are pairwise disjoint (a group) gives the same velocities and forces
-// whether its points run one after another or at once.  The walk (one CTA)
-// takes the groups in order and runs a group's points at once, one warp
-// each: the lanes stage the candidates' products v_j m_j in the warp's
-// shared buffer (the same f64 products), lane 0 adds them in visit order
-// (the reference's sequential sums), and the lanes apply the reaction to the
-// candidates they hold (v_j + share, with the velocities they gathered).
-// Points with more than kPB candidates have no list and read their
-// candidates through their cell table.
-constexpr int kGW = 16;         // warps of the walk: points per group at most
+// The points' walk.  Only velocities change from one point to the
+// next, so everything else is prepared in parallel first: one warp per point
+// finds its 27 cell ranges and centre cell (k_point_tables), and, after a
+// prefix sum of the candidate counts, writes its candidates' particle indices
+// and masses in visit order (k_point_candidates).  Two points whose centre
+// cells are more than 2 apart on some axis have disjoint 27-cell
+// neighbourhoods, so they read and write disjoint particles and give the same
+// velocities and forces in any order; only overlapping points must keep
+// theirs.  The walk takes the points in order, one warp each over the whole
+// GPU, and a warp waits for the earlier points that overlap its own
+// (k_couple_points_flow): the time is that of the longest chain of overlaps
+// instead of the number of points (400 points in 32,805 particles: 622 us while
+// one CTA took runs of up to 16 disjoint neighbours).  A warp stages its
+// candidates' products v_j m_j in its shared buffer (the same f64 products),
+// lane 0 adds them in visit order (the reference's sequential sums), and the
+// lanes apply the reaction to the candidates they hold (v_j + share, with the
+// velocities they gathered).  Points with more than kPB candidates have no
+// list and read their candidates through their cell table.
+constexpr int kFW = 4;          // warps per block of the walk
 constexpr int kPer = 8;         // candidates a lane holds per chunk
 constexpr int kWB = 32 * kPer;  // candidates per chunk of a warp
 constexpr int kPB = 4096;       // candidates a point may have for a list
 constexpr int kTabU = 56;       // u32 per point table: in, total, beg[27], cnt[27]
+
+// The walk's words: ticket, error flag (two words, kFlowHead in all), then a
+// done flag per point.
+constexpr int kFlowHead = 2;
 
 // world.rs:704-711 (a NaN coordinate passes, as there).
 __device__ __forceinline__ bool point_in(const StepConsts& c, const double* q) {
@@ -192,11 +114,15 @@ __device__ __forceinline__ bool point_in(const StepConsts& c, const double* q) {
 }
 
 // One warp per point w of the batch: in-bounds flag, candidate count and
-// cell ranges, and conf[w]: bit m (1 <= m < kGW) when the neighbourhood of
-// point w overlaps that of point w - m (both in bounds, centre cells at most
-// 2 apart on every axis).
+// cell ranges, and key[w]: the centre cell in box coordinates (clamped far
+// outside the box, where a false overlap only costs a wait) and the in-bounds
+// flag.  Also clears the walk's done flags and ticket.
+__device__ __forceinline__ int box_coord(long long k, long long b0) {
+  const long long d = k - b0, far = 1ll << 28;
+  return (int)(d < -far ? -far : d > far ? far : d);
+}
 __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a, int nb, uint32_t* tab,
-                                                      uint32_t* totals, uint16_t* conf) {
+                                                      uint32_t* totals, int4* key, uint32_t* done) {
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= nb) return;
   const double* q = a.pts + 10 * (size_t)w;
@@ -211,16 +137,6 @@ __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a
       cnt = a.cell_start[lin + 1] - beg;
     }
   }
-  bool overlap = false;
-  if (in && lane >= 1 && lane < kGW && w - lane >= 0) {
-    const double* p = a.pts + 10 * (size_t)(w - lane);
-    if (point_in(c, p)) {
-      const long long dx = key_axis(p[0], c.inv_cell) - kx, dy = key_axis(p[1], c.inv_cell) - ky,
-                      dz = key_axis(p[2], c.inv_cell) - kz;
-      overlap = dx >= -2 && dx <= 2 && dy >= -2 && dy <= 2 && dz >= -2 && dz <= 2;
-    }
-  }
-  const uint32_t bits = __ballot_sync(0xffffffffu, overlap);
   const uint32_t total = __reduce_add_sync(0xffffffffu, cnt);
   uint32_t* t = tab + (size_t)w * kTabU;
   if (lane < 27) {
@@ -231,7 +147,9 @@ __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a
     t[0] = in ? 1u : 0u;
     t[1] = total;
     totals[w] = in && total <= (uint32_t)kPB ? total : 0u;
-    conf[w] = (uint16_t)bits;
+    key[w] = make_int4(box_coord(kx, c.bx0), box_coord(ky, c.by0), box_coord(kz, c.bz0), in ? 1 : 0);
+    done[kFlowHead + w] = 0u;
+    if (w < kFlowHead) done[w] = 0u;
   }
 }
 
@@ -239,7 +157,8 @@ __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a
 // order (cell after cell, ascending slot: ascending insertion index), from
 // off[w].
 __global__ void __launch_bounds__(256) k_point_candidates(CoupleArgs a, int nb, const uint32_t* tab,
-                                                          const uint32_t* off, uint32_t* idx, double* m) {
+                                                          const uint32_t* off, uint32_t* idx, double* m,
+                                                          double* msum) {
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= nb) return;
   const uint32_t* t = tab + (size_t)w * kTabU;
@@ -254,6 +173,19 @@ __global__ void __launch_bounds__(256) k_point_candidates(CoupleArgs a, int nb, 
     }
     o += cnt;
   }
+  // The masses' sum in visit order, for the points the walk holds in
+  // registers.
+  const uint32_t total = t[1];
+  if (total <= (uint32_t)kWB) {
+    __syncwarp();
+    if (lane == 0) {
+      const double* p = m + off[w];
+      double sw = 0.0;
+#pragma unroll 8
+      for (uint32_t e = 0; e < total; ++e) sw = sw + p[e];
+      msum[w] = sw;
+    }
+  }
 }
 
 struct PointLists {
@@ -261,7 +193,9 @@ struct PointLists {
   const uint32_t* off;
   const uint32_t* idx;
   const double* m;
-  const uint16_t* conf;
+  const double* msum;
+  const int4* key;
+  uint32_t* flow;  // ticket, error, done flags
 };
 
 // Cell table of a point without a list (its warp's copy).
@@ -270,7 +204,7 @@ struct WarpTable {
   uint32_t pre[28];
 };
 
-// One warp: all of point j's work in the walk.  `pw` is the warp's buffer of
+// One warp: the work of a point of many candidates.  `pw` is the warp's buffer of
 // 2 kWB products, `r` its reaction and mass sum.
 __device__ __forceinline__ void walk_point(const StepConsts& c, const CoupleArgs& a, const PointLists& L, int j,
                                            double2* pw, WarpTable& T, double* r) {
@@ -295,8 +229,6 @@ __device__ __forceinline__ void walk_point(const StepConsts& c, const CoupleArgs
     __syncwarp();
   }
   double sx = 0.0, sy = 0.0, sz = 0.0, sw = 0.0;  // lane 0's sums
-  uint32_t ci[kPer];
-  double cm[kPer], cx[kPer], cy[kPer], cz[kPer];
   for (uint32_t base = 0; base < total; base += kWB) {
     const uint32_t cnt = min((uint32_t)kWB, total - base);
 #pragma unroll
@@ -305,14 +237,10 @@ __device__ __forceinline__ void walk_point(const StepConsts& c, const CoupleArgs
       if (e < cnt) {
         const uint32_t i = listed ? L.idx[o + base + e] : candidate(a, T.beg, T.pre, base + e);
         const double m = listed ? L.m[o + base + e] : a.mass[i];
-        const double vx = a.vx[i], vy = a.vy[i], vz = a.vz[i];
+        // (From L2: another SM may have written them during this launch.)
+        const double vx = __ldcg(a.vx + i), vy = __ldcg(a.vy + i), vz = __ldcg(a.vz + i);
         pw[2 * e] = make_double2(vx * m, vy * m);
         pw[2 * e + 1] = make_double2(vz * m, m);
-        ci[k] = i;
-        cm[k] = m;
-        cx[k] = vx;
-        cy[k] = vy;
-        cz[k] = vz;
       }
     }
     __syncwarp();
@@ -350,60 +278,141 @@ __device__ __forceinline__ void walk_point(const StepConsts& c, const CoupleArgs
   const double msum = r[3];
   if (!(msum > 0.0)) return;
   const double rx = r[0], ry = r[1], rz = r[2];
-  if (total <= (uint32_t)kWB) {
+  for (uint32_t e = lane; e < total; e += 32) {
+    const uint32_t i = listed ? L.idx[o + e] : candidate(a, T.beg, T.pre, e);
+    const double frac = (listed ? L.m[o + e] : a.mass[i]) / msum;
+    a.vx[i] = __ldcg(a.vx + i) + rx * frac;
+    a.vy[i] = __ldcg(a.vy + i) + ry * frac;
+    a.vz[i] = __ldcg(a.vz + i) + rz * frac;
+  }
+}
+
+// A listed point of at most kWB candidates: its indices, masses and mass
+// fractions are loaded before the wait, so that between two overlapping points
+// only the velocities' gather, their ordered sums (three lanes, one component
+// each) and the reaction remain.
+struct HeldPoint {
+  uint32_t ci[kPer];
+  double cm[kPer], frac[kPer];
+  uint32_t total;
+  double msum;
+};
+__device__ __forceinline__ void hold_point(const PointLists& L, int j, uint32_t total, HeldPoint& h) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t o = L.off[j];
+  h.total = total;
+  h.msum = L.msum[j];
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const uint32_t e = (uint32_t)lane + 32u * k;
-      if (e < total) {
-        const double frac = cm[k] / msum;
-        a.vx[ci[k]] = cx[k] + rx * frac;
-        a.vy[ci[k]] = cy[k] + ry * frac;
-        a.vz[ci[k]] = cz[k] + rz * frac;
-      }
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t e = (uint32_t)lane + 32u * k;
+    if (e < total) {
+      h.ci[k] = L.idx[o + e];
+      h.cm[k] = L.m[o + e];
+      h.frac[k] = h.cm[k] / h.msum;
     }
-  } else {
-    for (uint32_t e = lane; e < total; e += 32) {
-      const uint32_t i = listed ? L.idx[o + e] : candidate(a, T.beg, T.pre, e);
-      const double frac = (listed ? L.m[o + e] : a.mass[i]) / msum;
-      a.vx[i] = a.vx[i] + rx * frac;
-      a.vy[i] = a.vy[i] + ry * frac;
-      a.vz[i] = a.vz[i] + rz * frac;
+  }
+}
+__device__ __forceinline__ void walk_held(const StepConsts& c, const CoupleArgs& a, int j, const HeldPoint& h,
+                                          double* pv, double* r) {
+  const int lane = threadIdx.x & 31;
+  double v[kPer][3];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t e = (uint32_t)lane + 32u * k;
+    if (e < h.total) {
+      v[k][0] = __ldcg(a.vx + h.ci[k]);
+      v[k][1] = __ldcg(a.vy + h.ci[k]);
+      v[k][2] = __ldcg(a.vz + h.ci[k]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t e = (uint32_t)lane + 32u * k;
+    if (e < h.total)
+      for (int q = 0; q < 3; ++q) pv[q * kWB + e] = v[k][q] * h.cm[k];
+  }
+  __syncwarp();
+  double sum = 0.0;
+  if (lane < 3) {
+    const double* p = pv + lane * kWB;
+    uint32_t e = 0;
+    for (; e + 8 <= h.total; e += 8) {
+      double t[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) t[u] = p[e + u];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sum = sum + t[u];
+    }
+    for (; e < h.total; ++e) sum = sum + p[e];
+  }
+  const double sx = __shfl_sync(0xffffffffu, sum, 0), sy = __shfl_sync(0xffffffffu, sum, 1),
+               sz = __shfl_sync(0xffffffffu, sum, 2);
+  if (lane == 0) point_force(c, a, a.pts + 10 * (size_t)j, sx, sy, sz, h.msum, r);
+  __syncwarp();
+  if (!(h.msum > 0.0)) return;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t e = (uint32_t)lane + 32u * k;
+    if (e < h.total) {
+      a.vx[h.ci[k]] = v[k][0] + r[0] * h.frac[k];
+      a.vy[h.ci[k]] = v[k][1] + r[1] * h.frac[k];
+      a.vz[h.ci[k]] = v[k][2] + r[2] * h.frac[k];
     }
   }
 }
 
-// The walk over the nb points of a batch: group after group, a group being
-// the longest run (at most kGW) of points after its first whose
-// neighbourhoods overlap none of the run's earlier points.
-__global__ void __launch_bounds__(kGW * 32, 1) k_couple_points_grouped(StepConsts c, CoupleArgs a, int nb,
-                                                                       PointLists L) {
+// The walk over the nb points of a batch.  Warps take points by ticket, in
+// order, so the points a warp waits for are held by running warps (or done)
+// and the wait ends; it gives up after a poll limit all the same, with the
+// error word set and the remaining points unwalked.
+__global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, CoupleArgs a, int nb, PointLists L) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double2* s_pw = reinterpret_cast<double2*>(smem);                    // [kGW][2 kWB]
-  uint16_t* s_conf = reinterpret_cast<uint16_t*>(s_pw + 2 * kWB * kGW);  // [nb]
-  __shared__ WarpTable s_tab[kGW];
-  __shared__ double s_r[kGW][4];
-  __shared__ int s_group;
+  __shared__ WarpTable s_tab[kFW];
+  __shared__ double s_r[kFW][4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int k = threadIdx.x; k < nb; k += kGW * 32) s_conf[k] = L.conf[k];
-  __syncthreads();
-  for (int j = 0; j < nb;) {
-    if (warp == 0) {
-      // Lane l < kGW stops the group before point j + l when that point
-      // overlaps one of j .. j + l - 1 (conf bits 1..l) or is past the batch.
-      bool stop = false;
-      if (lane >= 1 && lane < kGW) stop = j + lane >= nb || (s_conf[j + lane] & ((2u << lane) - 1u)) != 0u;
-      const uint32_t b = __ballot_sync(0xffffffffu, stop) | (1u << kGW);
-      if (lane == 0) s_group = __ffs((int)(b >> 1));
+  double2* pw = reinterpret_cast<double2*>(smem) + (size_t)warp * 2 * kWB;
+  uint32_t* done = L.flow + kFlowHead;
+  for (;;) {
+    uint32_t k = 0;
+    if (lane == 0) k = atomicAdd(L.flow, 1u);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= (uint32_t)nb) return;
+    const int4 own = L.key[k];
+    if (!own.w) continue;  // outside the bounds: skipped, nothing waits for it
+    const uint32_t total = L.tab[(size_t)k * kTabU + 1];
+    const bool held = total <= (uint32_t)kWB;
+    HeldPoint h;
+    if (held) hold_point(L, (int)k, total, h);
+    bool ok = true;
+    for (uint32_t j = (uint32_t)lane; j < k; j += 32u) {
+      const int4 p = L.key[j];
+      const bool overlap = p.w && abs(p.x - own.x) <= 2 && abs(p.y - own.y) <= 2 && abs(p.z - own.z) <= 2;
+      if (!overlap) continue;
+      uint32_t seen = 0;
+      for (int polls = 0; polls < (1 << 22); ++polls) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(done + j) : "memory");
+        if (seen) break;
+        if ((polls & 255) == 255 && *(volatile uint32_t*)(L.flow + 1)) break;
+      }
+      ok = ok && seen != 0u;
     }
-    __syncthreads();
-    const int g = s_group;
-    if (warp < g) walk_point(c, a, L, j + warp, s_pw + (size_t)warp * 2 * kWB, s_tab[warp], s_r[warp]);
-    __syncthreads();  // the group's reactions are applied before the next group gathers
-    j += g;
+    if (!__all_sync(0xffffffffu, ok)) {
+      if (lane == 0) atomicOr(L.flow + 1, 1u);
+      return;
+    }
+    if (held)
+      walk_held(c, a, (int)k, h, reinterpret_cast<double*>(pw), s_r[warp]);
+    else
+      walk_point(c, a, L, (int)k, pw, s_tab[warp], s_r[warp]);
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(done + k), "r"(1u) : "memory");
+    }
   }
 }
 
-constexpr size_t kGroupedSmemFixed = (size_t)kGW * 2 * kWB * sizeof(double2);
+constexpr size_t kFlowSmem = (size_t)kFW * 2 * kWB * sizeof(double2);
 
 // ---- couple_heat (world.rs:555-678) ------------------------------------------------
 //
@@ -1134,15 +1143,16 @@ void scratch_grow(T*& p, size_t& cap, size_t count, cudaStream_t s) {
 }  // namespace
 
 void CouplePointsScratch::release() {
-  for (uint32_t** p : {&tab, &totals, &off, &idx}) {
+  for (uint32_t** p : {&tab, &totals, &off, &idx, &flow}) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
   if (m) cudaFree(m);
-  m = nullptr;
-  if (conf) cudaFree(conf);
-  conf = nullptr;
-  cap_tab = cap_totals = cap_off = cap_idx = cap_m = cap_conf = 0;
+  if (msum) cudaFree(msum);
+  m = msum = nullptr;
+  if (key) cudaFree(key);
+  key = nullptr;
+  cap_tab = cap_totals = cap_off = cap_idx = cap_m = cap_key = cap_flow = cap_msum = 0;
 }
 
 void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int np, double dt, double drag,
@@ -1162,14 +1172,13 @@ void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int
   // Points run in batches (one ordered walk per batch, in order on the
   // stream), which bounds the candidate lists and the walk's shared memory.
   constexpr int kBatch = 16384;
-  static const bool smem_ok = [] {
-    return cudaFuncSetAttribute(k_couple_points_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(kGroupedSmemFixed + kBatch * sizeof(uint16_t))) == cudaSuccess;
+  static const int flow_blocks = [] {
+    int dev = 0, sms = 1, per = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_couple_points_flow, kFW * 32, kFlowSmem);
+    return std::max(sms, 1) * std::max(per, 1);
   }();
-  if (!smem_ok) {
-    k_couple_points<<<1, kCT, 0, s>>>(c, a);
-    return;
-  }
   std::vector<uint32_t> totals, off;
   for (int p0 = 0; p0 < np; p0 += kBatch) {
     const int nb = std::min(kBatch, np - p0);
@@ -1177,9 +1186,10 @@ void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int
     ab.pts = d_pts + 10 * (size_t)p0;
     scratch_grow(sc.tab, sc.cap_tab, (size_t)nb * kTabU, s);
     scratch_grow(sc.totals, sc.cap_totals, (size_t)nb, s);
-    scratch_grow(sc.conf, sc.cap_conf, (size_t)nb, s);
+    scratch_grow(sc.key, sc.cap_key, (size_t)nb, s);
+    scratch_grow(sc.flow, sc.cap_flow, (size_t)nb + kFlowHead, s);
     const int warps_per_block = 256 / 32, blocks = (nb + warps_per_block - 1) / warps_per_block;
-    k_point_tables<<<blocks, 256, 0, s>>>(c, ab, nb, sc.tab, sc.totals, sc.conf);
+    k_point_tables<<<blocks, 256, 0, s>>>(c, ab, nb, sc.tab, sc.totals, sc.key, sc.flow);
     cuda_check(cudaGetLastError(), "point tables");
     totals.resize(nb);
     cuda_check(cudaMemcpyAsync(totals.data(), sc.totals, nb * sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
@@ -1197,12 +1207,16 @@ void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int
     scratch_grow(sc.m, sc.cap_m, (size_t)sum, s);
     cuda_check(cudaMemcpyAsync(sc.off, off.data(), (nb + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s),
                "point offsets");
-    k_point_candidates<<<blocks, 256, 0, s>>>(ab, nb, sc.tab, sc.off, sc.idx, sc.m);
-    PointLists L{sc.tab, sc.off, sc.idx, sc.m, sc.conf};
-    k_couple_points_grouped<<<1, kGW * 32, kGroupedSmemFixed + (size_t)nb * sizeof(uint16_t), s>>>(c, ab, nb, L);
+    scratch_grow(sc.msum, sc.cap_msum, (size_t)nb, s);
+    k_point_candidates<<<blocks, 256, 0, s>>>(ab, nb, sc.tab, sc.off, sc.idx, sc.m, sc.msum);
+    PointLists L{sc.tab, sc.off, sc.idx, sc.m, sc.msum, sc.key, sc.flow};
+    k_couple_points_flow<<<std::min(flow_blocks, (nb + kFW - 1) / kFW), kFW * 32, kFlowSmem, s>>>(c, ab, nb, L);
     cuda_check(cudaGetLastError(), "couple points");
+    uint32_t failed = 0;
+    cuda_check(cudaMemcpyAsync(&failed, sc.flow + 1, sizeof(failed), cudaMemcpyDeviceToHost, s), "couple points status");
     // The offsets' host copy must outlive the upload.
     cuda_check(cudaStreamSynchronize(s), "couple points sync");
+    if (failed) throw std::runtime_error("couple_points: a point's wait for an earlier one ran out of polls");
   }
 }
 

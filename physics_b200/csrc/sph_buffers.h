@@ -134,16 +134,18 @@ void launch_cell_index(const StepConsts& c, DevBuffers& b, uint32_t* flags, cuda
 void cuda_check(cudaError_t e, const char* what);
 
 // Scratch of couple_points (owned by the world, grown on demand): per-point
-// cell tables, candidate counts and offsets, neighbourhood overlaps with the
-// points just before, candidate indices and masses.
+// cell tables, candidate counts and offsets, centre cells, the walk's ticket
+// and done flags, candidate indices and masses.
 struct CouplePointsScratch {
   uint32_t* tab = nullptr;
   uint32_t* totals = nullptr;
   uint32_t* off = nullptr;
   uint32_t* idx = nullptr;
   double* m = nullptr;
-  uint16_t* conf = nullptr;
-  size_t cap_tab = 0, cap_totals = 0, cap_off = 0, cap_idx = 0, cap_m = 0, cap_conf = 0;
+  double* msum = nullptr;
+  int4* key = nullptr;
+  uint32_t* flow = nullptr;
+  size_t cap_tab = 0, cap_totals = 0, cap_off = 0, cap_idx = 0, cap_m = 0, cap_key = 0, cap_flow = 0, cap_msum = 0;
   void release();
 };
 void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int np, double dt, double drag,
