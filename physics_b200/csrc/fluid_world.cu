@@ -514,7 +514,7 @@ void FluidWorld::free_all() {
   dfree(b_.task_mcount);
   dfree(b_.mask_hdr);
   dfree(b_.mask_bits);
-  dfree(b_.mask_ctl);
+  b_.mask_ctl = nullptr;
   b_.mask_cap = 0;
   mask_tried_ = 0;
   if (b_.mask_demand) cudaFreeHost(b_.mask_demand);
@@ -629,7 +629,7 @@ void FluidWorld::ensure_mode_buffers() {
     if (!b_.dense_q0) dalloc(b_.dense_q0, cap + cap / 32 + 64);
     if (!b_.task_mbase) dalloc(b_.task_mbase, cap + cap / 32 + 64);
     if (!b_.task_mcount) dalloc(b_.task_mcount, cap + cap / 32 + 64);
-    if (!b_.mask_ctl) dalloc(b_.mask_ctl, 1);
+    b_.mask_ctl = reinterpret_cast<unsigned long long*>(b_.flags + 6);
     if (!b_.mask_demand) {
       cuda_check(cudaMallocHost((void**)&b_.mask_demand, sizeof(unsigned long long)), "cudaMallocHost");
       *b_.mask_demand = 0;

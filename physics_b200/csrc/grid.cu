@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <climits>
 
+#include "launch.cuh"
 #include "sph_buffers.h"
 
 namespace phy {
@@ -783,6 +784,7 @@ __device__ __forceinline__ void move_particle(const GatherArgs& g, uint32_t s, u
 }
 
 __global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __restrict__ perm, GatherArgs g) {
+  allow_next();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) move_particle(g, (uint32_t)s, perm[s]);
 }
@@ -880,6 +882,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_fused(StepConsts c, SortArgs 
   for (int i0 = first; i0 < n; i0 += step)
     scatter(n, a.h.bucket_shift, a.h.cell_of, a.h.rank, a.h.count, a.tmp, i0 + (int)threadIdx.x);
   if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  allow_next();
   auto list = [&](uint32_t slot, uint32_t i) { a.perm[slot] = i; };
   if (kCells == 0 && *a.h.crowded == 0u) {  // settled by the histogram: uniform across the grid
     for (int s0 = first; s0 < n; s0 += step)

@@ -85,7 +85,8 @@ struct DevBuffers {
   // entry (kNoMasks: none stored) and entry count; per entry the chunk's
   // first sorted slot << 5 | neighbour cell, and 32 lane masks.  mask_ctl
   // counts the entries the tasks reserved (their upper bounds, stored or
-  // not), so the host can grow mask_cap; mask_demand is its pinned host copy.
+  // not), so the host can grow mask_cap; mask_demand is its copy in mapped host
+  // memory, written by the force pass.
   uint32_t* task_mbase = nullptr;
   uint32_t* task_mcount = nullptr;
   uint32_t* mask_hdr = nullptr;
@@ -108,7 +109,7 @@ struct DevBuffers {
   double* stage = nullptr;   // 8 * capacity doubles
   // [0] error bits, [1] f64 plain step outside the reciprocals' safe range,
   // [2] the sort's large-cell count, [3] its barrier arrivals, [4] whether a
-  // bucket is crowded; zeroed by one memset per step (device).
+  // bucket is crowded, [6..7] mask_ctl; zeroed by one memset per step (device).
   uint32_t* flags = nullptr;
   uint32_t* order_count = nullptr;  // sort: cells of more than kOrderSmall particles (flags + 2)
   unsigned long long* counters = nullptr;  // candidates, pairs (device)

@@ -23,6 +23,7 @@
 #include <cmath>
 #include <limits>
 
+#include "launch.cuh"
 #include "segment_filter.cuh"
 #include "sph_buffers.h"
 
@@ -184,6 +185,7 @@ __device__ __forceinline__ void density_term(const StepConsts& c, const PlainArg
 // its record, and queries in sparse surroundings, are left to the density
 // pass's own walk (PlainArgs::walkers).
 __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_search_plain(StepConsts c, PlainArgs a) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   SegmentStage& st = reinterpret_cast<SegmentStage*>(smem)[threadIdx.x >> 5];
@@ -322,6 +324,7 @@ struct DensityStage {
 // Issue-bound: ~33 candidates of ~80 instructions, a third of them f64.
 template <bool kCount, bool kSame>
 __global__ void __launch_bounds__(kDensityWarps * 32, kDensityCtas) k_density_plain(StepConsts c, PlainArgs a) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   DensityStage& st = reinterpret_cast<DensityStage*>(smem)[threadIdx.x >> 5];
@@ -741,6 +744,7 @@ __device__ __forceinline__ PlainAcc plain_sums(const StepConsts& c, const PlainA
 // (same visit order); a particle whose list overflowed rescans its 27 cells.
 template <int kG, bool kShear>
 __global__ void __launch_bounds__(kThreads, kForceCtas) k_force_plain(StepConsts c, PlainArgs a) {
+  after_previous();
   __shared__ __align__(16) double s_buf[kG == 1 ? 1 : kThreads / 32][kG == 1 ? 1 : (kShear ? 10 : 9) * 32];
   const int lane = threadIdx.x & 31;
   const int i = (blockIdx.x * kThreads + (int)threadIdx.x) / kG;
@@ -820,17 +824,18 @@ void launch_plain_passes(const StepConsts& c, DevBuffers& b, cudaStream_t s, con
   const int groups = (c.n + 31) / 32;
   // Few groups spread over the SMs one warp each before they share one.
   const int spread = std::max(1, groups / kSms);
+  const bool overlap = c.n < kOverlapBelow;
   const int sw = std::min(kSearchWarps, spread), dw = std::min(kDensityWarps, spread);
-  k_search_plain<<<(groups + sw - 1) / sw, sw * 32, sw * sizeof(SegmentStage), s>>>(c, a);
+  launch_after(overlap, k_search_plain, (groups + sw - 1) / sw, sw * 32, sw * sizeof(SegmentStage), s, c, a);
   const bool same = c.h <= c.h0;
   auto density = a.counters ? (same ? k_density_plain<true, true> : k_density_plain<true, false>)
                             : (same ? k_density_plain<false, true> : k_density_plain<false, false>);
-  density<<<(groups + dw - 1) / dw, dw * 32, dw * sizeof(DensityStage), s>>>(c, a);
+  launch_after(overlap, density, (groups + dw - 1) / dw, dw * 32, dw * sizeof(DensityStage), s, c, a);
   if (ev.after_density) cudaEventRecord(ev.after_density, s);
   const int lanes = c.n < kLanesBelow ? 4 : 1;
   auto force = lanes == 4 ? (c.shear_live ? k_force_plain<4, true> : k_force_plain<4, false>)
                           : (c.shear_live ? k_force_plain<1, true> : k_force_plain<1, false>);
-  force<<<(int)(((long long)c.n * lanes + kThreads - 1) / kThreads), kThreads, 0, s>>>(c, a);
+  launch_after(overlap, force, (int)(((long long)c.n * lanes + kThreads - 1) / kThreads), kThreads, 0, s, c, a);
 }
 
 }  // namespace phy

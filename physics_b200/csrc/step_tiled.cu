@@ -26,6 +26,7 @@
 
 #include <algorithm>
 
+#include "launch.cuh"
 #include "sph_buffers.h"
 
 namespace phy {
@@ -100,6 +101,7 @@ struct TiledArgs {
   uint32_t* mask_hdr;
   uint32_t* mask_bits;
   unsigned long long* mask_ctl;
+  unsigned long long* mask_demand;  // mapped host memory (null: none)
   unsigned long long mask_cap;
   int stride;
   uint32_t* flags;
@@ -184,10 +186,13 @@ __device__ __forceinline__ uint32_t first_outside(const TiledArgs& a) {
 // more SMs; one CTA took 31 us for a tile's ~512 queries however few tiles
 // there were.  Both passes use the same split: list entries are slots of the
 // slab's staging.
-constexpr uint32_t kSplitItems = 2 * 148;
+// (us of the density and force passes with 1, 2 and 4 parts: 76,800
+// particles in ~250 tiles 46 + 41, 39 + 43, 40 + 40; 147,456 in ~440 60 + 51,
+// 50 + 47, -; 524,288 in ~1,200 119 + 116, 124 + 127, -.)
+constexpr uint32_t kSplit4Below = 150, kSplit2Below = 600;
 template <int TB>
 __device__ __forceinline__ uint32_t tile_parts(uint32_t ntiles) {
-  return TB * ntiles <= kSplitItems ? (uint32_t)TB : (TB == 4 && 2u * ntiles <= kSplitItems) ? 2u : 1u;
+  return ntiles < kSplit4Below ? (uint32_t)TB : (TB == 4 && ntiles < kSplit2Below) ? 2u : 1u;
 }
 
 struct TileGeom {
@@ -460,6 +465,7 @@ __device__ __forceinline__ void queue_dense_tasks(const TiledArgs& a, const Tile
 // that matches it (40) costs no spill.
 template <int TB, bool kCount, bool kExact>
 __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArgs a) {
+  after_previous();
   using T = Tile<TB>;
   extern __shared__ __align__(16) unsigned char smem[];
   float* s_pp = reinterpret_cast<float*>(smem);  // kHaloCap slots, pair-interleaved
@@ -800,6 +806,7 @@ __device__ __forceinline__ void fold2(CompAcc& q, ForcePart2& b) {
 // 65536 / (3 x 256) cost no occupancy.
 template <int TB, bool kShear>
 __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs a) {
+  after_previous();
   using T = Tile<TB>;
   extern __shared__ __align__(16) unsigned char smem[];
   // Staged neighbour records as separate 16-byte arrays (a 32-byte record
@@ -1055,6 +1062,7 @@ __device__ __forceinline__ void neighbour_offset(const StepConsts& c, int nb, fl
 // f32x2 arithmetic (the filter of the tiled pass without the list).
 template <int TB, bool kCount, bool kExact>
 __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArgs a) {
+  after_previous();
   __shared__ __align__(16) float s_pp[kWarps][32 * 4];  // 32 candidates, pair-interleaved
   const int lane = threadIdx.x & 31;
   float* sp = s_pp[threadIdx.x >> 5];
@@ -1175,6 +1183,9 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
 // end of the chunk, uniformly across the warp.
 template <int TB, bool kShear>
 __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs a) {
+  after_previous();
+  // The entries this step's tasks asked for, for the host's next sizing.
+  if (a.mask_demand && blockIdx.x == 0 && threadIdx.x == 0) *a.mask_demand = *a.mask_ctl;
   // The chunk's 32 candidates, and in slot 32 a weightless copy of its first
   // (mass and m/rho 0) that pads the two-candidate rounds.
   __shared__ float4 s_pos[kWarps][33];
@@ -1372,20 +1383,16 @@ const Occupancy& occupancy() {
 template <int TB>
 void launch_passes(const StepConsts& c, const TiledArgs& a, cudaStream_t s, const PassEvents& ev, bool exact,
                    int density_blocks, int force_blocks, int dense_d_blocks, int dense_f_blocks) {
+  const bool overlap = c.n < kOverlapBelow;
   auto density = a.counters ? (exact ? k_density_tiled<TB, true, true> : k_density_tiled<TB, true, false>)
                             : (exact ? k_density_tiled<TB, false, true> : k_density_tiled<TB, false, false>);
-  density<<<density_blocks, kTT, kDensitySmem, s>>>(c, a);
+  launch_after(overlap, density, density_blocks, kTT, kDensitySmem, s, c, a);
   auto dense = a.counters ? (exact ? k_density_dense<TB, true, true> : k_density_dense<TB, true, false>)
                           : (exact ? k_density_dense<TB, false, true> : k_density_dense<TB, false, false>);
-  dense<<<dense_d_blocks, kWT, 0, s>>>(c, a);
+  launch_after(overlap, dense, dense_d_blocks, kWT, 0, s, c, a);
   if (ev.after_density) cudaEventRecord(ev.after_density, s);
-  if (c.shear_live) {
-    k_force_tiled<TB, true><<<force_blocks, kTT, kForceSmem, s>>>(c, a);
-    k_force_dense<TB, true><<<dense_f_blocks, kWT, 0, s>>>(c, a);
-  } else {
-    k_force_tiled<TB, false><<<force_blocks, kTT, kForceSmem, s>>>(c, a);
-    k_force_dense<TB, false><<<dense_f_blocks, kWT, 0, s>>>(c, a);
-  }
+  launch_after(overlap, c.shear_live ? k_force_tiled<TB, true> : k_force_tiled<TB, false>, force_blocks, kTT, kForceSmem, s, c, a);
+  launch_after(overlap, c.shear_live ? k_force_dense<TB, true> : k_force_dense<TB, false>, dense_f_blocks, kWT, 0, s, c, a);
 }
 
 }  // namespace
@@ -1440,6 +1447,7 @@ void launch_comp_tiled(const StepConsts& c, DevBuffers& b, cudaStream_t s, const
   a.mask_hdr = b.mask_hdr;
   a.mask_bits = b.mask_bits;
   a.mask_ctl = masks ? b.mask_ctl : nullptr;
+  a.mask_demand = masks ? b.mask_demand : nullptr;
   a.mask_cap = b.mask_cap;
   a.stride = b.capacity;
   a.flags = b.flags;
@@ -1455,14 +1463,10 @@ void launch_comp_tiled(const StepConsts& c, DevBuffers& b, cudaStream_t s, const
   if (ev.after_prep) cudaEventRecord(ev.after_prep, s);
   const int dense_d_blocks = o.sms * o.dense_density, dense_f_blocks = o.sms * o.dense_force;
   const bool exact = std::min(c.h2f, c.h0sqf) == c.h0sqf;
-  if (masks) cudaMemsetAsync(b.mask_ctl, 0, sizeof(unsigned long long), s);
   if (c.tile == 2)
     launch_passes<2>(c, a, s, ev, exact, density_blocks, force_blocks, dense_d_blocks, dense_f_blocks);
   else
     launch_passes<4>(c, a, s, ev, exact, density_blocks, force_blocks, dense_d_blocks, dense_f_blocks);
-  // The entries this step's tasks asked for, for the host's next sizing.
-  if (masks && b.mask_demand)
-    cudaMemcpyAsync(b.mask_demand, b.mask_ctl, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
 }
 
 }  // namespace phy
