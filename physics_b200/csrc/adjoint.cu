@@ -76,6 +76,25 @@ __device__ __forceinline__ KernelDerivs kernel_derivs(const StepConsts& c, doubl
   return k;
 }
 
+// The pair kernels' operands of a slot as 32-byte parts, one array each: x and
+// mass; v and m/rho; the seeds P and p/rho^2; Q and sig; Y.  A neighbour is
+// five loads instead of seventeen.
+struct d4 {
+  double x, y, z, w;
+};
+__device__ __forceinline__ d4 load_part(const AdjWork& w, int part, size_t n, int j) {
+  const double* p = w.rec + 4 * (part * n + (size_t)j);
+  d4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void store_part(const AdjWork& w, int part, size_t n, int j, double x, double y, double z,
+                                           double v) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(w.rec + 4 * (part * n + (size_t)j)), "d"(x), "d"(y),
+               "d"(z), "d"(v)
+               : "memory");
+}
+
 __global__ void __launch_bounds__(kThreads) k_adj_integrate(StepConsts c, AdjTape t, AdjWork w) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= c.n) return;
@@ -84,7 +103,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_integrate(StepConsts c, AdjTap
   const double v3[3] = {t.v[0][s], t.v[1][s], t.v[2][s]};
   const double acc3[3] = {t.acc[0][s], t.acc[1][s], t.acc[2][s]};
   const double xs3[3] = {t.xsph[0][s], t.xsph[1][s], t.xsph[2][s]};
-  double accb[3];
+  double accb[3], P[3], Q[3], Y[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     // The forward's integrate and enforce_bounds, operation for operation, to
@@ -100,7 +119,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_integrate(StepConsts c, AdjTap
     vb2 += xb1 * c.dt;
     w.gx[a][s] = xb1;
     w.gv[a][s] = vb2;
-    w.Y[a][s] = vb2 * c.xsph_eps;
+    Y[a] = vb2 * c.xsph_eps;
     accb[a] = vb2 * c.dt;
   }
   const double rho = t.rho[s], mu = t.mu[s];
@@ -109,16 +128,16 @@ __global__ void __launch_bounds__(kThreads) k_adj_integrate(StepConsts c, AdjTap
     const double inv = 1.0 / rho;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      w.P[a][s] = accb[a] * inv;
-      w.Q[a][s] = accb[a] * mu * inv;
+      P[a] = accb[a] * inv;
+      Q[a] = accb[a] * mu * inv;
       mub += accb[a] * t.fv[a][s] * inv;
       rbar -= accb[a] * acc3[a] * inv;
     }
   } else {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      w.P[a][s] = 0.0;
-      w.Q[a][s] = 0.0;
+      P[a] = 0.0;
+      Q[a] = 0.0;
     }
   }
   // mu = kc * (n == 1 ? 1 : max(s, shear_min)^(n-1))  (world.rs:319-327)
@@ -131,7 +150,13 @@ __global__ void __launch_bounds__(kThreads) k_adj_integrate(StepConsts c, AdjTap
   const double sreg = shear > c.shear_min ? shear : c.shear_min;
   const double fac = ex == 0.0 ? 1.0 : pow(sreg, ex);
   w.cc[s] = midx == 0 ? mub * fac : 0.0;
-  w.sig[s] = (ex != 0.0 && shear > c.shear_min) ? mub * kc * ex * pow(sreg, ex - 1.0) : 0.0;
+  const double sig = (ex != 0.0 && shear > c.shear_min) ? mub * kc * ex * pow(sreg, ex - 1.0) : 0.0;
+  const size_t n = (size_t)c.n;
+  store_part(w, 0, n, s, x3[0], x3[1], x3[2], t.mass[s]);
+  store_part(w, 1, n, s, v3[0], v3[1], v3[2], t.mr[s]);
+  store_part(w, 2, n, s, P[0], P[1], P[2], t.pr2[s]);
+  store_part(w, 3, n, s, Q[0], Q[1], Q[2], sig);
+  store_part(w, 4, n, s, Y[0], Y[1], Y[2], 0.0);
   w.rbar[s] = rbar;
 }
 
@@ -148,7 +173,13 @@ __device__ __forceinline__ void for_each_listed(const StepConsts& c, const AdjTa
                                                 double yi, double zi, F&& f) {
   const uint32_t cnt = t.nbr_count[i];
   if (cnt <= (uint32_t)kMaxNeighbors) {
-    for (uint32_t k = q; k < cnt; k += kLanes) f((int)t.nbr[(size_t)k * c.n + i]);
+    // The next index is loaded while this neighbour is computed.
+    uint32_t j = (uint32_t)q < cnt ? t.nbr[(size_t)q * c.n + i] : 0u;
+    for (uint32_t k = q; k < cnt; k += kLanes) {
+      const int jc = (int)j;
+      if (k + kLanes < cnt) j = t.nbr[(size_t)(k + kLanes) * c.n + i];
+      f(jc);
+    }
     return;
   }
   const long long kx = key_axis(xi, c.inv_cell), ky = key_axis(yi, c.inv_cell), kz = key_axis(zi, c.inv_cell);
@@ -175,18 +206,20 @@ __global__ void __launch_bounds__(kThreads) k_adj_force(StepConsts c, AdjTape t,
   const int i = g / kLanes, q = g % kLanes;
   const bool live = i < c.n;  // whole particles per warp: kLanes divides 32
   const int ii = live ? i : 0;
-  const double xi = t.x[0][ii], yi = t.x[1][ii], zi = t.x[2][ii];
-  const double vxi = t.v[0][ii], vyi = t.v[1][ii], vzi = t.v[2][ii];
-  const double m_i = t.mass[ii], pr2_i = t.pr2[ii], mr_i = t.mr[ii];
-  const double Pi[3] = {w.P[0][ii], w.P[1][ii], w.P[2][ii]};
-  const double Qi[3] = {w.Q[0][ii], w.Q[1][ii], w.Q[2][ii]};
-  const double Yi[3] = {w.Y[0][ii], w.Y[1][ii], w.Y[2][ii]};
-  const double sig_i = w.sig[ii];
+  const size_t n = (size_t)c.n;
+  const d4 xo = load_part(w, 0, n, ii), vo = load_part(w, 1, n, ii), po = load_part(w, 2, n, ii),
+           qo = load_part(w, 3, n, ii), yo = load_part(w, 4, n, ii);
+  const double xi = xo.x, yi = xo.y, zi = xo.z, vxi = vo.x, vyi = vo.y, vzi = vo.z;
+  const double m_i = xo.w, pr2_i = po.w, mr_i = vo.w;
+  const double Pi[3] = {po.x, po.y, po.z}, Qi[3] = {qo.x, qo.y, qo.z}, Yi[3] = {yo.x, yo.y, yo.z};
+  const double sig_i = qo.w;
   double gx[3] = {0.0, 0.0, 0.0}, gv[3] = {0.0, 0.0, 0.0};
   double pibar = 0.0, rsum = 0.0;
   if (live) for_each_listed(c, t, i, q, xi, yi, zi, [&](int j) {
     // The forward's neighbour test (d = p_j - p_i, world.rs:295-299).
-    const double d[3] = {__dsub_rn(t.x[0][j], xi), __dsub_rn(t.x[1][j], yi), __dsub_rn(t.x[2][j], zi)};
+    const d4 xj = load_part(w, 0, n, j), vj = load_part(w, 1, n, j), pj = load_part(w, 2, n, j),
+             qj = load_part(w, 3, n, j), yj = load_part(w, 4, n, j);
+    const double d[3] = {__dsub_rn(xj.x, xi), __dsub_rn(xj.y, yi), __dsub_rn(xj.z, zi)};
     const double r2 = norm2(d[0], d[1], d[2]);
     if (r2 > c.r2_guard) return;
     const double r = __dsqrt_rn(r2);
@@ -194,18 +227,16 @@ __global__ void __launch_bounds__(kThreads) k_adj_force(StepConsts c, AdjTape t,
     const KernelDerivs k = kernel_derivs(c, r);
     const double inv_r = __drcp_rn(r);
     const double u[3] = {d[0] * inv_r, d[1] * inv_r, d[2] * inv_r};
-    const double dv[3] = {t.v[0][j] - vxi, t.v[1][j] - vyi, t.v[2][j] - vzi};
+    const double dv[3] = {vj.x - vxi, vj.y - vyi, vj.z - vzi};
     const double dv2 = dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2];
     const double inv_dvn = dv2 > 0.0 ? rsqrt(dv2) : 0.0;
     const double dvn = dv2 * inv_dvn;
-    const double m_j = t.mass[j], mr_j = t.mr[j];
+    const double m_j = xj.w, mr_j = vj.w;
     const double mm = m_i * m_j;
-    const double A = mm * (pr2_i + t.pr2[j]);
+    const double A = mm * (pr2_i + pj.w);
     const double inv_re = __drcp_rn(r + kShearEps);
-    const double Pj[3] = {w.P[0][j], w.P[1][j], w.P[2][j]};
-    const double Qj[3] = {w.Q[0][j], w.Q[1][j], w.Q[2][j]};
-    const double Yj[3] = {w.Y[0][j], w.Y[1][j], w.Y[2][j]};
-    const double sig_j = w.sig[j];
+    const double Pj[3] = {pj.x, pj.y, pj.z}, Qj[3] = {qj.x, qj.y, qj.z}, Yj[3] = {yj.x, yj.y, yj.z};
+    const double sig_j = qj.w;
     // Own terms (i's seeds): variables d, dv, pi_i, pi_j, rho_j.
     const double uP = u[0] * Pi[0] + u[1] * Pi[1] + u[2] * Pi[2];
     const double dvQ = dv[0] * Qi[0] + dv[1] * Qi[1] + dv[2] * Qi[2];
@@ -272,20 +303,24 @@ __global__ void __launch_bounds__(kThreads) k_adj_density(StepConsts c, AdjTape 
   const int i = g / kLanes, q = g % kLanes;
   const bool live = i < c.n;
   const int ii = live ? i : 0;
-  const double xi = t.x[0][ii], yi = t.x[1][ii], zi = t.x[2][ii];
-  const double m_i = t.mass[ii], rb_i = w.rbar_tot[ii];
+  const size_t n = (size_t)c.n;
+  const d4 xo = load_part(w, 0, n, ii);
+  const double xi = xo.x, yi = xo.y, zi = xo.z;
+  const double m_i = xo.w, rb_i = w.rbar_tot[ii];
   double gd[3] = {0.0, 0.0, 0.0};
   if (live) for_each_listed(c, t, i, q, xi, yi, zi, [&](int j) {
     // The forward's density test (p_i - p_j, world.rs:226-229); r = 0 pairs
     // (self, coincident particles) have W'(0) = 0.
-    const double d[3] = {__dsub_rn(xi, t.x[0][j]), __dsub_rn(yi, t.x[1][j]), __dsub_rn(zi, t.x[2][j])};
+    const d4 xj = load_part(w, 0, n, j);
+    const double rb_j = w.rbar_tot[j];
+    const double d[3] = {__dsub_rn(xi, xj.x), __dsub_rn(yi, xj.y), __dsub_rn(zi, xj.z)};
     const double r2 = norm2(d[0], d[1], d[2]);
     if (r2 > c.r2_guard) return;
     const double r = __dsqrt_rn(r2);
     if (!(r < c.h) || r <= 0.0 || r >= c.h0) return;
     const double qq = c.h0sq - r2;
     // W'(r) / r = -6 poly6_c (h0^2 - r^2)^2
-    const double f = -6.0 * c.poly6_c * qq * qq * (t.mass[j] * rb_i + m_i * w.rbar_tot[j]);
+    const double f = -6.0 * c.poly6_c * qq * qq * (xj.w * rb_i + m_i * rb_j);
 #pragma unroll
     for (int a = 0; a < 3; ++a) gd[a] += f * d[a];
   });
@@ -300,28 +335,55 @@ __global__ void __launch_bounds__(kThreads) k_adj_density(StepConsts c, AdjTape 
   }
 }
 
-// acc[0] += sum a[0..n), acc[1] += sum b[0..n): one block, fixed order.
-__global__ void __launch_bounds__(1024) k_adj_sum2(int n, const double* __restrict__ a,
-                                                   const double* __restrict__ b, double* acc) {
-  __shared__ double sa[1024], sb[1024];
-  double x = 0.0, y = 0.0;
-  for (int k = threadIdx.x; k < n; k += 1024) {
-    x += a[k];
-    y += b[k];
-  }
+// acc[0] += sum a[0..n), acc[1] += sum b[0..n) in a fixed order: kSumBlocks
+// blocks write partial sums, the last one to arrive adds them up (`arrived`
+// ends at zero again).  One block took 17 us for 65,536 values.
+constexpr int kSumThreads = 256;
+__device__ __forceinline__ void block_sum2(double& x, double& y) {
+  __shared__ double sa[kSumThreads], sb[kSumThreads];
+  __syncthreads();
   sa[threadIdx.x] = x;
   sb[threadIdx.x] = y;
   __syncthreads();
-  for (int o = 512; o > 0; o >>= 1) {
+  for (int o = kSumThreads / 2; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) {
       sa[threadIdx.x] += sa[threadIdx.x + o];
       sb[threadIdx.x] += sb[threadIdx.x + o];
     }
     __syncthreads();
   }
+  x = sa[0];
+  y = sb[0];
+}
+__global__ void __launch_bounds__(kSumThreads) k_adj_sum2(int n, const double* __restrict__ a,
+                                                          const double* __restrict__ b, double* acc, double* part,
+                                                          unsigned* arrived) {
+  __shared__ bool s_last;
+  double x = 0.0, y = 0.0;
+  for (int k = blockIdx.x * kSumThreads + threadIdx.x; k < n; k += kAdjSumBlocks * kSumThreads) {
+    x += a[k];
+    y += b[k];
+  }
+  block_sum2(x, y);
   if (threadIdx.x == 0) {
-    acc[0] += sa[0];
-    acc[1] += sb[0];
+    part[2 * blockIdx.x] = x;
+    part[2 * blockIdx.x + 1] = y;
+    __threadfence();
+    s_last = atomicAdd(arrived, 1u) == (unsigned)kAdjSumBlocks - 1u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  x = y = 0.0;
+  if (threadIdx.x < kAdjSumBlocks) {
+    x = __ldcg(part + 2 * threadIdx.x);
+    y = __ldcg(part + 2 * threadIdx.x + 1);
+  }
+  block_sum2(x, y);
+  if (threadIdx.x == 0) {
+    acc[0] += x;
+    acc[1] += y;
+    *arrived = 0;
   }
 }
 
@@ -336,7 +398,8 @@ void launch_adjoint_step(const StepConsts& c, const AdjTape& t, const AdjWork& w
   k_adj_force<<<pair_grid, kThreads, 0, s>>>(c, t, w);
   k_adj_density<<<pair_grid, kThreads, 0, s>>>(c, t, w);
   // param_acc = {d/d stiffness, d/d visc_k[0]}
-  k_adj_sum2<<<1, 1024, 0, s>>>(c.n, w.kk, w.cc, w.param_acc);
+  static_assert(kAdjSumBlocks <= kSumThreads, "one partial per thread");
+  k_adj_sum2<<<kAdjSumBlocks, kSumThreads, 0, s>>>(c.n, w.kk, w.cc, w.param_acc, w.sum_part, w.sum_arrived);
 }
 
 }  // namespace phy

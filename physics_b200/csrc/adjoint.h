@@ -34,6 +34,9 @@ struct AdjTape {
   const uint32_t* nbr_count;
 };
 
+constexpr int kAdjRec = 20;        // doubles per slot of AdjWork::rec
+constexpr int kAdjSumBlocks = 64;  // blocks of the parameter sums
+
 // Adjoint state: gx_ins / gv_ins hold dL/dx, dL/dv in insertion order
 // between steps (dL/dx', dL/dv' on entry to a reverse step, dL/dx, dL/dv on
 // exit); the rest is per-step scratch in sorted order.
@@ -42,15 +45,17 @@ struct AdjWork {
   double* gv_ins[3];
   double* gx[3];
   double* gv[3];
-  double* P[3];   // dL/d f_press
-  double* Q[3];   // dL/d f_visc_raw
-  double* Y[3];   // dL/d xsph
-  double* sig;    // dL/d shear
+  // The pair kernels' packed operands (32-byte aligned): the state and the
+  // seeds P = dL/d f_press, Q = dL/d f_visc_raw, Y = dL/d xsph and
+  // sig = dL/d shear, kAdjRec doubles per slot.
+  double* rec;
   double* rbar;   // direct dL/d rho (through acc)
   double* rbar_tot;
   double* cc;     // per-particle dL/d visc_k[0] terms
   double* kk;     // per-particle dL/d stiffness terms
   double* param_acc;  // device {dL/d stiffness, dL/d visc_k[0]}, accumulated
+  double* sum_part;   // 2 kAdjSumBlocks partial sums
+  unsigned* sum_arrived;  // zero between launches
 };
 
 void launch_adjoint_step(const StepConsts& c, const AdjTape& t, const AdjWork& w, cudaStream_t s);

@@ -245,19 +245,36 @@ struct TapeCopy {
   uint32_t* slot_of;        // nullable: insertion index -> recorded slot
 };
 
-__global__ void k_tape_copy(int n, TapeCopy t) {
+// blockIdx.y: half of the f64 arrays (0, 1; the u32 arrays with 1), then
+// kTapeRows list entries each.  (One thread per particle copying its whole
+// list took 29 us for 65,536 particles.)
+constexpr int kTapeRows = 8;
+constexpr int kTapeParts = 2 + kMaxNeighbors / kTapeRows;
+__global__ void __launch_bounds__(kThreads) k_tape_copy(int n, TapeCopy t) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
+  const int part = blockIdx.y;
+  if (part == 0) {
 #pragma unroll
-  for (int k = 0; k < 22; ++k) t.dst[k][s] = t.src[k][s];
-  t.udst[0][s] = t.usrc[0][s];
-  const uint32_t id = t.usrc[1][s];
-  t.udst[1][s] = id;
-  if (t.slot_of) t.slot_of[id] = (uint32_t)s;
-  const uint32_t cnt = t.usrc[2][s];
-  t.udst[2][s] = cnt;
-  const uint32_t m = cnt < (uint32_t)kMaxNeighbors ? cnt : (uint32_t)kMaxNeighbors;
-  for (uint32_t k = 0; k < m; ++k) t.nbr_dst[(size_t)k * n + s] = t.nbr[(size_t)k * t.nbr_stride + s];
+    for (int k = 0; k < 11; ++k) t.dst[k][s] = t.src[k][s];
+    return;
+  }
+  if (part == 1) {
+#pragma unroll
+    for (int k = 11; k < 22; ++k) t.dst[k][s] = t.src[k][s];
+    t.udst[0][s] = t.usrc[0][s];
+    const uint32_t id = t.usrc[1][s];
+    t.udst[1][s] = id;
+    if (t.slot_of) t.slot_of[id] = (uint32_t)s;
+    t.udst[2][s] = t.usrc[2][s];
+    return;
+  }
+  const uint32_t m = min(t.usrc[2][s], (uint32_t)kMaxNeighbors), k0 = (uint32_t)(part - 2) * kTapeRows;
+#pragma unroll
+  for (uint32_t q = 0; q < (uint32_t)kTapeRows; ++q) {
+    const uint32_t k = k0 + q;
+    if (k < m) t.nbr_dst[(size_t)k * n + s] = t.nbr[(size_t)k * t.nbr_stride + s];
+  }
 }
 
 // Several device arrays copied in one launch (blockIdx.y = array): 16-byte
@@ -1979,6 +1996,9 @@ void FluidWorld::save_checkpoint() {
   ++tape_.nckpt;
 }
 
+// Arrays of n doubles in the reverse sweep's work buffer (step_backward).
+static constexpr size_t kAdjWorkArrays = kAdjRec + 4 * 3 + 4 + 4;
+
 // Ends the tape.  Its buffers stay for the next tape of the same size while
 // they are small (an optimisation loop clears and begins a tape every
 // iteration; allocating and freeing them took two thirds of it at 65,536
@@ -1988,7 +2008,7 @@ void FluidWorld::tape_clear() {
   tape_.nckpt = 0;
   tape_.dts.clear();
   tape_.on = false;
-  size_t bytes = (6 * tape_.ckpt.size() + 22 * adj_slot_f_.size() + (adj_work_ ? 30 : 0)) * tape_.n * sizeof(double) +
+  size_t bytes = (6 * tape_.ckpt.size() + 22 * adj_slot_f_.size() + (adj_work_ ? kAdjWorkArrays : 0)) * tape_.n * sizeof(double) +
                  comp_rec_cap_ * sizeof(uint32_t);
   for (size_t u : adj_slot_ucount_) bytes += u * sizeof(uint32_t);
   for (size_t q : snap_bytes_) bytes += q;
@@ -2076,11 +2096,11 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
   if (!tape_.on) throw std::invalid_argument("step_backward: no adjoint tape (call tape_begin before stepping)");
   if (n == 0) return;
   cudaStream_t s = stream_;
-  // Work arrays: gx_ins, gv_ins, gx, gv, P, Q, Y (3 each), sig, rbar,
-  // rbar_tot, cc, kk, the tape's fv and shear outputs (4): 30 arrays of n,
-  // then the two parameter accumulators.
-  constexpr size_t kWorkArrays = 30;
-  if (!adj_work_) dalloc(adj_work_, kWorkArrays * n + 2);
+  // Work arrays: the packed operands (kAdjRec), gx_ins, gv_ins, gx, gv (3
+  // each), rbar, rbar_tot, cc, kk, the tape's fv and shear outputs (4): arrays
+  // of n, then the two parameter accumulators with their partial sums.
+  constexpr size_t kWorkArrays = kAdjWorkArrays;
+  if (!adj_work_) dalloc(adj_work_, kWorkArrays * n + 2 + 2 * kAdjSumBlocks + 1);
   double* work = adj_work_;
   AdjWork w;
   {
@@ -2092,14 +2112,12 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
       q += n;
       return r;
     };
+    w.rec = q;
+    for (int k = 0; k < kAdjRec; ++k) (void)take();
     for (int k = 0; k < 3; ++k) w.gx_ins[k] = take();
     for (int k = 0; k < 3; ++k) w.gv_ins[k] = take();
     for (int k = 0; k < 3; ++k) w.gx[k] = take();
     for (int k = 0; k < 3; ++k) w.gv[k] = take();
-    for (int k = 0; k < 3; ++k) w.P[k] = take();
-    for (int k = 0; k < 3; ++k) w.Q[k] = take();
-    for (int k = 0; k < 3; ++k) w.Y[k] = take();
-    w.sig = take();
     w.rbar = take();
     w.rbar_tot = take();
     w.cc = take();
@@ -2107,6 +2125,8 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
     for (int k = 0; k < 3; ++k) b_.tape_fv[k] = take();
     b_.tape_shear = take();
     w.param_acc = q;
+    w.sum_part = q + 2;
+    w.sum_arrived = reinterpret_cast<unsigned*>(q + 2 + 2 * kAdjSumBlocks);
   }
   const int nslots = std::min(tape_.every, std::max(T, 1));
   std::vector<TapeSlot> slots(nslots);
@@ -2140,8 +2160,8 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
   try {
     snapshot(false);  // the world returns to x_T, v_T afterwards
     // Seeds (insertion order): dL/dx_T, dL/dv_T.
-    cuda_check(cudaMemsetAsync(work, 0, (6 * n + 0) * sizeof(double), s), "seed clear");
-    cuda_check(cudaMemsetAsync(w.param_acc, 0, 2 * sizeof(double), s), "param clear");
+    cuda_check(cudaMemsetAsync(w.gx_ins[0], 0, 6 * n * sizeof(double), s), "seed clear");
+    cuda_check(cudaMemsetAsync(w.param_acc, 0, (2 + 2 * kAdjSumBlocks + 1) * sizeof(double), s), "param clear");
     if (gx) {
       cuda_check(cudaMemcpyAsync(b_.stage, gx, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s), "seed upload");
       launch_deinterleave3(b_.stage, w.gx_ins[0], w.gx_ins[1], w.gx_ins[2], (int)n, s);
@@ -2214,7 +2234,7 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
         tc.nbr_dst = const_cast<uint32_t*>(v.nbr);
         tc.nbr_stride = b_.capacity;
         tc.slot_of = slot_of;
-        k_tape_copy<<<grid_for(n), kThreads, 0, s>>>((int)n, tc);
+        k_tape_copy<<<dim3((unsigned)grid_for(n), kTapeParts), kThreads, 0, s>>>((int)n, tc);
         cuda_check(cudaMemcpyAsync(const_cast<uint32_t*>(v.cell_start), b_.cell_start, ncs * 4,
                                    cudaMemcpyDeviceToDevice, s),
                    "tape copy");
