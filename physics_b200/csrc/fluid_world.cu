@@ -527,6 +527,7 @@ void FluidWorld::free_all() {
   dfree(b_.queue);
   dfree(b_.tile_crowd);
   dfree(b_.dense_q0);
+  dfree(b_.task_done);
   dfree(b_.task_mbase);
   dfree(b_.task_mcount);
   dfree(b_.mask_hdr);
@@ -607,6 +608,7 @@ void FluidWorld::ensure_capacity(size_t n) {
   dfree(b_.tile_slot);
   dfree(b_.tile_crowd);
   dfree(b_.dense_q0);
+  dfree(b_.task_done);
   dfree(b_.task_mbase);
   dfree(b_.task_mcount);
   dfree(b_.okey);
@@ -644,8 +646,10 @@ void FluidWorld::ensure_mode_buffers() {
     if (!b_.queue) dalloc(b_.queue, 5);
     // Dense-cell tasks: at most one per 32 particles plus one per occupied cell.
     if (!b_.dense_q0) dalloc(b_.dense_q0, cap + cap / 32 + 64);
-    if (!b_.task_mbase) dalloc(b_.task_mbase, cap + cap / 32 + 64);
-    if (!b_.task_mcount) dalloc(b_.task_mcount, cap + cap / 32 + 64);
+    // (two halves per task)
+    if (!b_.task_done) dalloc(b_.task_done, 2 * (cap + cap / 32 + 64));
+    if (!b_.task_mbase) dalloc(b_.task_mbase, 2 * (cap + cap / 32 + 64));
+    if (!b_.task_mcount) dalloc(b_.task_mcount, 2 * (cap + cap / 32 + 64));
     b_.mask_ctl = reinterpret_cast<unsigned long long*>(b_.flags + 6);
     if (!b_.mask_demand) {
       cuda_check(cudaMallocHost((void**)&b_.mask_demand, sizeof(unsigned long long)), "cudaMallocHost");

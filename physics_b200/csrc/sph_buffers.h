@@ -81,12 +81,13 @@ struct DevBuffers {
   uint32_t* queue = nullptr;
   uint32_t* dense_q0 = nullptr;
   // In-range masks of the dense-cell density pass, read back by the force
-  // pass of the same step instead of filtering again: per task its first
+  // pass of the same step instead of filtering again: per half task its first
   // entry (kNoMasks: none stored) and entry count; per entry the chunk's
   // first sorted slot << 5 | neighbour cell, and 32 lane masks.  mask_ctl
   // counts the entries the tasks reserved (their upper bounds, stored or
   // not), so the host can grow mask_cap; mask_demand is its copy in mapped host
   // memory, written by the force pass.
+  uint32_t* task_done = nullptr;  // per task: halves finished (density, force)
   uint32_t* task_mbase = nullptr;
   uint32_t* task_mcount = nullptr;
   uint32_t* mask_hdr = nullptr;

@@ -96,7 +96,8 @@ struct TiledArgs {
   uint32_t* dense_count;
   uint32_t* dense_taken;  // [0]: tasks taken by the density pass, [1]: by the force pass
   // The density pass's in-range masks for the force pass (null: none kept).
-  uint32_t* task_mbase;
+  uint32_t* task_done;  // per task: halves finished by the density and by the force pass
+  uint32_t* task_mbase;  // per half
   uint32_t* task_mcount;
   uint32_t* mask_hdr;
   uint32_t* mask_bits;
@@ -456,6 +457,7 @@ __device__ __forceinline__ void queue_dense_tasks(const TiledArgs& a, const Tile
       if (s_pre[mid] <= k) lo = mid; else hi = mid - 1;
     }
     a.dense_q0[base + k] = a.cell_start[first_cell + (uint32_t)lo] + 32u * (k - s_pre[lo]);
+    a.task_done[2u * (base + k)] = a.task_done[2u * (base + k) + 1u] = 0u;
   }
   __syncthreads();
 }
@@ -927,7 +929,15 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
 // of filtering again, which gives the same pairs in the same order; a task
 // whose reservation did not fit filters as before.
 
+// A task runs in two halves (every other chunk), which are work items of
+// their own: the warp that finishes a task second adds the halves' sums (half
+// 0 + half 1, so the result does not depend on which that is), and no warp
+// waits.  A whole task in cells of 160 takes one warp ~100 us, and a world of
+// 100,000 has barely more tasks than the GPU has warps.  The sums pass through
+// the queries' unused list rows.
 constexpr int kWT = 256;  // threads per dense-task CTA
+constexpr int kHalfWords = 17;  // floats of a half's sums in a list row
+static_assert(2 * kHalfWords * sizeof(float) <= kMaxNeighbors * sizeof(uint16_t), "both halves fit a list row");
 constexpr int kWarps = kWT / 32;
 constexpr uint32_t kNoMasks = 0xffffffffu;
 
@@ -999,7 +1009,7 @@ __device__ __forceinline__ CellGeom cell_geom(const StepConsts& c, const TiledAr
 // 27 neighbour ranges held by lanes 0..26 (empty when the neighbour cell's
 // box is out of reach of the queries' box).
 struct DenseTask {
-  uint32_t k;  // task index
+  uint32_t k, half;  // task and which of its halves
   uint32_t q0, qn;
   CellGeom cg;
   uint32_t nb_s, nb_e;  // this lane's neighbour range (lane < 27)
@@ -1012,13 +1022,34 @@ __device__ __forceinline__ bool next_task(const StepConsts& c, const TiledArgs& 
   uint32_t k = 0;
   if (lane == 0) k = atomicAdd(counter, 1u);
   k = __shfl_sync(0xffffffffu, k, 0);
-  if (k >= ntasks) return false;
+  if (k >= 2u * ntasks) return false;
+  t.half = k & 1u;
+  k >>= 1;
   t.k = k;
   t.q0 = a.dense_q0[k];
   const uint32_t cell = a.sorted_cell[t.q0];
   t.qn = min(32u, a.cell_start[cell + 1] - t.q0);
   t.cg = cell_geom<TB>(c, a, cell);
   return true;
+}
+
+// Word k of a half's sums of this lane's query: word after word over the
+// task's queries, in their list rows.
+__device__ __forceinline__ float* half_sum(const TiledArgs& a, const DenseTask& t, uint32_t half, int k) {
+  return reinterpret_cast<float*>(a.nbr16 + (size_t)t.q0 * kMaxNeighbors) + (half * kHalfWords + (uint32_t)k) * t.qn +
+         (threadIdx.x & 31u);
+}
+// Whether this warp finishes the task of `pass` (0 density, 1 force) second:
+// then the other half's sums are visible.  Its own must be written.
+__device__ __forceinline__ bool finishes_task(const TiledArgs& a, uint32_t task, int pass) {
+  __syncwarp();
+  uint32_t before = 0;
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    before = atomicAdd(a.task_done + 2u * task + pass, 1u);
+    __threadfence();
+  }
+  return __shfl_sync(0xffffffffu, before, 0) == 1u;
 }
 
 // Neighbour ranges of the task (lane nb < 27 holds neighbour nb), with
@@ -1083,19 +1114,23 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
     // every neighbour cell in reach).
     uint32_t mbase = kNoMasks, mcount = 0;
     if (a.mask_ctl) {
-      const uint32_t bound = __reduce_add_sync(0xffffffffu, (t.nb_e - t.nb_s + 31u) >> 5);
+      const uint32_t chunks = __reduce_add_sync(0xffffffffu, (t.nb_e - t.nb_s + 31u) >> 5);
+      const uint32_t bound = (chunks + 1u - t.half) >> 1;  // this half's
       unsigned long long base = 0;
       if (lane == 0) base = atomicAdd(a.mask_ctl, (unsigned long long)bound);
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base + bound <= a.mask_cap) mbase = (uint32_t)base;
     }
     float s = 0.f, comp = 0.f;
+    uint32_t skip = t.half;  // chunks of the other half before this half's next
     for (int nb = 0; nb < 27; ++nb) {
       const uint32_t s0 = __shfl_sync(0xffffffffu, t.nb_s, nb), e0 = __shfl_sync(0xffffffffu, t.nb_e, nb);
       if (s0 >= e0) continue;
       float off[3];
       neighbour_offset(c, nb, off);
-      for (uint32_t cb = s0; cb < e0; cb += 32) {
+      uint32_t cb = s0 + 32u * skip;
+      skip ^= ((e0 - s0 + 31u) >> 5) & 1u;
+      for (; cb < e0; cb += 64) {
         const uint32_t j = cb + (uint32_t)lane;
         const bool cv = j < e0;
         float4 p = cv ? a.cpos[j] : make_float4(kFar, kFar, kFar, 0.f);
@@ -1154,13 +1189,20 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
         __syncwarp();  // the chunk is consumed before the next one is staged
       }
     }
-    if (qv) {
-      write_density(c, a, (int)qi, (double)s - (double)comp);
-      a.nbr_count[qi] = kNoList;
-    }
     if (a.mask_ctl && lane == 0) {
-      a.task_mbase[t.k] = mbase;
-      a.task_mcount[t.k] = mcount;
+      a.task_mbase[2u * t.k + t.half] = mbase;
+      a.task_mcount[2u * t.k + t.half] = mcount;
+    }
+    if (qv) {
+      *half_sum(a, t, t.half, 0) = s;
+      *half_sum(a, t, t.half, 1) = comp;
+    }
+    if (finishes_task(a, t.k, 0) && qv) {
+      auto sum = [&](uint32_t half) {
+        return (double)__ldcg(half_sum(a, t, half, 0)) - (double)__ldcg(half_sum(a, t, half, 1));
+      };
+      write_density(c, a, (int)qi, sum(0) + sum(1));
+      a.nbr_count[qi] = kNoList;
     }
   }
   if (kCount) {
@@ -1252,8 +1294,8 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
         if (rounds & 7) fold<kShear>(acc, part, qp.w * c.spiky_cf, lapm);
       }
     };
-    uint32_t mbase = a.task_mbase ? a.task_mbase[t.k] : kNoMasks;
-    const uint32_t mcount = mbase != kNoMasks ? a.task_mcount[t.k] : 0u;
+    uint32_t mbase = a.task_mbase ? a.task_mbase[2u * t.k + t.half] : kNoMasks;
+    const uint32_t mcount = mbase != kNoMasks ? a.task_mcount[2u * t.k + t.half] : 0u;
     if (mbase != kNoMasks && ((unsigned long long)mbase + mcount > a.mask_cap || mcount > (1u << 20))) {
       if (lane == 0) atomicOr(a.flags, kFlagMaskTable);
       mbase = kNoMasks;
@@ -1292,12 +1334,15 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
     } else {
       const Box3 qb = warp_box(qp.x, qp.y, qp.z, qv);
       task_neighbours<TB>(c, a, t, qb, hc2);
+      uint32_t skip = t.half;  // chunks of the other half before this half's next
       for (int nb = 0; nb < 27; ++nb) {
         const uint32_t s0 = __shfl_sync(0xffffffffu, t.nb_s, nb), e0 = __shfl_sync(0xffffffffu, t.nb_e, nb);
         if (s0 >= e0) continue;
         float off[3];
         neighbour_offset(c, nb, off);
-        for (uint32_t cb = s0; cb < e0; cb += 32) {
+        uint32_t cb = s0 + 32u * skip;
+        skip ^= ((e0 - s0 + 31u) >> 5) & 1u;
+        for (; cb < e0; cb += 64) {
           const uint32_t j = cb + (uint32_t)lane;
           const bool cv = j < e0;
           float4 p = cv ? a.cpos[j] : make_float4(kFar, kFar, kFar, 0.f);
@@ -1331,7 +1376,33 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
         }
       }
     }
-    if (qv) finish_particle(c, a, (int)qi, acc, c.boxes[t.cg.sc]);
+    const float sums[kHalfWords] = {acc.fpx, acc.cpx, acc.fpy, acc.cpy, acc.fpz, acc.cpz, acc.fvx, acc.cvx, acc.fvy,
+                                    acc.cvy, acc.fvz, acc.cvz, acc.xsx, acc.xsy, acc.xsz, acc.shear, acc.csh};
+    if (qv) {
+#pragma unroll
+      for (int k = 0; k < (kShear ? 17 : 15); ++k) *half_sum(a, t, t.half, k) = sums[k];
+    }
+    if (finishes_task(a, t.k, 1) && qv) {
+      float v[kHalfWords], o[kHalfWords];
+#pragma unroll
+      for (int k = 0; k < kHalfWords; ++k) {
+        v[k] = k < (kShear ? 17 : 15) ? __ldcg(half_sum(a, t, 0, k)) : 0.f;
+        o[k] = k < (kShear ? 17 : 15) ? __ldcg(half_sum(a, t, 1, k)) : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 17; k += 2) {
+        if (k == 12) k = 15;  // the XSPH sums have no compensation
+        if (k == 15 && !kShear) break;
+        kahan_add(v[k], v[k + 1], o[k]);
+        kahan_add(v[k], v[k + 1], -o[k + 1]);
+      }
+      CompAcc q;
+      q.fpx = v[0], q.cpx = v[1], q.fpy = v[2], q.cpy = v[3], q.fpz = v[4], q.cpz = v[5];
+      q.fvx = v[6], q.cvx = v[7], q.fvy = v[8], q.cvy = v[9], q.fvz = v[10], q.cvz = v[11];
+      q.xsx = v[12] + o[12], q.xsy = v[13] + o[13], q.xsz = v[14] + o[14];
+      q.shear = v[15], q.csh = v[16];
+      finish_particle(c, a, (int)qi, q, c.boxes[t.cg.sc]);
+    }
   }
 }
 
@@ -1441,6 +1512,7 @@ void launch_comp_tiled(const StepConsts& c, DevBuffers& b, cudaStream_t s, const
   a.dense_count = b.queue + 2;
   a.dense_taken = b.queue + 3;
   a.dense_q0 = b.dense_q0;
+  a.task_done = b.task_done;
   const bool masks = t.dense_masks && b.mask_ctl != nullptr;
   a.task_mbase = masks ? b.task_mbase : nullptr;
   a.task_mcount = b.task_mcount;

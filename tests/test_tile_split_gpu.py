@@ -37,3 +37,45 @@ def test_split_changes_no_bit(gpu, dims, materials):
         w.step(0.005, 3)
     for k in FIELDS:
         assert_bits_equal(getattr(alone, k), getattr(both, k)[:len(pos)], k)
+
+
+@pytest.mark.parametrize("n,per_cell", [(33, 33), (700, 64), (6000, 160), (20000, 1100)])
+@pytest.mark.parametrize("materials", [1, 3])
+def test_dense_halves(gpu, oracle_mod, n, per_cell, materials):
+    """Dense-cell tasks run in halves joined by the second to finish: sheets with one and many
+    tasks per cell, kept masks and the filtering walk, against the oracle within the compensated
+    form's bounds (density 1e-5; the sums of ~per_cell terms keep it far below) and twice for the
+    same bits."""
+    O = oracle_mod
+    rng = np.random.default_rng(n)
+    edge = 0.2 * max(1.0, n / per_cell) ** 0.5
+    pos = rng.uniform(0.0, 1.0, (n, 3)) * [edge, 0.1, edge]
+    vel = rng.normal(0.0, 0.1, (n, 3))
+    mat = rng.integers(0, materials, n)
+    p = gpu.SphParams.defaults()
+    p.bounds_min, p.bounds_max = (0.0,) * 3, (max(1.0, edge),) * 3
+    if materials == 3:
+        p.visc_k, p.visc_n = [3.5, 2.0, 5.0], [1.0, 0.7, 1.3]
+    mass = scenes.lattice_mass(0.1)
+    ow = O.OracleWorld(p, threads=O.max_threads())
+    ow.add_particles(pos, mass, vel=vel, material=mat)
+    ow.step(0.001)
+    outs = []
+    for masks in (1, 1, 0):
+        w = gpu.FluidWorld(p, "comp")
+        w.set_tuning(dense_masks=masks)
+        w.add_particles(pos, mass, vel=vel, material=mat)
+        w.step(0.001)
+        w.synchronize()
+        if masks:  # a second step from the same state finds the mask buffer grown
+            w.set(gpu.FIELD_POS, pos)
+            w.set(gpu.FIELD_VEL, vel)
+            w.step(0.001)
+        outs.append({k: getattr(w, k).copy() for k in FIELDS})
+    for o in outs[1:]:
+        for k in FIELDS:
+            assert_bits_equal(o[k], outs[0][k], k)
+    rho = ow.get(O.F_RHO)
+    assert np.max(np.abs(outs[0]["rho"] - rho) / rho) <= 1e-5
+    acc = ow.get(O.F_ACC)
+    assert np.max(np.abs(outs[0]["acc"] - acc)) <= 1e-3 * np.max(np.abs(acc))
