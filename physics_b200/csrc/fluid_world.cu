@@ -510,7 +510,6 @@ void FluidWorld::free_all() {
   dfree(b_.mu);
   dfree(b_.cpos);
   dfree(b_.rec);
-  dfree(b_.search);
   dfree(b_.cvel);
   dfree(b_.cmr);
   dfree(b_.nbr);
@@ -599,8 +598,6 @@ void FluidWorld::ensure_capacity(size_t n) {
   dgrow(b_.nbr_count, 0, cap, s);
   dfree(b_.nbr);
   dfree(b_.rec);
-  dfree(b_.search);
-  if (prec_ == Precision::F64Plain) dfree(b_.cpos);
   dfree(b_.nbr16);
   dfree(b_.sorted_cell);
   dfree(b_.tile_of);
@@ -616,7 +613,7 @@ void FluidWorld::ensure_capacity(size_t n) {
   dgrow(b_.rank, 0, cap, s);
   dgrow(b_.tmp, 0, cap, s);
   dgrow(b_.perm, 0, cap, s);
-  dgrow(b_.stage, 0, 8 * cap, s);
+  dgrow(b_.stage, 0, 8 * ((cap + 31) / 32 * 32), s);
   b_.capacity = (int)cap;
   ++alloc_gen_;
   ensure_mode_buffers();
@@ -630,10 +627,8 @@ void FluidWorld::ensure_mode_buffers() {
   const bool tiled = prec_ == Precision::F32Comp && comp_tile_ > 0;
   if (!tiled && !b_.nbr) dalloc(b_.nbr, (size_t)kMaxNeighbors * cap);
   if (prec_ == Precision::F64Plain) {
-    if (!b_.rec) dalloc(b_.rec, (size_t)kPlainRec * cap);
-    if (!b_.cpos) dalloc(b_.cpos, cap);
+    if (!b_.rec) dalloc(b_.rec, plain_doubles(cap));
     if (!b_.sorted_cell) dalloc(b_.sorted_cell, cap);
-    if (!b_.search) dalloc(b_.search, (cap + 31) / 32 * (size_t)kSearchRecord);
   }
   if (tiled) {
     if (!b_.nbr16) dalloc(b_.nbr16, (size_t)kMaxNeighbors * cap);
@@ -2285,16 +2280,16 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
       cuda_check(cudaGetLastError(), "adjoint step");
     }
     recomputing_ = false;
-    std::vector<double> host(6 * n);
     launch_interleave3(w.gx_ins[0], w.gx_ins[1], w.gx_ins[2], b_.stage, (int)n, s);
     launch_interleave3(w.gv_ins[0], w.gv_ins[1], w.gv_ins[2], b_.stage + 3 * n, (int)n, s);
     double pa[2] = {0.0, 0.0};
-    cuda_check(cudaMemcpyAsync(host.data(), b_.stage, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, s),
-               "gradient read");
+    if (gx0)
+      cuda_check(cudaMemcpyAsync(gx0, b_.stage, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s), "gradient read");
+    if (gv0)
+      cuda_check(cudaMemcpyAsync(gv0, b_.stage + 3 * n, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s),
+                 "gradient read");
     cuda_check(cudaMemcpyAsync(pa, w.param_acc, sizeof(pa), cudaMemcpyDeviceToHost, s), "gradient read");
     cuda_check(cudaStreamSynchronize(s), "gradient sync");
-    if (gx0) std::memcpy(gx0, host.data(), 3 * n * sizeof(double));
-    if (gv0) std::memcpy(gv0, host.data() + 3 * n, 3 * n * sizeof(double));
     if (gparams) {
       gparams[0] = pa[0];
       gparams[1] = pa[1];

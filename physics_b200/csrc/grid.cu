@@ -1126,7 +1126,7 @@ void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, int block) 
   g.queue = c.tile ? b.queue : nullptr;
   g.inv_cell = c.inv_cell;
   g.h0 = c.h0;
-  g.fpos = c.plain ? b.cpos : nullptr;
+  g.fpos = c.plain ? reinterpret_cast<float4*>(b.rec + (size_t)kPlainRec * b.capacity) : nullptr;
   g.rec = c.plain ? b.rec : nullptr;
   g.unsafe = b.flags + 1;
   g.origin[0] = (double)c.bx0 * c.h0;

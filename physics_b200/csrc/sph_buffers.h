@@ -39,13 +39,11 @@ struct DevBuffers {
   double* xsph[3] = {};
   double* mu = nullptr;
   // f64 plain form: packed pair operands in three arrays of `capacity`
-  // records: x y z mass | vx vy vz rho | p/rho^2 1/rho.
+  // records: x y z mass | vx vy vz rho | p/rho^2 1/rho, then box-relative f32
+  // x, y, z with the z cell key, and the neighbour search's words per group
+  // (plain_doubles doubles in all).
   double* rec = nullptr;
-  // f64 plain form: the neighbour search's records (kSearchRecord words per
-  // group of 32 slots).
-  uint32_t* search = nullptr;
-  // f32-compensated form: per-particle packed operands.  (The f64 plain form
-  // keeps box-relative f32 x, y, z and the z cell key in cpos.)
+  // f32-compensated form: per-particle packed operands.
   float4* cpos = nullptr;  // cell-local x, y, z (f32) and mass
   float4* cvel = nullptr;  // vx, vy, vz (f32) and p/rho^2 (f32)
   float* cmr = nullptr;    // mass/rho (f32)
@@ -107,7 +105,8 @@ struct DevBuffers {
   uint32_t* block_sums = nullptr;
   int block_sums_capacity = 0;
   // Insertion-order staging for uploads and downloads (f64 and u32 views).
-  double* stage = nullptr;   // 8 * capacity doubles
+  // (The f64 plain step keeps the search's candidate words there.)
+  double* stage = nullptr;   // 8 * capacity doubles, capacity rounded up to 32
   // [0] error bits, [1] f64 plain step outside the reciprocals' safe range,
   // [2] the sort's large-cell count, [3] its barrier arrivals, [4] whether a
   // bucket is crowded, [6..7] mask_ctl; zeroed by one memset per step (device).

@@ -32,10 +32,13 @@ constexpr int kStagedNeighbors = 40;
 // of 4, 4 and 2).
 constexpr int kPlainRec = 10;
 // f64 plain form: 32-candidate words the neighbour search keeps per group of
-// 32 slots (512 candidates; a group of a column at rest density has ~215), and
-// the u32 words of a group's record.
+// 32 slots (512 candidates; a group of a column at rest density has ~215).
+// Candidate words live in the staging buffer (64 bytes per particle).
 constexpr int kSearchWords = 16;
-constexpr int kSearchRecord = 2 * kSearchWords * 32 + 2;
+// The buffer of packed operands (doubles): kPlainRec per slot, then the f32
+// positions (2 per slot), then the groups' words (1 per group).
+constexpr size_t plain_group_offset(size_t cap) { return (kPlainRec + 2) * cap; }
+constexpr size_t plain_doubles(size_t cap) { return plain_group_offset(cap) + (cap + 31) / 32; }
 
 // Tiled form: by default a tile whose occupied cells hold more than this many
 // particles on average goes to the dense-cell passes even when its halo could

@@ -58,8 +58,10 @@ struct PlainArgs {
   const float4* __restrict__ fpos;  // box-relative f32 position, z cell (bits)
   const uint32_t* __restrict__ sorted_cell;
   // The search's record per group of 32 slots: kSearchWords * 32 candidate
-  // words, kSearchWords * 32 hit words, and (hit words used, lanes that walk
-  // their 27 cells themselves).
+  // words, kSearchWords rows of hit words (one word per slot and row, rows of
+  // `stride`), and (hit words used, lanes that walk their 27 cells
+  // themselves).  The hit rows are the neighbour lists' last rows: a group's
+  // hits are read before its lists are written.
   uint32_t* cand;
   uint32_t* hits;
   uint2* group;
@@ -200,7 +202,8 @@ __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_search_plain
   const int bz = __float_as_int(own.w);
   const int col = (int)cell - bz;  // first cell of the column
   uint32_t* slots = a.cand + (size_t)group * (kSearchWords * 32);
-  uint32_t* hits = a.hits + (size_t)group * (kSearchWords * 32);
+  uint32_t* hits = a.hits + (size_t)group * 32 + lane;
+  const bool own_slot = group * 32 + lane < c.n;
   uint32_t words = 0;
   unsigned todo = __ballot_sync(0xffffffffu, inside), walkers = 0;
   bool sparse_known = false;
@@ -274,7 +277,8 @@ __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_search_plain
       if (m + add > (uint32_t)kBatch || !more) {
         filter_batch(st, m, seg);
         const uint32_t w1 = (m + 31u) >> 5;
-        for (uint32_t w = 0; w < w1; ++w) hits[(words + w) * 32u + lane] = mine ? st.hits[w][lane] : 0u;
+        if (own_slot)
+          for (uint32_t w = 0; w < w1; ++w) hits[(size_t)(words + w) * a.stride] = mine ? st.hits[w][lane] : 0u;
         __syncwarp();
         words += w1;
         m = 0;
@@ -336,10 +340,10 @@ __global__ void __launch_bounds__(kDensityWarps * 32, kDensityCtas) k_density_pl
   const uint2 rec = a.group[group];
   {
     const uint32_t* slots = a.cand + (size_t)group * (kSearchWords * 32) + lane;
-    const uint32_t* hits = a.hits + (size_t)group * (kSearchWords * 32) + lane;
+    const uint32_t* hits = a.hits + ii;
 #pragma unroll 4
     for (uint32_t w = 0; w < rec.x; ++w) {
-      st.hits[w][lane] = hits[w * 32u];
+      st.hits[w][lane] = valid ? hits[(size_t)w * a.stride] : 0u;
       st.slot[w * 32u + lane] = slots[w * 32u];
     }
     st.hits[rec.x][lane] = 1u;
@@ -779,14 +783,11 @@ static float plain_cull2(const StepConsts& c) {
 void launch_plain_passes(const StepConsts& c, DevBuffers& b, cudaStream_t s, const PassEvents& ev) {
   const ParticleConsts& pc = b.pc[b.cur];
   PlainArgs a;
-  a.fpos = b.cpos;
+  a.fpos = reinterpret_cast<const float4*>(b.rec + (size_t)kPlainRec * b.capacity);
   a.sorted_cell = b.sorted_cell;
-  {
-    const size_t groups = ((size_t)b.capacity + 31) / 32;
-    a.cand = b.search;
-    a.hits = a.cand + groups * (kSearchWords * 32);
-    a.group = reinterpret_cast<uint2*>(a.hits + groups * (kSearchWords * 32));
-  }
+  a.cand = reinterpret_cast<uint32_t*>(b.stage);
+  a.hits = b.nbr + (size_t)(kMaxNeighbors - kSearchWords) * b.capacity;
+  a.group = reinterpret_cast<uint2*>(b.rec + plain_group_offset(b.capacity));
   a.rec0 = b.rec;
   a.rec1 = b.rec + 4 * (size_t)b.capacity;
   a.rec2 = reinterpret_cast<double2*>(b.rec + 8 * (size_t)b.capacity);
