@@ -513,21 +513,38 @@ __global__ void __launch_bounds__(kCT) k_heat_particles(StepConsts c, HeatArgs h
 }
 
 // Stable LSD radix sort of 32-bit keys with a 32-bit payload, 8 bits a pass.
-// Block b owns keys [b * kRTile, (b + 1) * kRTile); hist[d * nblocks + b]
+// Block b owns `rounds` times kRT consecutive keys; hist[d * nblocks + b]
 // counts digit d in block b, and its exclusive scan (digit-major) is the
 // first output slot of block b's keys of digit d.
 constexpr int kRT = 256;
 constexpr int kRRounds = 32;
-constexpr int kRTile = kRT * kRRounds;
+// Rounds per block: about 64 blocks, at most kRRounds rounds. A block of 32
+// rounds takes 50 us a pass, and 32,768 keys had four of them: with 64 blocks
+// of two rounds a pass is 8 us, and points, heat and a step there take 584 us
+// together instead of 643. More blocks only lengthen the histogram that one
+// block scans (9 us at 64).
+int radix_rounds(size_t n) {
+  return (int)std::min<size_t>(kRRounds, std::max<size_t>(1, (n + (size_t)kRT * 64 - 1) / ((size_t)kRT * 64)));
+}
+int radix_blocks(size_t n) {
+  const size_t tile = (size_t)kRT * radix_rounds(n);
+  return (int)((n + tile - 1) / tile);
+}
+// The most blocks that any count up to n takes (fewer keys can take more
+// blocks, where the rounds go up by one).
+size_t radix_blocks_most(size_t n) {
+  const size_t one = (n + kRT - 1) / kRT, all = (size_t)kRT * kRRounds;
+  return std::max(std::min<size_t>(one, 64), (n + all - 1) / all);
+}
 
 __global__ void __launch_bounds__(kRT) k_radix_hist(const uint32_t* key, int n, int shift, uint32_t* hist,
-                                                     int nblocks) {
+                                                     int nblocks, int rounds) {
   __shared__ uint32_t s_h[256];
   const int t = threadIdx.x;
   s_h[t] = 0;
   __syncthreads();
-  const int base = blockIdx.x * kRTile;
-  for (int r = 0; r < kRRounds; ++r) {
+  const int base = blockIdx.x * kRT * rounds;
+  for (int r = 0; r < rounds; ++r) {
     const int e = base + r * kRT + t;
     if (e < n) atomicAdd(&s_h[(key[e] >> shift) & 255u], 1u);
   }
@@ -538,24 +555,30 @@ __global__ void __launch_bounds__(kRT) k_radix_hist(const uint32_t* key, int n, 
 // In-place exclusive scan of len values by one block (each thread scans a
 // contiguous run).
 __global__ void __launch_bounds__(1024) k_scan_single(uint32_t* v, int len) {
-  __shared__ uint32_t s_part[1024];
-  const int t = threadIdx.x;
+  __shared__ uint32_t s_part[32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int per = (len + 1023) / 1024;
   const int lo = min(t * per, len), hi = min(lo + per, len);
   uint32_t sum = 0;
+#pragma unroll 4
   for (int i = lo; i < hi; ++i) sum += v[i];
-  s_part[t] = sum;
+  uint32_t incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_part[warp] = incl;
   __syncthreads();
-  if (t == 0) {
-    uint32_t run = 0;
-    for (int k = 0; k < 1024; ++k) {
-      const uint32_t x = s_part[k];
-      s_part[k] = run;
-      run += x;
+  if (warp == 0) {
+    uint32_t w = s_part[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
     }
+    s_part[lane] = w;
   }
   __syncthreads();
-  uint32_t run = s_part[t];
+  uint32_t run = incl - sum + (warp > 0 ? s_part[warp - 1] : 0u);
   for (int i = lo; i < hi; ++i) {
     const uint32_t x = v[i];
     v[i] = run;
@@ -568,15 +591,15 @@ __global__ void __launch_bounds__(1024) k_scan_single(uint32_t* v, int len) {
 // of this round) + (earlier lanes of its warp).
 __global__ void __launch_bounds__(kRT) k_radix_scatter(const uint32_t* key_in, const uint32_t* val_in,
                                                         uint32_t* key_out, uint32_t* val_out, int n, int shift,
-                                                        const uint32_t* off, int nblocks) {
+                                                        const uint32_t* off, int nblocks, int rounds) {
   __shared__ uint32_t s_w[kRT / 32][256];
   __shared__ uint32_t s_run[256];
   __shared__ uint32_t s_base[256];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   s_run[t] = 0;
   s_base[t] = off[(size_t)t * nblocks + blockIdx.x];
-  const int base = blockIdx.x * kRTile;
-  for (int r = 0; r < kRRounds; ++r) {
+  const int base = blockIdx.x * kRT * rounds;
+  for (int r = 0; r < rounds; ++r) {
     for (int w = 0; w < kRT / 32; ++w) s_w[w][t] = 0;
     __syncthreads();
     const int e = base + r * kRT + t;
@@ -989,7 +1012,7 @@ __global__ void __launch_bounds__(kCT) k_body_contacts(StepConsts c, BodyArgs a,
 
 size_t couple_bodies_scratch_bytes(int n, int nb, uint64_t n_data, uint64_t n_faces) {
   return (size_t)nb * sizeof(PhyCoupleBody) + 8 * (size_t)nb + 8 * (size_t)n_data + 4 * (size_t)n_faces +
-         20 * (size_t)n + 1024 * (size_t)((n + kRTile - 1) / kRTile) + 512;
+         20 * (size_t)n + 1024 * radix_blocks_most((size_t)n) + 512;
 }
 
 int launch_couple_bodies(const StepConsts& c, DevBuffers& b, const CoupleBodiesLaunch& l, cudaStream_t s) {
@@ -997,7 +1020,7 @@ int launch_couple_bodies(const StepConsts& c, DevBuffers& b, const CoupleBodiesL
   if (cudaMemcpyAsync(l.scratch, l.bodies, (size_t)l.nb * sizeof(PhyCoupleBody), cudaMemcpyHostToDevice, s) !=
       cudaSuccess)
     return -1;
-  const size_t nbk = (size_t)((n + kRTile - 1) / kRTile);
+  const size_t nbk = radix_blocks_most((size_t)n);
   unsigned char* base = l.scratch;
   PhyCoupleBody* bodies = reinterpret_cast<PhyCoupleBody*>(base);
   double* displaced = reinterpret_cast<double*>(bodies + l.nb);
@@ -1032,13 +1055,13 @@ int launch_couple_bodies(const StepConsts& c, DevBuffers& b, const CoupleBodiesL
     return -1;
   uint32_t *kin = key0, *kout = key1, *vin = val0, *vout = val1;
   if (m > 1) {
-    const int mb = (int)((m + kRTile - 1) / kRTile);
+    const int mb = radix_blocks((size_t)m), rounds = radix_rounds((size_t)m);
     int bits = 0;
     while (bits < 32 && ((uint32_t)(n - 1) >> bits) != 0u) ++bits;
     for (int shift = 0; shift < bits; shift += 8) {
-      k_radix_hist<<<mb, kRT, 0, s>>>(kin, (int)m, shift, hist, mb);
+      k_radix_hist<<<mb, kRT, 0, s>>>(kin, (int)m, shift, hist, mb, rounds);
       k_scan_single<<<1, 1024, 0, s>>>(hist, 256 * mb);
-      k_radix_scatter<<<mb, kRT, 0, s>>>(kin, vin, kout, vout, (int)m, shift, hist, mb);
+      k_radix_scatter<<<mb, kRT, 0, s>>>(kin, vin, kout, vout, (int)m, shift, hist, mb, rounds);
       uint32_t* t = kin;
       kin = kout;
       kout = t;
@@ -1059,7 +1082,7 @@ int launch_couple_bodies(const StepConsts& c, DevBuffers& b, const CoupleBodiesL
 }
 
 size_t couple_heat_scratch_bytes(int n, uint64_t cells) {
-  const size_t nb = (size_t)((n + kRTile - 1) / kRTile);
+  const size_t nb = radix_blocks_most((size_t)n);
   return 16 * (size_t)cells + 8 * (size_t)n + 16 * (size_t)n + 1024 * nb + 256;
 }
 
@@ -1067,7 +1090,7 @@ void launch_couple_heat(const StepConsts& c, DevBuffers& b, const HeatGrid& g, u
                         cudaStream_t s) {
   const int n = c.n;
   const uint64_t cells = g.nx * g.ny * g.nz;
-  const size_t nb = (size_t)((n + kRTile - 1) / kRTile);
+  const int nb = radix_blocks((size_t)n), rounds = radix_rounds((size_t)n);
   double* u = reinterpret_cast<double*>(scratch);
   double* src = u + cells;
   double* val = src + cells;
@@ -1112,9 +1135,9 @@ void launch_couple_heat(const StepConsts& c, DevBuffers& b, const HeatGrid& g, u
   k_iota_u32<<<blocks, kCT, 0, s>>>(id0, n);
   uint32_t *kin = key0, *kout = key1, *iin = id0, *iout = id1;
   for (int shift = 0; shift < bits; shift += 8) {
-    k_radix_hist<<<(int)nb, kRT, 0, s>>>(kin, n, shift, hist, (int)nb);
-    k_scan_single<<<1, 1024, 0, s>>>(hist, (int)(256 * nb));
-    k_radix_scatter<<<(int)nb, kRT, 0, s>>>(kin, iin, kout, iout, n, shift, hist, (int)nb);
+    k_radix_hist<<<nb, kRT, 0, s>>>(kin, n, shift, hist, nb, rounds);
+    k_scan_single<<<1, 1024, 0, s>>>(hist, 256 * nb);
+    k_radix_scatter<<<nb, kRT, 0, s>>>(kin, iin, kout, iout, n, shift, hist, nb, rounds);
     uint32_t* tk = kin;
     kin = kout;
     kout = tk;
