@@ -352,7 +352,9 @@ int32_t phy_fluid_autotune_horizon(PhyWorldHandle *w, uint32_t sub, double dt, u
  * `checkpoint_every` steps; parameters must stay unchanged and body
  * accelerations unset while recording.  phy_fluid_step_backward runs the
  * reverse sweep over all recorded steps, re-running each segment forward
- * from its checkpoint (the f64 plain step repeats bit-exactly): given
+ * from its checkpoint (the f64 plain step repeats bit-exactly; the first
+ * steps of an f64 tape, up to 512 MiB of them, are recorded as they run and
+ * not run again): given
  * dL/dpos_T and dL/dvel_T (3n doubles each, insertion order, xyz
  * interleaved; NULL = zero) it writes dL/dpos_0, dL/dvel_0 (3n each) and
  * grad_params2 = {dL/d stiffness, dL/d visc_k[0]} (any output may be NULL).

@@ -976,6 +976,7 @@ void FluidWorld::add_particles(size_t m, const double* pos, const double* vel, c
   if (!pos || !mass) throw std::invalid_argument("add_particles: pos and mass are required");
   if (!scenes_.empty())
     throw std::invalid_argument("add_particles: the world holds batched scenes (clear_scenes first)");
+  tape_.direct = -1;
   ensure_capacity(n_ + m);
   // Staging layout: pos 3m | vel 3m | mass m | material m (as doubles).
   std::vector<double> st(8 * m, 0.0);
@@ -1193,6 +1194,7 @@ void FluidWorld::set_field(int field, const double* in) {
   int nc = components(field);
   if (nc == 0) throw std::invalid_argument("set_field: unknown field");
   if (n_ == 0) return;
+  tape_.direct = -1;  // a sweep re-runs the steps from their checkpoints
   const int n = (int)n_;
   ParticleConsts& pc = b_.pc[b_.cur];
   double* st = b_.stage;
@@ -1338,6 +1340,8 @@ StepConsts FluidWorld::step_impl(double dt) {
     tape_.dts.push_back(dt);
   }
   StepConsts c = prepare_step(dt);
+  const bool direct = tape_.on && !recomputing_ && direct_slot(c);
+  if (direct) set_tape_outputs(true);
   PassEvents pe;
   cudaEvent_t* ev = nullptr;
   if (timing_) {
@@ -1351,8 +1355,18 @@ StepConsts FluidWorld::step_impl(double dt) {
     pe.after_prep = ev[2];
     pe.after_density = ev[3];
   }
-  enqueue_step(c, pe, ev);
-  if (ev) cuda_check(cudaEventRecord(ev[4], stream_), "event");
+  try {
+    enqueue_step(c, pe, ev);
+    if (ev) cuda_check(cudaEventRecord(ev[4], stream_), "event");
+    if (direct) {
+      record_step(c, (int)tape_.dts.size() - 1, nullptr);
+      ++tape_.direct;
+    }
+  } catch (...) {
+    if (direct) set_tape_outputs(false);
+    throw;
+  }
+  if (direct) set_tape_outputs(false);
   return c;
 }
 
@@ -1637,6 +1651,7 @@ std::vector<TuneTrial> FluidWorld::autotune(double dt, int steps, int horizon) {
   if (n_ == 0 || steps <= 0) return trials;
   if (timing_) throw std::invalid_argument("autotune: phase timing is on");
   if (horizon < 0) throw std::invalid_argument("autotune: negative horizon");
+  tape_.direct = -1;
   const bool tiled = prec_ == Precision::F32Comp && comp_tile_ > 0;
   const int max_per_sm = tiled ? tiled_max_ctas_per_sm() : 1;
   std::vector<std::pair<LaunchTuning, int>> cands;
@@ -2007,10 +2022,23 @@ void FluidWorld::tape_clear() {
   tape_.nckpt = 0;
   tape_.dts.clear();
   tape_.on = false;
-  size_t bytes = (6 * tape_.ckpt.size() + 22 * adj_slot_f_.size() + (adj_work_ ? kAdjWorkArrays : 0)) * tape_.n * sizeof(double) +
+  size_t slots = 0;
+  for (const double* p : adj_slot_f_) slots += p ? 1 : 0;
+  size_t bytes = (6 * tape_.ckpt.size() + 22 * slots + (adj_work_ ? kAdjWorkArrays : 0)) * tape_.n * sizeof(double) +
                  comp_rec_cap_ * sizeof(uint32_t);
   for (size_t u : adj_slot_ucount_) bytes += u * sizeof(uint32_t);
   for (size_t q : snap_bytes_) bytes += q;
+  // Over it, the slots past one interval go first (recorded steps, not the
+  // sweep's own).
+  while (bytes > kKeepBytes && adj_slot_f_.size() > (size_t)tape_.every) {
+    bytes -= (adj_slot_f_.back() ? 22 * tape_.n * sizeof(double) : 0) + adj_slot_ucount_.back() * sizeof(uint32_t);
+    dfree(adj_slot_f_.back());
+    dfree(adj_slot_u_.back());
+    adj_slot_f_.pop_back();
+    adj_slot_u_.pop_back();
+    adj_slot_ucount_.pop_back();
+    adj_slot_c_.pop_back();
+  }
   if (bytes > kKeepBytes) tape_free();
   for (auto& c : snap_count_) c = 0;  // the saved states are void
 }
@@ -2030,6 +2058,7 @@ void FluidWorld::tape_free() {
   adj_slot_f_.clear();
   adj_slot_u_.clear();
   adj_slot_ucount_.clear();
+  adj_slot_c_.clear();
   release_snapshot();
 }
 
@@ -2045,6 +2074,7 @@ void FluidWorld::tape_begin(int every) {
   tape_.n = n_;
   tape_.nckpt = 0;
   tape_.dts.clear();
+  tape_.direct = 0;
   tape_.every = every;
   tape_.params = params.to_c();
   save_checkpoint();
@@ -2053,41 +2083,131 @@ void FluidWorld::tape_begin(int every) {
 
 namespace {
 
-// Device arrays of one recorded step (sorted order) plus its launch constants.
-struct TapeSlot {
-  double* f = nullptr;       // 22 arrays of n doubles
-  uint32_t* u = nullptr;     // mat, id, nbr_count (n each), nbr (96 n), cell_start
-  StepConsts c;
-  AdjTape view(size_t n) const {
-    AdjTape t;
-    double* q = f;
-    auto take = [&]() {
-      double* r = q;
-      q += n;
-      return r;
-    };
-    for (int k = 0; k < 3; ++k) t.x[k] = take();
-    for (int k = 0; k < 3; ++k) t.v[k] = take();
-    t.mass = take();
-    t.rho = take();
-    t.p = take();
-    t.pr2 = take();
-    t.mr = take();
-    for (int k = 0; k < 3; ++k) t.acc[k] = take();
-    for (int k = 0; k < 3; ++k) t.xsph[k] = take();
-    t.mu = take();
-    for (int k = 0; k < 3; ++k) t.fv[k] = take();
-    t.shear = take();
-    t.mat = u;
-    t.id = u + n;
-    t.nbr_count = u + 2 * n;
-    t.nbr = u + 3 * n;
-    t.cell_start = u + (3 + (size_t)kMaxNeighbors) * n;
-    return t;
-  }
-};
+// Device arrays of one recorded step (sorted order): f holds 22 arrays of n
+// doubles; u mat, id, nbr_count (n each), nbr (96 n), cell_start.
+AdjTape tape_view(double* f, uint32_t* u, size_t n) {
+  AdjTape t;
+  auto take = [&]() {
+    double* r = f;
+    f += n;
+    return r;
+  };
+  for (int k = 0; k < 3; ++k) t.x[k] = take();
+  for (int k = 0; k < 3; ++k) t.v[k] = take();
+  t.mass = take();
+  t.rho = take();
+  t.p = take();
+  t.pr2 = take();
+  t.mr = take();
+  for (int k = 0; k < 3; ++k) t.acc[k] = take();
+  for (int k = 0; k < 3; ++k) t.xsph[k] = take();
+  t.mu = take();
+  for (int k = 0; k < 3; ++k) t.fv[k] = take();
+  t.shear = take();
+  t.mat = u;
+  t.id = u + n;
+  t.nbr_count = u + 2 * n;
+  t.nbr = u + 3 * n;
+  t.cell_start = u + (3 + (size_t)kMaxNeighbors) * n;
+  return t;
+}
+
+size_t tape_ucount(const StepConsts& c) { return (3 + (size_t)kMaxNeighbors) * (size_t)c.n + (size_t)c.ncells + 2; }
 
 }  // namespace
+
+// Makes slot `si` large enough for a step with constants c.
+void FluidWorld::ensure_slot(const StepConsts& c, int si) {
+  if ((int)adj_slot_f_.size() <= si) {
+    adj_slot_f_.resize(si + 1, nullptr);
+    adj_slot_u_.resize(si + 1, nullptr);
+    adj_slot_ucount_.resize(si + 1, 0);
+    adj_slot_c_.resize(si + 1);
+  }
+  if (!adj_slot_f_[si]) dalloc(adj_slot_f_[si], 22 * n_);
+  if (adj_slot_ucount_[si] < tape_ucount(c)) {
+    adj_slot_ucount_[si] = 0;
+    dalloc(adj_slot_u_[si], tape_ucount(c));
+    adj_slot_ucount_[si] = tape_ucount(c);
+  }
+}
+
+void FluidWorld::ensure_adj_work() {
+  if (!adj_work_) dalloc(adj_work_, kAdjWorkArrays * n_ + 2 + 2 * kAdjSumBlocks + 1);
+}
+
+// The force pass's viscous and shear sums, kept for the reverse step, in the
+// last four arrays of the work buffer.
+void FluidWorld::set_tape_outputs(bool on) {
+  double* q = on ? adj_work_ + (kAdjWorkArrays - 4) * n_ : nullptr;
+  for (int k = 0; k < 3; ++k) b_.tape_fv[k] = on ? q + k * n_ : nullptr;
+  b_.tape_shear = on ? q + 3 * n_ : nullptr;
+}
+
+// Whether the step being taken is recorded as it runs: an f64 step, every
+// earlier one recorded too, and the recorded steps within kDirectBytes.  The
+// reverse sweep then need not run it again from a checkpoint (65,536
+// particles: the copy takes 12 us, the step 90; ten steps and their sweep
+// 3,470 -> 2,470 us).  Where memory runs out the
+// step is left to the sweep.
+bool FluidWorld::direct_slot(const StepConsts& c) {
+  constexpr size_t kDirectBytes = size_t(1) << 29;
+  if (prec_ != Precision::F64Plain || tape_.direct != (int)tape_.dts.size() - 1) return false;
+  const size_t slot = 22 * n_ * sizeof(double) + tape_ucount(c) * sizeof(uint32_t);
+  if ((size_t)(tape_.direct + 1) * slot > kDirectBytes) return false;
+  try {
+    ensure_adj_work();
+    ensure_slot(c, tape_.direct);
+  } catch (const std::exception&) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
+// Copies the step just enqueued (constants c) to slot `si`.
+AdjTape FluidWorld::record_step(const StepConsts& c, int si, uint32_t* slot_of) {
+  const size_t n = n_;
+  ensure_slot(c, si);
+  adj_slot_c_[si] = c;
+  const AdjTape v = tape_view(adj_slot_f_[si], adj_slot_u_[si], n);
+  const ParticleConsts& q = b_.pc[b_.cur];
+  TapeCopy tc;
+  int k = 0;
+  auto add = [&](const double* dst, const double* src) {
+    tc.dst[k] = const_cast<double*>(dst);
+    tc.src[k] = src;
+    ++k;
+  };
+  for (int a = 0; a < 3; ++a) add(v.x[a], b_.pv0[a]);
+  for (int a = 0; a < 3; ++a) add(v.v[a], b_.pv0[3 + a]);
+  add(v.mass, q.mass);
+  add(v.rho, b_.rho);
+  add(v.p, b_.p);
+  add(v.pr2, b_.pr2);
+  add(v.mr, b_.mr);
+  for (int a = 0; a < 3; ++a) add(v.acc[a], b_.acc[a]);
+  for (int a = 0; a < 3; ++a) add(v.xsph[a], b_.xsph[a]);
+  add(v.mu, b_.mu);
+  for (int a = 0; a < 3; ++a) add(v.fv[a], b_.tape_fv[a]);
+  add(v.shear, b_.tape_shear);
+  if (k != 22) throw std::logic_error("step_backward: tape layout");
+  tc.usrc[0] = q.mat;
+  tc.udst[0] = const_cast<uint32_t*>(v.mat);
+  tc.usrc[1] = q.id;
+  tc.udst[1] = const_cast<uint32_t*>(v.id);
+  tc.usrc[2] = b_.nbr_count;
+  tc.udst[2] = const_cast<uint32_t*>(v.nbr_count);
+  tc.nbr = b_.nbr;
+  tc.nbr_dst = const_cast<uint32_t*>(v.nbr);
+  tc.nbr_stride = b_.capacity;
+  tc.slot_of = slot_of;
+  k_tape_copy<<<dim3((unsigned)grid_for(n), kTapeParts), kThreads, 0, stream_>>>((int)n, tc);
+  cuda_check(cudaMemcpyAsync(const_cast<uint32_t*>(v.cell_start), b_.cell_start, ((size_t)c.ncells + 2) * 4,
+                             cudaMemcpyDeviceToDevice, stream_),
+             "tape copy");
+  return v;
+}
 
 void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, double* gv0, double* gparams) {
   const size_t n = n_;
@@ -2099,7 +2219,7 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
   // each), rbar, rbar_tot, cc, kk, the tape's fv and shear outputs (4): arrays
   // of n, then the two parameter accumulators with their partial sums.
   constexpr size_t kWorkArrays = kAdjWorkArrays;
-  if (!adj_work_) dalloc(adj_work_, kWorkArrays * n + 2 + 2 * kAdjSumBlocks + 1);
+  ensure_adj_work();
   double* work = adj_work_;
   AdjWork w;
   {
@@ -2121,19 +2241,17 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
     w.rbar_tot = take();
     w.cc = take();
     w.kk = take();
-    for (int k = 0; k < 3; ++k) b_.tape_fv[k] = take();
-    b_.tape_shear = take();
+    for (int k = 0; k < 4; ++k) (void)take();  // set_tape_outputs
+    set_tape_outputs(true);
     w.param_acc = q;
     w.sum_part = q + 2;
     w.sum_arrived = reinterpret_cast<unsigned*>(q + 2 + 2 * kAdjSumBlocks);
   }
-  const int nslots = std::min(tape_.every, std::max(T, 1));
-  std::vector<TapeSlot> slots(nslots);
-  if ((int)adj_slot_f_.size() < nslots) {
-    adj_slot_f_.resize(nslots, nullptr);
-    adj_slot_u_.resize(nslots, nullptr);
-    adj_slot_ucount_.resize(nslots, 0);
-  }
+  // Steps recorded as they ran are in the first slots; the parameters must be
+  // those of the recording, as a re-run takes the current ones.
+  const PhySphParams now = params.to_c();
+  if (std::memcmp(&now, &tape_.params, sizeof(now)) != 0) tape_.direct = -1;
+  const int ndirect = std::max(tape_.direct, 0);
   // A compensated world is differentiated along its own trajectory: each
   // re-run step first takes an f64 plain recording step from the same state
   // (the records of the exact step map at that state), then returns to the
@@ -2151,13 +2269,13 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
     slot_of = comp_rec_;
   }
   auto cleanup = [&]() {
-    for (int k = 0; k < 3; ++k) b_.tape_fv[k] = nullptr;
-    b_.tape_shear = nullptr;
+    set_tape_outputs(false);
     recomputing_ = false;
     prec_ = form;
   };
   try {
-    snapshot(false);  // the world returns to x_T, v_T afterwards
+    const bool rerun = ndirect < T;
+    if (rerun) snapshot(false);  // the world returns to x_T, v_T afterwards
     // Seeds (insertion order): dL/dx_T, dL/dv_T.
     cuda_check(cudaMemsetAsync(w.gx_ins[0], 0, 6 * n * sizeof(double), s), "seed clear");
     cuda_check(cudaMemsetAsync(w.param_acc, 0, (2 + 2 * kAdjSumBlocks + 1) * sizeof(double), s), "param clear");
@@ -2176,6 +2294,12 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
     const int nseg = (T + every - 1) / every;
     for (int seg = nseg - 1; seg >= 0; --seg) {
       const int t0 = seg * every, t1 = std::min(T, t0 + every);
+      if (t1 <= ndirect) {
+        for (int t = t1 - 1; t >= t0; --t)
+          launch_adjoint_step(adj_slot_c_[t], tape_view(adj_slot_f_[t], adj_slot_u_[t], n), w, s);
+        cuda_check(cudaGetLastError(), "adjoint step");
+        continue;
+      }
       // Restore checkpoint `seg` and re-run its steps, recording each.
       const ParticleConsts& pc = b_.pc[b_.cur];
       const double* ck = tape_.ckpt[seg];
@@ -2183,60 +2307,13 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
       k_set_vec_by_id<<<grid_for(n), kThreads, 0, s>>>((int)n, pc.id, ck + 3 * n, b_.pv1[3], b_.pv1[4],
                                                        b_.pv1[5]);
       for (int t = t0; t < t1; ++t) {
-        TapeSlot& sl = slots[t - t0];
-        const int si = t - t0;
         if (comp) {
           // The f64 recording step from state t first.
           prec_ = Precision::F64Plain;
           ensure_mode_buffers();  // f64 neighbour lists, kept for later sweeps
         }
         const StepConsts c = step_impl(tape_.dts[t]);
-        const size_t ncs = (size_t)c.ncells + 2;
-        const size_t ucount = (3 + (size_t)kMaxNeighbors) * n + ncs;
-        if (!adj_slot_f_[si]) dalloc(adj_slot_f_[si], 22 * n);
-        if (adj_slot_ucount_[si] < ucount) {
-          dalloc(adj_slot_u_[si], ucount);
-          adj_slot_ucount_[si] = ucount;
-        }
-        sl.f = adj_slot_f_[si];
-        sl.u = adj_slot_u_[si];
-        sl.c = c;
-        const AdjTape v = sl.view(n);
-        const ParticleConsts& q = b_.pc[b_.cur];
-        TapeCopy tc;
-        int k = 0;
-        auto add = [&](const double* dst, const double* src) {
-          tc.dst[k] = const_cast<double*>(dst);
-          tc.src[k] = src;
-          ++k;
-        };
-        for (int a = 0; a < 3; ++a) add(v.x[a], b_.pv0[a]);
-        for (int a = 0; a < 3; ++a) add(v.v[a], b_.pv0[3 + a]);
-        add(v.mass, q.mass);
-        add(v.rho, b_.rho);
-        add(v.p, b_.p);
-        add(v.pr2, b_.pr2);
-        add(v.mr, b_.mr);
-        for (int a = 0; a < 3; ++a) add(v.acc[a], b_.acc[a]);
-        for (int a = 0; a < 3; ++a) add(v.xsph[a], b_.xsph[a]);
-        add(v.mu, b_.mu);
-        for (int a = 0; a < 3; ++a) add(v.fv[a], b_.tape_fv[a]);
-        add(v.shear, b_.tape_shear);
-        if (k != 22) throw std::logic_error("step_backward: tape layout");
-        tc.usrc[0] = q.mat;
-        tc.udst[0] = const_cast<uint32_t*>(v.mat);
-        tc.usrc[1] = q.id;
-        tc.udst[1] = const_cast<uint32_t*>(v.id);
-        tc.usrc[2] = b_.nbr_count;
-        tc.udst[2] = const_cast<uint32_t*>(v.nbr_count);
-        tc.nbr = b_.nbr;
-        tc.nbr_dst = const_cast<uint32_t*>(v.nbr);
-        tc.nbr_stride = b_.capacity;
-        tc.slot_of = slot_of;
-        k_tape_copy<<<dim3((unsigned)grid_for(n), kTapeParts), kThreads, 0, s>>>((int)n, tc);
-        cuda_check(cudaMemcpyAsync(const_cast<uint32_t*>(v.cell_start), b_.cell_start, ncs * 4,
-                                   cudaMemcpyDeviceToDevice, s),
-                   "tape copy");
+        const AdjTape v = record_step(c, ndirect + t - t0, slot_of);
         if (comp) {
           // Back to state t for the compensated step to state t+1: the
           // recording step left state t, sorted, in pv0 with the constants of
@@ -2276,7 +2353,10 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
           cuda_check(cudaGetLastError(), "tape override");
         }
       }
-      for (int t = t1 - 1; t >= t0; --t) launch_adjoint_step(slots[t - t0].c, slots[t - t0].view(n), w, s);
+      for (int t = t1 - 1; t >= t0; --t) {
+        const int si = ndirect + t - t0;
+        launch_adjoint_step(adj_slot_c_[si], tape_view(adj_slot_f_[si], adj_slot_u_[si], n), w, s);
+      }
       cuda_check(cudaGetLastError(), "adjoint step");
     }
     recomputing_ = false;
@@ -2294,10 +2374,10 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
       gparams[0] = pa[0];
       gparams[1] = pa[1];
     }
-    snapshot(true);
+    if (rerun) snapshot(true);
   } catch (...) {
     cleanup();
-    if (snap_count_[0]) snapshot(true);
+    if (ndirect < T && snap_count_[0]) snapshot(true);
     throw;
   }
   cleanup();

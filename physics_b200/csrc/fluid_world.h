@@ -23,6 +23,8 @@
 
 namespace phy {
 
+struct AdjTape;
+
 struct Vec3 {
   double x, y, z;
 };
@@ -108,7 +110,8 @@ class FluidWorld {
   // state checkpoint every `every` steps; parameters must not change and
   // body accelerations must not be set while recording.  step_backward runs
   // the reverse sweep over the recorded steps, re-running each segment
-  // forward from its checkpoint: given dL/dx_T and dL/dv_T (insertion order,
+  // forward from its checkpoint unless its steps were recorded as they ran
+  // (direct_slot; the same bits): given dL/dx_T and dL/dv_T (insertion order,
   // xyz interleaved; null = zero) it returns dL/dx_0, dL/dv_0 and
   // {dL/d stiffness, dL/d visc_k[0]} (outputs may be null) and leaves the
   // world in its state x_T, v_T.  The tape is kept for further sweeps.
@@ -298,9 +301,15 @@ class FluidWorld {
     std::vector<double> dts;
     std::vector<double*> ckpt;  // pool; the first nckpt are this tape's
     size_t nckpt = 0;
+    int direct = -1;  // leading steps recorded as they ran; -1: none can be
     PhySphParams params;
   } tape_;
   void tape_free();
+  void ensure_slot(const StepConsts& c, int si);
+  void ensure_adj_work();
+  void set_tape_outputs(bool on);
+  bool direct_slot(const StepConsts& c);
+  AdjTape record_step(const StepConsts& c, int si, uint32_t* slot_of);
   // Reverse-sweep buffers kept between sweeps and tapes (tape_clear).
   double* adj_work_ = nullptr;
   uint32_t* comp_rec_ = nullptr;  // compensated adjoint: insertion index -> recorded slot
@@ -308,6 +317,7 @@ class FluidWorld {
   std::vector<double*> adj_slot_f_;
   std::vector<uint32_t*> adj_slot_u_;
   std::vector<size_t> adj_slot_ucount_;
+  std::vector<StepConsts> adj_slot_c_;
   bool recomputing_ = false;
   // Saved states (autotuner, reverse sweep): per slot one arena reused while
   // large enough.
