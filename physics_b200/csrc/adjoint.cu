@@ -35,9 +35,9 @@
 // reduction, so a gradient repeats bit-exactly run to run.
 //
 // The forward quantities the reverse needs (sorted state, rho, p, pi, m/rho,
-// acc, xsph, mu, fv and s, the cell ranges) are recorded by re-running the
-// forward step from checkpoints; the wall decisions are recomputed here with
-// the forward's exact operation order.
+// acc, xsph, mu, fv and s, the cell ranges) are recorded as the forward
+// steps run, or by re-running them from checkpoints; the wall decisions are
+// recomputed here with the forward's exact operation order.
 #include <cuda_runtime.h>
 
 #include "adjoint.h"
@@ -162,13 +162,19 @@ __global__ void __launch_bounds__(kThreads) k_adj_integrate(StepConsts c, AdjTap
 
 // Lanes per particle of the pair kernels: a particle's neighbours are dealt
 // round-robin to kLanes consecutive lanes of a warp, whose partial sums are
-// then combined by a fixed shuffle tree (deterministic).
-constexpr int kLanes = 4;
+// then combined by a fixed shuffle tree (deterministic).  Two lanes, since
+// more of them drift apart in their list rows (65,536 particles, force and
+// density pass: 75 + 26 us with one lane, 66 + 18 with two, 71 + 24 with four,
+// 91 + 30 with eight); four in small worlds, where the longest lane is what
+// takes the time (a whole reverse step with four and two lanes: 512 particles
+// 31 / 43 us, 3,920 36 / 42, 15,488 41 / 49, 26,656 50 / 56, 32,768 57 / 57,
+// 65,600 110 / 97, 196,608 252 / 230).
+constexpr int kLanesBelow = 30000;
 
 // Visits lane `q`'s share of the step's force/density neighbours of slot i:
 // its recorded list, or the 27 cells when the list overflowed (and, for a
 // particle outside the grid box, nothing).  `f(j)` applies the pair tests.
-template <class F>
+template <int kLanes, class F>
 __device__ __forceinline__ void for_each_listed(const StepConsts& c, const AdjTape& t, int i, int q, double xi,
                                                 double yi, double zi, F&& f) {
   const uint32_t cnt = t.nbr_count[i];
@@ -195,13 +201,17 @@ __device__ __forceinline__ void for_each_listed(const StepConsts& c, const AdjTa
 }
 
 // Sum over the kLanes lanes of a particle (all lanes receive the total).
+template <int kLanes>
 __device__ __forceinline__ double lane_sum(double v) {
 #pragma unroll
   for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-__global__ void __launch_bounds__(kThreads) k_adj_force(StepConsts c, AdjTape t, AdjWork w) {
+// 128 registers (four blocks per SM) spill nothing and beat the 146 that the
+// compiler would take: 66 -> 64 us; 102 of them spill (101 us).
+template <int kLanes>
+__global__ void __launch_bounds__(kThreads, 4) k_adj_force(StepConsts c, AdjTape t, AdjWork w) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = g / kLanes, q = g % kLanes;
   const bool live = i < c.n;  // whole particles per warp: kLanes divides 32
@@ -215,7 +225,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_force(StepConsts c, AdjTape t,
   const double sig_i = qo.w;
   double gx[3] = {0.0, 0.0, 0.0}, gv[3] = {0.0, 0.0, 0.0};
   double pibar = 0.0, rsum = 0.0;
-  if (live) for_each_listed(c, t, i, q, xi, yi, zi, [&](int j) {
+  if (live) for_each_listed<kLanes>(c, t, i, q, xi, yi, zi, [&](int j) {
     // The forward's neighbour test (d = p_j - p_i, world.rs:295-299).
     const d4 xj = load_part(w, 0, n, j), vj = load_part(w, 1, n, j), pj = load_part(w, 2, n, j),
              qj = load_part(w, 3, n, j), yj = load_part(w, 4, n, j);
@@ -272,11 +282,11 @@ __global__ void __launch_bounds__(kThreads) k_adj_force(StepConsts c, AdjTape t,
   });
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    gx[a] = lane_sum(gx[a]);
-    gv[a] = lane_sum(gv[a]);
+    gx[a] = lane_sum<kLanes>(gx[a]);
+    gv[a] = lane_sum<kLanes>(gv[a]);
   }
-  pibar = lane_sum(pibar);
-  rsum = lane_sum(rsum);
+  pibar = lane_sum<kLanes>(pibar);
+  rsum = lane_sum<kLanes>(rsum);
   if (!live || q != 0) return;
   // pi_i = p_i / rho_i^2, p_i = k max(0, rho_i - rho0).
   const double rho_i = t.rho[i], p_i = t.p[i];
@@ -298,6 +308,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_force(StepConsts c, AdjTape t,
   w.kk[i] = kk;
 }
 
+template <int kLanes>
 __global__ void __launch_bounds__(kThreads) k_adj_density(StepConsts c, AdjTape t, AdjWork w) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = g / kLanes, q = g % kLanes;
@@ -308,7 +319,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_density(StepConsts c, AdjTape 
   const double xi = xo.x, yi = xo.y, zi = xo.z;
   const double m_i = xo.w, rb_i = w.rbar_tot[ii];
   double gd[3] = {0.0, 0.0, 0.0};
-  if (live) for_each_listed(c, t, i, q, xi, yi, zi, [&](int j) {
+  if (live) for_each_listed<kLanes>(c, t, i, q, xi, yi, zi, [&](int j) {
     // The forward's density test (p_i - p_j, world.rs:226-229); r = 0 pairs
     // (self, coincident particles) have W'(0) = 0.
     const d4 xj = load_part(w, 0, n, j);
@@ -325,7 +336,7 @@ __global__ void __launch_bounds__(kThreads) k_adj_density(StepConsts c, AdjTape 
     for (int a = 0; a < 3; ++a) gd[a] += f * d[a];
   });
 #pragma unroll
-  for (int a = 0; a < 3; ++a) gd[a] = lane_sum(gd[a]);
+  for (int a = 0; a < 3; ++a) gd[a] = lane_sum<kLanes>(gd[a]);
   if (!live || q != 0) return;
   const uint32_t ins = t.id[i];
 #pragma unroll
@@ -391,12 +402,12 @@ __global__ void __launch_bounds__(kSumThreads) k_adj_sum2(int n, const double* _
 
 void launch_adjoint_step(const StepConsts& c, const AdjTape& t, const AdjWork& w, cudaStream_t s) {
   if (c.n == 0) return;
-  static_assert(32 % kLanes == 0, "a particle's lanes share a warp");
   const int grid = (c.n + kThreads - 1) / kThreads;
-  const int pair_grid = (int)(((long long)c.n * kLanes + kThreads - 1) / kThreads);
+  const int lanes = c.n < kLanesBelow ? 4 : 2;  // they share a warp
+  const int pair_grid = (int)(((long long)c.n * lanes + kThreads - 1) / kThreads);
   k_adj_integrate<<<grid, kThreads, 0, s>>>(c, t, w);
-  k_adj_force<<<pair_grid, kThreads, 0, s>>>(c, t, w);
-  k_adj_density<<<pair_grid, kThreads, 0, s>>>(c, t, w);
+  (lanes == 4 ? k_adj_force<4> : k_adj_force<2>)<<<pair_grid, kThreads, 0, s>>>(c, t, w);
+  (lanes == 4 ? k_adj_density<4> : k_adj_density<2>)<<<pair_grid, kThreads, 0, s>>>(c, t, w);
   // param_acc = {d/d stiffness, d/d visc_k[0]}
   static_assert(kAdjSumBlocks <= kSumThreads, "one partial per thread");
   k_adj_sum2<<<kAdjSumBlocks, kSumThreads, 0, s>>>(c.n, w.kk, w.cc, w.param_acc, w.sum_part, w.sum_arrived);
