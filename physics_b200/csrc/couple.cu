@@ -90,8 +90,8 @@ __device__ __forceinline__ void point_force(const StepConsts& c, const CoupleArg
 // theirs.  The walk takes the points in order, one warp each over the whole
 // GPU, and a warp waits for the earlier points that overlap its own
 // (k_couple_points_flow): the time is that of the longest chain of overlaps
-// instead of the number of points (400 points in 32,805 particles: 622 us while
-// one CTA took runs of up to 16 disjoint neighbours).  A warp stages its
+// instead of the number of points (400 points in 32,805 particles: 110 us; 622
+// while one CTA took runs of up to 16 disjoint neighbours).  A warp stages its
 // candidates' products v_j m_j in its shared buffer (the same f64 products),
 // lane 0 adds them in visit order (the reference's sequential sums), and the
 // lanes apply the reaction to the candidates they hold (v_j + share, with the
@@ -116,7 +116,7 @@ __device__ __forceinline__ bool point_in(const StepConsts& c, const double* q) {
 // One warp per point w of the batch: in-bounds flag, candidate count and
 // cell ranges, and key[w]: the centre cell in box coordinates (clamped far
 // outside the box, where a false overlap only costs a wait) and the in-bounds
-// flag.  Also clears the walk's done flags and ticket.
+// flag.  Also clears the walk's ticket, error and done words.
 __device__ __forceinline__ int box_coord(long long k, long long b0) {
   const long long d = k - b0, far = 1ll << 28;
   return (int)(d < -far ? -far : d > far ? far : d);
@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a
     totals[w] = in && total <= (uint32_t)kPB ? total : 0u;
     key[w] = make_int4(box_coord(kx, c.bx0), box_coord(ky, c.by0), box_coord(kz, c.bz0), in ? 1 : 0);
     done[kFlowHead + w] = 0u;
-    if (w < kFlowHead) done[w] = 0u;
+    if (w == 0)
+      for (int h = 0; h < kFlowHead; ++h) done[h] = 0u;
   }
 }
 

@@ -6,8 +6,16 @@
 // is also compiled with -fmad=false), division and square root are the
 // IEEE-exact double operations, and each particle's neighbour reduction runs
 // sequentially in the reference's visit order (27 cells, di outer / dk inner,
-// ascending insertion index within a cell).  One thread owns one particle, so
-// the result does not depend on scheduling and repeats bit-exactly.
+// ascending insertion index within a cell).  One thread forms each sum, in
+// that order, so the result does not depend on scheduling and repeats
+// bit-exactly.
+//
+// Three passes: the search finds each particle's likely neighbours on f32
+// coordinates (segment_filter.cuh; nothing in range is lost), the density
+// pass tests and sums them in f64 and writes the neighbour lists, and the
+// force pass walks the lists.  At 1,024,000 particles they take 113, 171 and
+// 305 us; a density pass that tested every candidate in f64 took 479, and the
+// force pass on one array per operand 317.
 //
 // Two exact shortcuts are used:
 //   * a candidate whose squared distance exceeds `r2_guard` (the first double

@@ -29,3 +29,22 @@ def test_heat_sources_at_the_edges_of_the_sort_blocks(gpu, oracle_mod, n):
         assert_bits_equal(got, want, "sources")
         assert_bits_equal(w.body_acc, ow.get(O.F_BODY_ACC), "body accelerations")
         src = got
+
+
+def test_one_point_in_memory_that_held_other_data(gpu, oracle_mod):
+    """The words of couple_points' walk in a buffer that is not zero when it is allocated."""
+    import torch
+    O = oracle_mod
+    for _ in range(4):
+        dirty = [torch.full((1 << k,), -1, dtype=torch.int32, device="cuda") for k in range(7, 23)]
+        torch.cuda.synchronize()
+        del dirty
+        torch.cuda.empty_cache()
+        p = ref_test_params(gravity=(0.0, -9.81, 0.0))
+        w, ow = gpu.FluidWorld(p), O.OracleWorld(p)
+        for f in (w, ow):
+            f.fill_box((-0.5,) * 3, (0.5,) * 3, 0.1, 0.05)
+            f.step(0.0025, 2)
+        args = (np.zeros((1, 3)), np.zeros((1, 3)), np.array([0.02]), 0.0025, 1.0, 1000.0)
+        assert_bits_equal(w.couple_points(*args), ow.couple_points(*args), "forces")
+        assert_bits_equal(w.vel, ow.get(O.F_VEL), "velocities")

@@ -119,3 +119,21 @@ def test_quotients_by_reciprocal(gpu, oracle_mod):
     pos = np.concatenate([centre, centre + d])
     mass = 2.0 ** rng.uniform(-20.0, 20.0, n)
     _check(gpu, oracle_mod, _params(gpu, 6.0), pos, rng.normal(0.0, 0.2, (n, 3)), mass, steps=1)
+
+
+@pytest.mark.parametrize("n", [257, 20000, 90000])
+def test_graph_chunks_change_no_bit(gpu, n):
+    """Steps replayed as CUDA graphs: overlapped launches and the one-launch sort (and, past their
+    sizes, the separate kernels) captured."""
+    rng = np.random.default_rng(n)
+    edge = (n / 1000.0) ** (1.0 / 3.0) + 0.05
+    pos, vel = _random(rng, n, (edge, edge, edge))
+    outs = []
+    for chunk in (0, 3):
+        w = gpu.FluidWorld(_params(gpu, 2.0 * edge))
+        w.add_particles(pos, np.full(n, 1.0), vel=vel)
+        w.set_tuning(graph_chunk=chunk)
+        w.step(0.0025, 8)
+        outs.append((w.pos, w.vel, w.acc))
+    for a, b, name in zip(*outs, ("pos", "vel", "acc")):
+        assert_bits_equal(b, a, name)
