@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, C
       if (lane == 0) atomicOr(L.flow + 1, 1u);
       return;
     }
+    __syncwarp();  // what a lane's acquire makes visible, every lane reads
     if (held)
       walk_held(c, a, (int)k, h, reinterpret_cast<double*>(pw), s_r[warp]);
     else
