@@ -364,7 +364,9 @@ int32_t phy_fluid_autotune_horizon(PhyWorldHandle *w, uint32_t sub, double dt, u
  * the compensated state, so the sweep is the exact adjoint of the step map at
  * the states the compensated forward visited.  The world is left in its
  * recorded end state and the tape is kept for further sweeps until
- * phy_fluid_tape_clear or the next phy_fluid_tape_begin.  The reference has
+ * phy_fluid_tape_clear or the next phy_fluid_tape_begin.  Particles added
+ * after phy_fluid_tape_begin are stepped, but the tape's checkpoints lack
+ * them: phy_fluid_step_backward then fails.  The reference has
  * no adjoint; these calls replace nothing in phy_ffi.h. */
 int32_t phy_fluid_tape_begin(PhyWorldHandle *w, uint32_t sub, uint32_t checkpoint_every);
 int32_t phy_fluid_tape_clear(PhyWorldHandle *w, uint32_t sub);

@@ -1336,11 +1336,13 @@ StepConsts FluidWorld::step_impl(double dt) {
     if (std::memcmp(&now, &tape_.params, sizeof(now)) != 0)
       throw std::invalid_argument("step: parameters changed while the adjoint tape is recording");
     if (b_.has_ba) throw std::invalid_argument("step: body accelerations are not recorded by the adjoint tape");
-    if (!tape_.dts.empty() && tape_.dts.size() % (size_t)tape_.every == 0) save_checkpoint();
+    // (Particles added since tape_begin: its buffers hold fewer, and
+    // step_backward refuses the tape.)
+    if (n_ == tape_.n && !tape_.dts.empty() && tape_.dts.size() % (size_t)tape_.every == 0) save_checkpoint();
     tape_.dts.push_back(dt);
   }
   StepConsts c = prepare_step(dt);
-  const bool direct = tape_.on && !recomputing_ && direct_slot(c);
+  const bool direct = tape_.on && !recomputing_ && n_ == tape_.n && direct_slot(c);
   if (direct) set_tape_outputs(true);
   PassEvents pe;
   cudaEvent_t* ev = nullptr;
@@ -2051,6 +2053,7 @@ void FluidWorld::tape_free() {
   tape_.on = false;
   tape_.n = 0;
   dfree(adj_work_);
+  adj_work_n_ = 0;
   dfree(comp_rec_);
   comp_rec_cap_ = 0;
   for (auto& p : adj_slot_f_) dfree(p);
@@ -2133,7 +2136,10 @@ void FluidWorld::ensure_slot(const StepConsts& c, int si) {
 }
 
 void FluidWorld::ensure_adj_work() {
-  if (!adj_work_) dalloc(adj_work_, kAdjWorkArrays * n_ + 2 + 2 * kAdjSumBlocks + 1);
+  if (adj_work_n_ >= n_) return;
+  adj_work_n_ = 0;
+  dalloc(adj_work_, kAdjWorkArrays * n_ + 2 + 2 * kAdjSumBlocks + 1);
+  adj_work_n_ = n_;
 }
 
 // The force pass's viscous and shear sums, kept for the reverse step, in the
@@ -2214,6 +2220,8 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
   const int T = (int)tape_.dts.size();
   if (!tape_.on) throw std::invalid_argument("step_backward: no adjoint tape (call tape_begin before stepping)");
   if (n == 0) return;
+  if (T > 0 && n != tape_.n)
+    throw std::invalid_argument("step_backward: particles were added while the tape was recording");
   cudaStream_t s = stream_;
   // Work arrays: the packed operands (kAdjRec), gx_ins, gv_ins, gx, gv (3
   // each), rbar, rbar_tot, cc, kk, the tape's fv and shear outputs (4): arrays

@@ -114,7 +114,9 @@ class FluidWorld {
   // (direct_slot; the same bits): given dL/dx_T and dL/dv_T (insertion order,
   // xyz interleaved; null = zero) it returns dL/dx_0, dL/dv_0 and
   // {dL/d stiffness, dL/d visc_k[0]} (outputs may be null) and leaves the
-  // world in its state x_T, v_T.  The tape is kept for further sweeps.
+  // world in its state x_T, v_T.  The tape is kept for further sweeps.  A
+  // world that took particles after tape_begin steps on, but its tape is not
+  // swept any more (step_backward throws).
   void tape_begin(int every);
   void tape_clear();
   int tape_steps() const { return (int)tape_.dts.size(); }
@@ -312,6 +314,7 @@ class FluidWorld {
   AdjTape record_step(const StepConsts& c, int si, uint32_t* slot_of);
   // Reverse-sweep buffers kept between sweeps and tapes (tape_clear).
   double* adj_work_ = nullptr;
+  size_t adj_work_n_ = 0;  // particles it is sized for
   uint32_t* comp_rec_ = nullptr;  // compensated adjoint: insertion index -> recorded slot
   size_t comp_rec_cap_ = 0;
   std::vector<double*> adj_slot_f_;

@@ -1,0 +1,96 @@
+"""The library's host side on a CUDA runtime without a GPU (fake_cudart.cpp): what it
+allocates, copies, refuses and reports.  Kernels do nothing there, so no values are compared."""
+import ctypes as C
+import gc
+import importlib.util
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+import physics_b200 as pb
+from physics_b200 import _lib as L
+
+ROOT = Path(__file__).resolve().parent.parent
+DT = 0.0025
+
+
+@pytest.fixture(scope="session")
+def fake_library(tmp_path_factory):
+    spec = importlib.util.spec_from_file_location("phy_build", ROOT / "physics_b200" / "csrc" / "build.py")
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    try:
+        cuda = Path(build._nvcc()).parents[1] / "include"
+    except RuntimeError as e:
+        pytest.skip(str(e))
+    build.build_product()
+    out = tmp_path_factory.mktemp("fake") / "libphysph_fake.so"
+    objs = [build.OBJDIR / (s + ".o") for s in build.SOURCES]
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", cuda, "-Wl,-Bsymbolic",
+                    ROOT / "tests" / "fake_cudart.cpp", *objs, "-o", out, "-lpthread", "-ldl"], check=True)
+    lib = C.CDLL(str(out))
+    for name, (res, args) in L.SIGNATURES.items():
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = res, args
+    lib.fake_live.restype = C.c_ulonglong
+    lib.fake_set_budget.argtypes = [C.c_ulonglong]
+    lib.fake_poke_pinned.argtypes = [C.c_ulonglong, C.c_uint32]
+    lib.fake_launches.argtypes = [C.c_char_p]
+    return lib
+
+
+@pytest.fixture
+def fake(fake_library, monkeypatch):
+    monkeypatch.setattr(L, "_lib", fake_library)
+    fake_library.fake_reset()
+    yield fake_library
+    for o in gc.get_objects():  # worlds go before the library is switched back
+        if isinstance(o, pb.World):
+            o.close()
+
+
+def _world(form="f64", n=64, **kw):
+    p = pb.SphParams.defaults()
+    p.bounds_min, p.bounds_max = (0.0,) * 3, (2.0,) * 3
+    w = pb.FluidWorld(p, form)
+    w.add_particles(np.random.default_rng(n).uniform(0.1, 1.9, (n, 3)), 0.02, **kw)
+    return w
+
+
+@pytest.mark.parametrize("form", ["f64", "comp"])
+@pytest.mark.parametrize("swept", [False, True])
+def test_particles_added_while_a_tape_records(fake, form, swept):
+    """The world takes them and steps on; the tape, whose checkpoints hold the old ones, is not
+    swept any more, and no buffer sized for them is written past its end."""
+    w = _world(form)
+    w.tape_begin(2)
+    w.step(DT, 3)
+    g = np.ones((64, 3))
+    if swept:
+        w.step_backward(g, g)
+    w.add_particles(np.full((200, 3), 0.5), 0.02)
+    w.step(DT, 6)
+    assert len(w) == 264 and w.tape_steps == 9
+    g = np.ones((264, 3))
+    with pytest.raises(L.PhyError, match="particles were added"):
+        w.step_backward(g, g)
+    assert fake.fake_violations() == 0
+    w.tape_clear()
+    w.tape_begin(2)
+    w.step(DT, 3)
+    w.step_backward(g, g)
+    assert fake.fake_violations() == 0
+
+
+def test_particles_added_to_a_tape_without_steps(fake):
+    """Nothing to sweep: the seeds are the gradients, as for any such tape."""
+    w = _world()
+    w.tape_begin(2)
+    w.step(DT, 2)
+    w.step_backward(np.ones((64, 3)), None)
+    w.tape_begin(2)
+    w.add_particles(np.full((200, 3), 0.5), 0.02)
+    w.step_backward(np.ones((264, 3)), None)
+    assert fake.fake_violations() == 0
