@@ -367,6 +367,16 @@ void dalloc(T*& p, size_t count) {
   cuda_check(cudaMalloc((void**)&p, count * sizeof(T)), "cudaMalloc");
 }
 
+// Makes a device array of at least `need` elements out of one of `cap`; after a
+// failure it has none.
+template <class T, class C>
+void dreserve(T*& p, C& cap, size_t need) {
+  if (p && (size_t)cap >= need) return;
+  cap = 0;
+  dalloc(p, need);
+  cap = (C)need;
+}
+
 // Grows a device array to `cap` elements, keeping the first `keep`.
 template <class T>
 void dgrow(T*& p, size_t keep, size_t cap, cudaStream_t s) {
@@ -562,6 +572,7 @@ void FluidWorld::ensure_capacity(size_t n) {
   if (n >= (1ull << (32 - kCodeBits)))
     throw std::invalid_argument("FluidWorld: more than 2^27 particles in one subsystem");
   if ((int)n <= b_.capacity) return;
+  ++alloc_gen_;  // also where a later allocation fails
   if (!tape_.on && tape_.n) tape_free();
   for (auto& p : scene_keep_) dfree(p);
   size_t cap = std::max<size_t>(n, (size_t)b_.capacity + b_.capacity / 2);
@@ -596,6 +607,7 @@ void FluidWorld::ensure_capacity(size_t n) {
     dgrow(b_.cmr, 0, cap, s);
   }
   dgrow(b_.nbr_count, 0, cap, s);
+  mode_ready_ = false;
   dfree(b_.nbr);
   dfree(b_.rec);
   dfree(b_.nbr16);
@@ -652,6 +664,7 @@ void FluidWorld::ensure_mode_buffers() {
     }
     if (!b_.okey) dalloc(b_.okey, cap);
   }
+  mode_ready_ = true;
   ++alloc_gen_;
 }
 
@@ -718,7 +731,7 @@ void FluidWorld::grow_box_with_device_positions(size_t n, const double* d_pos3) 
 
 void FluidWorld::ensure_box_scratch() {
   if (d_bbox_) return;
-  cuda_check(cudaMallocHost((void**)&h_bbox_, 7 * sizeof(long long)), "cudaMallocHost");
+  if (!h_bbox_) cuda_check(cudaMallocHost((void**)&h_bbox_, 7 * sizeof(long long)), "cudaMallocHost");
   cuda_check(cudaMalloc(&d_bbox_, sizeof(BoxScratch)), "cudaMalloc");
   cuda_check(cudaMemsetAsync(&static_cast<BoxScratch*>(d_bbox_)->arrived, 0, sizeof(unsigned), stream_), "memset");
 }
@@ -827,8 +840,8 @@ void FluidWorld::ensure_cells() {
        std::memcmp(boxes.data(), host_boxes_.data(), boxes.size() * sizeof(SceneBox)) != 0)) {
     if ((int)boxes.size() > boxes_capacity_) {
       cuda_check(cudaStreamSynchronize(stream_), "boxes sync");
-      dalloc(b_.boxes, boxes.size());
-      boxes_capacity_ = (int)boxes.size();
+      host_boxes_.clear();
+      dreserve(b_.boxes, boxes_capacity_, boxes.size());
       ++alloc_gen_;
     }
     host_boxes_ = boxes;
@@ -841,6 +854,7 @@ void FluidWorld::ensure_cells() {
     int cap = (int)std::min<long long>(kMaxCells, std::max<long long>(ncells_, (long long)b_.cell_capacity * 3 / 2));
     size_t scan_len = scan_block_sums_needed(cap) * 4096;
     cuda_check(cudaStreamSynchronize(stream_), "cells sync");
+    b_.cell_capacity = 0;
     dalloc(b_.cell_start, scan_len);
     b_.cell_capacity = cap;
     ++alloc_gen_;
@@ -849,8 +863,7 @@ void FluidWorld::ensure_cells() {
   if (tile_ && tile_scan_length(b_.cell_capacity) > b_.tile_scan_entries) {
     const size_t len = tile_scan_length(b_.cell_capacity);
     cuda_check(cudaStreamSynchronize(stream_), "tile scan sync");
-    dalloc(b_.tile_head, len);
-    b_.tile_scan_entries = len;
+    dreserve(b_.tile_head, b_.tile_scan_entries, len);
     ++alloc_gen_;
   }
   // The scan's tile sums serve the cell scan and the tile scan alike.
@@ -858,8 +871,7 @@ void FluidWorld::ensure_cells() {
       (int)std::max(2 * scan_block_sums_needed(b_.cell_capacity), tile_scan_sums_needed(b_.cell_capacity));
   if (sums > b_.block_sums_capacity) {
     cuda_check(cudaStreamSynchronize(stream_), "sums sync");
-    dalloc(b_.block_sums, (size_t)sums);
-    b_.block_sums_capacity = sums;
+    dreserve(b_.block_sums, b_.block_sums_capacity, (size_t)sums);
     ++alloc_gen_;
   }
 }
@@ -1260,6 +1272,7 @@ StepConsts FluidWorld::prepare_step(double dt) {
   if (!scenes_.empty() && !(prec_ == Precision::F32Comp && comp_tile_ > 0))
     throw std::invalid_argument("step: batched scenes need the tiled compensated form");
   ensure_cells();
+  if (!mode_ready_) ensure_mode_buffers();  // a growth that failed left some out
   if (prec_ == Precision::F32Comp && comp_tile_ > 0) ensure_masks();
   return make_consts(dt);
 }
@@ -1461,7 +1474,7 @@ void FluidWorld::set_scenes(const std::vector<uint64_t>& counts, const std::vect
   pbase[counts.size()] = (uint32_t)first;
   cuda_check(cudaStreamSynchronize(stream_), "scenes sync");
   if (pbase.size() > pbase_cap_) {
-    dalloc(d_pbase_, pbase.size());
+    dgrow(d_pbase_, 0, pbase.size(), stream_);  // (the old one stays if it fails: scenes_ may be in use)
     pbase_cap_ = pbase.size();
   }
   cuda_check(cudaMemcpy(d_pbase_, pbase.data(), pbase.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
@@ -1496,10 +1509,7 @@ void FluidWorld::grow_scene_boxes(const double* d_pos3) {
   // A few slices per scene keep every SM busy with few scenes.
   const int slices = std::max(1, std::min(32, 1184 / ns));
   const size_t words = 7 * (size_t)ns * slices;
-  if (words > scene_bbox_cap_) {
-    dalloc(d_scene_bbox_, words);
-    scene_bbox_cap_ = words;
-  }
+  dreserve(d_scene_bbox_, scene_bbox_cap_, words);
   k_scene_bbox<<<dim3((unsigned)ns, (unsigned)slices), kThreads, 0, stream_>>>(d_pos3, d_pbase_, 1.0 / h0_,
                                                                                d_scene_bbox_);
   cuda_check(cudaGetLastError(), "scene bbox");
@@ -1812,10 +1822,7 @@ void FluidWorld::couple_points(size_t np, const double* pos, const double* vel, 
   c.tile = 0;  // x-major cells for the index
   c.tile_log2 = 0;
   const size_t need = 10 * np + 1;
-  if (couple_cap_ < need) {
-    dalloc(d_couple_, need);
-    couple_cap_ = need;
-  }
+  dreserve(d_couple_, couple_cap_, need);
   std::vector<double> h(10 * np);
   for (size_t k = 0; k < np; ++k) {
     double* r = h.data() + 10 * k;
@@ -1866,10 +1873,7 @@ void FluidWorld::couple_heat(const uint64_t* dims3, const double* origin3, doubl
   ensure_cells();
   const StepConsts c = make_consts(dt);
   const size_t need = couple_heat_scratch_bytes((int)n_, cells);
-  if (heat_cap_ < need) {
-    dalloc(d_heat_, need);
-    heat_cap_ = need;
-  }
+  dreserve(d_heat_, heat_cap_, need);
   const size_t gbytes = cells * sizeof(double);
   cuda_check(cudaMemcpyAsync(d_heat_, temp, gbytes, cudaMemcpyHostToDevice, stream_), "couple_heat upload");
   if (deposit)
@@ -1938,10 +1942,7 @@ void FluidWorld::couple_bodies(PhyCoupleBody* bodies, uint32_t nb, const double*
   ensure_cells();
   const StepConsts c = make_consts(dt);
   const size_t need = couple_bodies_scratch_bytes((int)n_, (int)nb, n_data, n_faces);
-  if (bodies_cap_ < need) {
-    dalloc(d_bodies_, need);
-    bodies_cap_ = need;
-  }
+  dreserve(d_bodies_, bodies_cap_, need);
   CoupleBodiesLaunch l;
   l.scratch = d_bodies_;
   l.bodies = bodies;
@@ -1999,10 +2000,8 @@ namespace phy {
 
 void FluidWorld::save_checkpoint() {
   const size_t k = tape_.nckpt;
-  if (k >= tape_.ckpt.size()) {
-    tape_.ckpt.push_back(nullptr);
-    dalloc(tape_.ckpt.back(), 6 * n_);
-  }
+  if (k >= tape_.ckpt.size()) tape_.ckpt.push_back(nullptr);
+  if (!tape_.ckpt[k]) dalloc(tape_.ckpt[k], 6 * n_);
   double* ck = tape_.ckpt[k];
   const ParticleConsts& pc = b_.pc[b_.cur];
   k_get_vec_by_id<<<grid_for(n_), kThreads, 0, stream_>>>((int)n_, pc.id, b_.pv1[0], b_.pv1[1], b_.pv1[2], ck);
@@ -2270,10 +2269,7 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
   const bool comp = form == Precision::F32Comp;
   uint32_t* slot_of = nullptr;  // compensated: insertion index -> recorded slot of the step being re-run
   if (comp) {
-    if (comp_rec_cap_ < n) {
-      dalloc(comp_rec_, n);
-      comp_rec_cap_ = n;
-    }
+    dreserve(comp_rec_, comp_rec_cap_, n);
     slot_of = comp_rec_;
   }
   auto cleanup = [&]() {

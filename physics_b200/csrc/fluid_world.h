@@ -210,6 +210,7 @@ class FluidWorld {
  private:
   void ensure_capacity(size_t n);
   void ensure_mode_buffers();
+  bool mode_ready_ = true;  // the buffers of ensure_mode_buffers are those of the capacity
   void ensure_masks();
   void ensure_cells();
   void grow_box_with_bounds();

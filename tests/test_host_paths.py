@@ -94,3 +94,55 @@ def test_particles_added_to_a_tape_without_steps(fake):
     w.add_particles(np.full((200, 3), 0.5), 0.02)
     w.step_backward(np.ones((264, 3)), None)
     assert fake.fake_violations() == 0
+
+
+def test_failed_allocations_leave_no_stale_capacity(fake):
+    """A scene table, a grid or a particle array that could not be had: the call fails, and the
+    next one that fits an earlier capacity allocates instead of using what is gone."""
+    w = _world("comp")
+    w.set_scenes([32, 32], [(0.0,) * 3] * 2, [(2.0,) * 3] * 2)
+    w.step(DT)
+    w.clear_scenes()
+    fake.fake_set_budget(fake.fake_live())
+    counts = [64] + [0] * 3999
+    with pytest.raises(L.PhyError, match="out of memory"):
+        w.set_scenes(counts, [(0.0,) * 3] * 4000, [(0.1,) * 3] * 4000)
+    fake.fake_set_budget(1 << 40)
+    w.set_scenes([32, 32], [(0.0,) * 3] * 2, [(2.0,) * 3] * 2)
+    w.step(DT)
+    fake.fake_set_budget(fake.fake_live() + (1 << 19))  # room for the table of scenes, not for their boxes
+    with pytest.raises(L.PhyError, match="out of memory"):
+        w.set_scenes(counts, [(0.0,) * 3] * 4000, [(0.1,) * 3] * 4000)
+        w.step(DT)
+    fake.fake_set_budget(1 << 40)
+    w.set(pb.FIELD_POS, np.full((64, 3), 0.5))
+    w.clear_scenes()
+    w.set_scenes([32, 32], [(0.0,) * 3] * 2, [(2.0,) * 3] * 2)
+    w.step(DT)
+    assert fake.fake_violations() == 0
+
+
+@pytest.mark.parametrize("form", ["f64", "comp"])
+@pytest.mark.parametrize("room", [0.2, 0.5, 0.8, 0.95])
+def test_a_growth_that_fails_is_made_up_for(fake, form, room):
+    """add_particles fails part way through the growth: the world steps on with what it had,
+    allocating the arrays that the attempt gave up."""
+    sizes = []
+    for n in (64, 64 + 20000):
+        w = _world(form, n=n)
+        w.step(DT)
+        sizes.append(fake.fake_live())
+        w._world.close()
+    w = _world(form)
+    w.step(DT)
+    fake.fake_set_budget(int(fake.fake_live() + room * (sizes[1] - sizes[0])))
+    with pytest.raises(L.PhyError, match="out of memory"):
+        w.add_particles(np.full((20000, 3), 0.5), 0.02)
+    fake.fake_set_budget(1 << 40)
+    calls = fake.fake_device_calls()
+    w.step(DT)
+    # (The first fifth of the memory goes to arrays that keep their old ones until then.)
+    assert len(w) == 64 and (fake.fake_device_calls() > calls) == (room > 0.2)
+    w.add_particles(np.full((20000, 3), 0.5), 0.02)
+    w.step(DT)
+    assert fake.fake_violations() == 0
