@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 
 #include "launch.cuh"
@@ -1059,17 +1060,21 @@ void launch_cell_index(const StepConsts& c, DevBuffers& b, uint32_t* flags, cuda
 }
 
 // Blocks of the fused sort: resident, at most four per SM (the barrier takes
-// 1.3 us with 35 blocks and 1.6 us with 296).
+// 1.3 us with 35 blocks and 1.6 us with 296).  Per device: the shared-memory
+// limit belongs to the device's context, and the grid to its size.
 template <int kCells>
 static int fused_blocks() {
-  static const int blocks = [] {
-    int dev = 0, sms = 1, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_sort_fused<kCells>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LargeStage));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sort_fused<kCells>, kThreads, sizeof(LargeStage));
-    return std::max(sms, 1) * std::min(std::max(per, 1), 4);
-  }();
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < kDevices && known[dev].load()) return known[dev].load();
+  int sms = 1, per = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaFuncSetAttribute(k_sort_fused<kCells>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LargeStage));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sort_fused<kCells>, kThreads, sizeof(LargeStage));
+  const int blocks = std::max(sms, 1) * std::min(std::max(per, 1), 4);
+  if (dev < kDevices) known[dev].store(blocks);
   return blocks;
 }
 

@@ -146,3 +146,14 @@ def test_a_growth_that_fails_is_made_up_for(fake, form, room):
     w.add_particles(np.full((20000, 3), 0.5), 0.02)
     w.step(DT)
     assert fake.fake_violations() == 0
+
+
+def test_worlds_on_a_second_device(fake):
+    """An f64 world on another device of the process after one on the first: the one-launch
+    sort's shared-memory limit is set on each."""
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        w = _world()
+        w.step(DT, 2)
+        w.synchronize()
+    assert fake.fake_launches(b"k_sort_fused") == 4
