@@ -470,19 +470,23 @@ SphParams SphParams::from_c(const PhySphParams& c) {
 FluidWorld::FluidWorld(const SphParams& p, Precision prec) : params(p), prec_(prec), h0_(p.h) {
   cuda_check(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
   stream_ = own_stream_;
-  dalloc(b_.flags, kStepWords);
+  // The step's words, the counters and the box scratch, which all start at zero.
+  static_assert(kStepWords * sizeof(uint32_t) <= 256, "counters follow the words");
+  dalloc(d_words_, 512 + sizeof(BoxScratch));
+  cuda_check(cudaMemsetAsync(d_words_, 0, 512 + sizeof(BoxScratch), stream_), "memset");
+  b_.flags = reinterpret_cast<uint32_t*>(d_words_);
   b_.order_count = b_.flags + 2;
-  dalloc(b_.counters, 2);
-  cuda_check(cudaMemsetAsync(b_.flags, 0, kStepWords * sizeof(uint32_t), stream_), "memset");
-  cuda_check(cudaMemsetAsync(b_.counters, 0, 2 * sizeof(unsigned long long), stream_), "memset");
+  b_.counters = reinterpret_cast<unsigned long long*>(d_words_ + 256);
+  cuda_check(cudaMallocHost((void**)&host_, sizeof(HostWords)), "cudaMallocHost");
+  std::memset(host_, 0, sizeof(HostWords));
 }
 
 FluidWorld::~FluidWorld() {
   if (stream_) cudaStreamSynchronize(stream_);
   drop_graphs();
   free_all();
-  if (d_bbox_) cudaFree(d_bbox_);
-  if (h_bbox_) cudaFreeHost(h_bbox_);
+  dfree(d_words_);
+  if (host_) cudaFreeHost(host_);
   dfree(d_couple_);
   couple_scratch_.release();
   dfree(d_heat_);
@@ -519,44 +523,21 @@ void FluidWorld::free_all() {
   }
   dfree(b_.mu);
   dfree(b_.cpos);
-  dfree(b_.rec);
   dfree(b_.cvel);
   dfree(b_.cmr);
-  dfree(b_.nbr);
+  dfree(b_.nbr);  // and rec
   dfree(b_.nbr_count);
   dfree(b_.nbr16);
-  dfree(b_.sorted_cell);
   dfree(b_.tile_head);
-  b_.tile_scan_entries = 0;
-  dfree(b_.tile_of);
-  dfree(b_.large_cells);
-  dfree(b_.tile_slot);
-  dfree(b_.num_tiles);
   dfree(b_.boxes);
-  dfree(b_.queue);
-  dfree(b_.tile_crowd);
-  dfree(b_.dense_q0);
-  dfree(b_.task_done);
-  dfree(b_.task_mbase);
-  dfree(b_.task_mcount);
+  dfree(tile_words_);
   dfree(b_.mask_hdr);
   dfree(b_.mask_bits);
-  b_.mask_ctl = nullptr;
-  b_.mask_cap = 0;
-  mask_tried_ = 0;
-  if (b_.mask_demand) cudaFreeHost(b_.mask_demand);
-  b_.mask_demand = nullptr;
   dfree(b_.okey);
-  dfree(b_.cell_of);
-  dfree(b_.rank);
-  dfree(b_.tmp);
-  dfree(b_.perm);
+  dfree(sort_words_);
   dfree(b_.cell_start);
   dfree(b_.block_sums);
   dfree(b_.stage);
-  dfree(b_.flags);
-  dfree(b_.counters);
-  b_.order_count = nullptr;
 }
 
 void FluidWorld::set_stream(cudaStream_t s) {
@@ -609,22 +590,17 @@ void FluidWorld::ensure_capacity(size_t n) {
   dgrow(b_.nbr_count, 0, cap, s);
   mode_ready_ = false;
   dfree(b_.nbr);
-  dfree(b_.rec);
+  b_.rec = nullptr;
   dfree(b_.nbr16);
-  dfree(b_.sorted_cell);
-  dfree(b_.tile_of);
-  dfree(b_.large_cells);
-  dfree(b_.tile_slot);
-  dfree(b_.tile_crowd);
-  dfree(b_.dense_q0);
-  dfree(b_.task_done);
-  dfree(b_.task_mbase);
-  dfree(b_.task_mcount);
+  dfree(tile_words_);
   dfree(b_.okey);
-  dgrow(b_.cell_of, 0, cap, s);
-  dgrow(b_.rank, 0, cap, s);
-  dgrow(b_.tmp, 0, cap, s);
-  dgrow(b_.perm, 0, cap, s);
+  const size_t stride = (cap + 63) / 64 * 64;
+  dgrow(sort_words_, 0, 5 * stride, s);
+  b_.cell_of = sort_words_;
+  b_.rank = sort_words_ + stride;
+  b_.tmp = sort_words_ + 2 * stride;
+  b_.perm = sort_words_ + 3 * stride;
+  b_.sorted_cell = sort_words_ + 4 * stride;
   dgrow(b_.stage, 0, 8 * ((cap + 31) / 32 * 32), s);
   b_.capacity = (int)cap;
   ++alloc_gen_;
@@ -637,31 +613,49 @@ void FluidWorld::ensure_mode_buffers() {
   const size_t cap = (size_t)b_.capacity;
   if (cap == 0) return;
   const bool tiled = prec_ == Precision::F32Comp && comp_tile_ > 0;
-  if (!tiled && !b_.nbr) dalloc(b_.nbr, (size_t)kMaxNeighbors * cap);
-  if (prec_ == Precision::F64Plain) {
-    if (!b_.rec) dalloc(b_.rec, plain_doubles(cap));
-    if (!b_.sorted_cell) dalloc(b_.sorted_cell, cap);
+  const bool f64 = prec_ == Precision::F64Plain;
+  // One allocation for what comes and goes together: mapping a block of memory
+  // takes ~0.3 ms whatever its size, most of a small world's creation.
+  if (f64 && !b_.rec) dfree(b_.nbr);
+  if (!tiled && !b_.nbr) {
+    const size_t lists = ((size_t)kMaxNeighbors * cap + 63) / 64 * 64;
+    dalloc(b_.nbr, lists + (f64 ? 2 * plain_doubles(cap) : 0));
+    b_.rec = f64 ? reinterpret_cast<double*>(b_.nbr + lists) : nullptr;
   }
   if (tiled) {
     if (!b_.nbr16) dalloc(b_.nbr16, (size_t)kMaxNeighbors * cap);
-    if (!b_.sorted_cell) dalloc(b_.sorted_cell, cap);
-    if (!b_.tile_of) dalloc(b_.tile_of, cap + 1);
-    if (!b_.large_cells) dalloc(b_.large_cells, cap / 16 + 64);  // cells of more than 16 particles
-    if (!b_.tile_slot) dalloc(b_.tile_slot, cap + 1);
-    if (!b_.tile_crowd) dalloc(b_.tile_crowd, cap + 1);
-    if (!b_.num_tiles) dalloc(b_.num_tiles, 1);
-    if (!b_.queue) dalloc(b_.queue, 5);
-    // Dense-cell tasks: at most one per 32 particles plus one per occupied cell.
-    if (!b_.dense_q0) dalloc(b_.dense_q0, cap + cap / 32 + 64);
-    // (two halves per task)
-    if (!b_.task_done) dalloc(b_.task_done, 2 * (cap + cap / 32 + 64));
-    if (!b_.task_mbase) dalloc(b_.task_mbase, 2 * (cap + cap / 32 + 64));
-    if (!b_.task_mcount) dalloc(b_.task_mcount, 2 * (cap + cap / 32 + 64));
-    b_.mask_ctl = reinterpret_cast<unsigned long long*>(b_.flags + 6);
-    if (!b_.mask_demand) {
-      cuda_check(cudaMallocHost((void**)&b_.mask_demand, sizeof(unsigned long long)), "cudaMallocHost");
-      *b_.mask_demand = 0;
+    if (!tile_words_) {
+      // Dense-cell tasks: at most one per 32 particles plus one per occupied
+      // cell, two halves each.
+      const size_t tasks = cap + cap / 32 + 64;
+      uint32_t* at = nullptr;
+      size_t words = 0;
+      auto carve = [&](uint32_t*& p, size_t count) {
+        p = at ? at + words : nullptr;
+        words += (count + 63) / 64 * 64;
+      };
+      uint32_t* crowd = nullptr;
+      auto all = [&]() {
+        words = 0;
+        carve(b_.num_tiles, 1);
+        carve(b_.queue, 5);
+        carve(b_.tile_of, cap + 1);
+        carve(b_.tile_slot, cap + 1);
+        carve(b_.large_cells, cap / 16 + 64);  // cells of more than 16 particles
+        carve(crowd, cap / 4 + 1);
+        carve(b_.dense_q0, tasks);
+        carve(b_.task_done, 2 * tasks);
+        carve(b_.task_mbase, 2 * tasks);
+        carve(b_.task_mcount, 2 * tasks);
+      };
+      all();
+      dalloc(tile_words_, words);
+      at = tile_words_;
+      all();
+      b_.tile_crowd = reinterpret_cast<uint8_t*>(crowd);
     }
+    b_.mask_ctl = reinterpret_cast<unsigned long long*>(b_.flags + 6);
+    b_.mask_demand = &host_->mask_demand;
     if (!b_.okey) dalloc(b_.okey, cap);
   }
   mode_ready_ = true;
@@ -721,19 +715,11 @@ void FluidWorld::grow_box_with_positions(size_t n, const double* pos3) {
 // (interleaved xyz), through a reduction kernel and one small readback.
 void FluidWorld::grow_box_with_device_positions(size_t n, const double* d_pos3) {
   if (n == 0) return;
-  ensure_box_scratch();
-  k_key_bbox<<<box_blocks(n), kThreads, 0, stream_>>>((int)n, d_pos3, 1.0 / h0_, static_cast<BoxScratch*>(d_bbox_),
-                                                      h_bbox_);
+  k_key_bbox<<<box_blocks(n), kThreads, 0, stream_>>>((int)n, d_pos3, 1.0 / h0_,
+                                                      reinterpret_cast<BoxScratch*>(d_words_ + 512), host_->box);
   cuda_check(cudaGetLastError(), "bbox kernel");
   cuda_check(cudaStreamSynchronize(stream_), "bbox sync");
-  merge_box(h_bbox_, h_bbox_ + 3, h_bbox_[6] != 0);
-}
-
-void FluidWorld::ensure_box_scratch() {
-  if (d_bbox_) return;
-  if (!h_bbox_) cuda_check(cudaMallocHost((void**)&h_bbox_, 7 * sizeof(long long)), "cudaMallocHost");
-  cuda_check(cudaMalloc(&d_bbox_, sizeof(BoxScratch)), "cudaMalloc");
-  cuda_check(cudaMemsetAsync(&static_cast<BoxScratch*>(d_bbox_)->arrived, 0, sizeof(unsigned), stream_), "memset");
+  merge_box(host_->box, host_->box + 3, host_->box[6] != 0);
 }
 
 // Merges a key range into the box (throws, leaving the box unchanged, when
@@ -1065,7 +1051,6 @@ void FluidWorld::set_particles_device(size_t m, const double* pos, const double*
   if (tape_.n && tape_.n != m) tape_free();
   if (m == 0) return;
   ensure_capacity(m);
-  ensure_box_scratch();
   ParticleConsts& pc = b_.pc[b_.cur];
   LoadArgs l{};
   l.pos = pos;
@@ -1080,11 +1065,12 @@ void FluidWorld::set_particles_device(size_t m, const double* pos, const double*
     l.zero[l.n_zero++] = z;
   if (b_.has_ba)
     for (int k = 0; k < 3; ++k) l.zero[l.n_zero++] = pc.ba[k];
-  k_load_dev<<<box_blocks(m), kThreads, 0, stream_>>>((int)m, l, 1.0 / h0_, static_cast<BoxScratch*>(d_bbox_), h_bbox_);
+  k_load_dev<<<box_blocks(m), kThreads, 0, stream_>>>((int)m, l, 1.0 / h0_,
+                                                      reinterpret_cast<BoxScratch*>(d_words_ + 512), host_->box);
   cuda_check(cudaGetLastError(), "set_particles_device kernel");
   cuda_check(cudaStreamSynchronize(stream_), "set_particles_device sync");
   // The positions may widen the grid box (a failure leaves the world empty).
-  merge_box(h_bbox_, h_bbox_ + 3, h_bbox_[6] != 0);
+  merge_box(host_->box, host_->box + 3, host_->box[6] != 0);
   n_ = m;
 }
 

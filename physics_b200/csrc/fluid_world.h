@@ -259,9 +259,17 @@ class FluidWorld {
   void collect_phase_times();
   double phase_ms_[4] = {0, 0, 0, 0};
   double timed_steps_ = 0;
-  void* d_bbox_ = nullptr;       // partial key boxes (BoxScratch)
-  long long* h_bbox_ = nullptr;  // mapped host memory: min xyz, max xyz, non-finite flag
-  void ensure_box_scratch();
+  // Device words of the world: the step's flags, the counters (byte 256), the
+  // partial key boxes (byte 512).
+  unsigned char* d_words_ = nullptr;
+  // Mapped host memory that kernels write.
+  struct HostWords {
+    long long box[7];  // min xyz, max xyz, non-finite flag
+    unsigned long long mask_demand;
+  };
+  HostWords* host_ = nullptr;
+  uint32_t* sort_words_ = nullptr;  // cell_of, rank, tmp, perm, sorted_cell
+  uint32_t* tile_words_ = nullptr;  // the tile list's and dense tasks' arrays
   // Point records of couple_points (10 doubles each) plus one word of flags.
   double* d_couple_ = nullptr;
   CouplePointsScratch couple_scratch_;

@@ -157,3 +157,12 @@ def test_worlds_on_a_second_device(fake):
         w.step(DT, 2)
         w.synchronize()
     assert fake.fake_launches(b"k_sort_fused") == 4
+
+
+@pytest.mark.parametrize("form,most", [("f64", 42), ("comp", 59)])
+def test_a_new_world_maps_few_blocks_of_memory(fake, form, most):
+    """Creating a world, adding its particles and the first step: device allocations (each a
+    block to map) no more than before the forms got further buffers, one page-locked one."""
+    w = _world(form, n=64000)
+    w.step(DT)
+    assert fake.fake_device_calls() <= most and fake.fake_pinned_calls() <= 1
