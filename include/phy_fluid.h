@@ -283,6 +283,11 @@ int32_t phy_fluid_phase_times(PhyWorldHandle *w, uint32_t sub, double *out5, int
  *                         grows with the tasks' demand, within a quarter of
  *                         the free device memory and 16 GiB), 0 = it filters
  *                         the candidates again.
+ *   PHY_TUNE_SORT_POLLS   polls after which a grid barrier of the one-launch
+ *                         sort (small worlds) gives up (default 2^22, seconds);
+ *                         that step does not happen, and the next call that
+ *                         waits for the world fails once (0: every such step,
+ *                         for tests of the caller's handling).
  * phy_fluid_get_tuning reads the same parameters. */
 enum {
   PHY_TUNE_COMP_TILE = 0,
@@ -292,7 +297,8 @@ enum {
   PHY_TUNE_SORT_BLOCK = 4,
   PHY_TUNE_GRAPH_CHUNK = 5,
   PHY_TUNE_DENSE_MEAN = 6,
-  PHY_TUNE_DENSE_MASKS = 7
+  PHY_TUNE_DENSE_MASKS = 7,
+  PHY_TUNE_SORT_POLLS = 8
 };
 int32_t phy_fluid_set_tuning(PhyWorldHandle *w, uint32_t sub, int32_t param, int64_t value);
 int32_t phy_fluid_get_tuning(PhyWorldHandle *w, uint32_t sub, int32_t param, int64_t *out);

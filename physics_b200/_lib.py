@@ -24,9 +24,10 @@ TUNE_SORT_BLOCK = 4
 TUNE_GRAPH_CHUNK = 5
 TUNE_DENSE_MEAN = 6
 TUNE_DENSE_MASKS = 7
+TUNE_SORT_POLLS = 8
 TUNE_PARAMS = {"comp_tile": TUNE_COMP_TILE, "halo_cap": TUNE_HALO_CAP, "ctas_per_sm": TUNE_CTAS_PER_SM,
                "queue": TUNE_QUEUE, "sort_block": TUNE_SORT_BLOCK, "graph_chunk": TUNE_GRAPH_CHUNK,
-               "dense_mean": TUNE_DENSE_MEAN, "dense_masks": TUNE_DENSE_MASKS}
+               "dense_mean": TUNE_DENSE_MEAN, "dense_masks": TUNE_DENSE_MASKS, "sort_polls": TUNE_SORT_POLLS}
 
 NOALLOC_MAX_PARTICLES = 65536
 NOALLOC_MAX_CELLS = 262144

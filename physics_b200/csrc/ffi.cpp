@@ -508,6 +508,10 @@ int32_t phy_fluid_set_tuning(PhyWorldHandle* w, uint32_t sub, int32_t param, int
         t.dense_masks = in_range(0, 1);
         fw.set_launch_tuning(t);
         break;
+      case PHY_TUNE_SORT_POLLS:
+        t.sort_polls = in_range(0, 1 << 30);
+        fw.set_launch_tuning(t);
+        break;
       default:
         throw std::invalid_argument("unknown tuning parameter");
     }
@@ -529,6 +533,7 @@ int32_t phy_fluid_get_tuning(PhyWorldHandle* w, uint32_t sub, int32_t param, int
       case PHY_TUNE_GRAPH_CHUNK: *out = fw.graph_chunk(); break;
       case PHY_TUNE_DENSE_MEAN: *out = fw.dense_mean(); break;
       case PHY_TUNE_DENSE_MASKS: *out = t.dense_masks; break;
+      case PHY_TUNE_SORT_POLLS: *out = t.sort_polls; break;
       default: throw std::invalid_argument("unknown tuning parameter");
     }
     return 0;

@@ -479,6 +479,7 @@ FluidWorld::FluidWorld(const SphParams& p, Precision prec) : params(p), prec_(pr
   b_.counters = reinterpret_cast<unsigned long long*>(d_words_ + 256);
   cuda_check(cudaMallocHost((void**)&host_, sizeof(HostWords)), "cudaMallocHost");
   std::memset(host_, 0, sizeof(HostWords));
+  b_.sort_lost = &host_->sort_lost;
 }
 
 FluidWorld::~FluidWorld() {
@@ -545,7 +546,18 @@ void FluidWorld::set_stream(cudaStream_t s) {
   stream_ = s ? s : own_stream_;
 }
 
-void FluidWorld::synchronize() { cuda_check(cudaStreamSynchronize(stream_), "synchronize"); }
+void FluidWorld::synchronize() {
+  cuda_check(cudaStreamSynchronize(stream_), "synchronize");
+  check_sort();
+}
+
+void FluidWorld::check_sort() {
+  volatile uint32_t* word = &host_->sort_lost;
+  if (*word == 0u) return;
+  *word = 0u;
+  if (tape_.on) tape_.lost = true;
+  throw std::runtime_error("step: a grid barrier of the sort ran out of polls; that step did not happen");
+}
 
 // Grows every per-particle array to hold n particles (geometric growth),
 // keeping the current n_ particles.
@@ -1081,6 +1093,7 @@ void FluidWorld::get_field_device(int field, double* out) {
   stage_field(field, out);
   cuda_check(cudaGetLastError(), "get_field_device kernel");
   cuda_check(cudaStreamSynchronize(stream_), "get_field_device sync");
+  check_sort();
 }
 
 int FluidWorld::components(int field) {
@@ -1154,6 +1167,7 @@ void FluidWorld::get_field(int field, double* out) {
   cuda_check(cudaMemcpyAsync(out, st, (size_t)nc * n_ * sizeof(double), cudaMemcpyDeviceToHost, stream_),
              "get_field copy");
   cuda_check(cudaStreamSynchronize(stream_), "get_field sync");
+  check_sort();
 }
 
 void FluidWorld::get_vec_f64(int field, double* out, size_t count) {
@@ -1172,6 +1186,7 @@ void FluidWorld::get_vec_f64(int field, double* out, size_t count) {
   cuda_check(cudaMemcpyAsync(out, st, 3 * count * sizeof(double), cudaMemcpyDeviceToHost, stream_),
              "get_vec_f64 copy");
   cuda_check(cudaStreamSynchronize(stream_), "get_vec_f64 sync");
+  check_sort();
 }
 
 void FluidWorld::get_vec_f32(int field, float* out, size_t count) {
@@ -1186,6 +1201,7 @@ void FluidWorld::get_vec_f32(int field, float* out, size_t count) {
   cuda_check(cudaGetLastError(), "get_vec_f32 kernel");
   cuda_check(cudaMemcpyAsync(out, st, 3 * count * sizeof(float), cudaMemcpyDeviceToHost, stream_), "get_vec_f32 copy");
   cuda_check(cudaStreamSynchronize(stream_), "get_vec_f32 sync");
+  check_sort();
 }
 
 void FluidWorld::set_field(int field, const double* in) {
@@ -1311,7 +1327,7 @@ void FluidWorld::enqueue_step(const StepConsts& c, const PassEvents& pe, const c
   unsigned long long* saved = b_.counters;
   if (!counting_) b_.counters = nullptr;
   if (ev) cuda_check(cudaEventRecord(ev[0], stream_), "event");
-  launch_sort(c, b_, stream_, tuning_.sort_block);
+  launch_sort(c, b_, stream_, tuning_);
   if (ev) cuda_check(cudaEventRecord(ev[1], stream_), "event");
   if (prec_ == Precision::F64Plain)
     launch_plain_passes(c, b_, stream_, pe);
@@ -1394,7 +1410,7 @@ void FluidWorld::run_graph(double dt, int k) {
   std::memcpy(key.data(), &c, sizeof(StepConsts));
   long long extra[8] = {k, (long long)alloc_gen_, b_.cur, counting_ ? 1 : 0, b_.has_ba ? 1 : 0,
                         tuning_.ctas_per_sm + 1000ll * tuning_.queue + 10000ll * tuning_.dense_masks,
-                        tuning_.sort_block,
+                        tuning_.sort_block + 1000ll * tuning_.sort_polls,
                         (long long)(uintptr_t)stream_};
   std::memcpy(key.data() + sizeof(StepConsts), extra, sizeof(extra));
   const int cur0 = b_.cur;
@@ -1662,6 +1678,7 @@ std::vector<TuneTrial> FluidWorld::autotune(double dt, int steps, int horizon) {
           t.ctas_per_sm = tiled ? per : 0;
           t.queue = queue;
           t.sort_block = sort_block;
+          t.sort_polls = tuning_.sort_polls;
           cands.push_back({t, tile});
         }
   const LaunchTuning saved = tuning_;
@@ -1949,7 +1966,7 @@ void FluidWorld::couple_bodies(PhyCoupleBody* bodies, uint32_t nb, const double*
 int FluidSubsystem::validate() {
   if (world->is_empty()) return 0;
   uint32_t f = world->last_step_flags();
-  if (f & kFlagSortLost) return -1;
+  world->check_sort();
   if (f & kFlagNonFinite) return 2;
   if (f & kFlagOutOfBox) return 5;
   return 0;
@@ -2063,6 +2080,7 @@ void FluidWorld::tape_begin(int every) {
   tape_.nckpt = 0;
   tape_.dts.clear();
   tape_.direct = 0;
+  tape_.lost = false;
   tape_.every = every;
   tape_.params = params.to_c();
   save_checkpoint();
@@ -2207,6 +2225,7 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
   if (n == 0) return;
   if (T > 0 && n != tape_.n)
     throw std::invalid_argument("step_backward: particles were added while the tape was recording");
+  if (tape_.lost) throw std::runtime_error("step_backward: a step of the tape did not happen (its sort was lost)");
   cudaStream_t s = stream_;
   // Work arrays: the packed operands (kAdjRec), gx_ins, gv_ins, gx, gv (3
   // each), rbar, rbar_tot, cc, kk, the tape's fv and shear outputs (4): arrays
@@ -2279,6 +2298,7 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
       launch_deinterleave3(b_.stage + 3 * n, w.gv_ins[0], w.gv_ins[1], w.gv_ins[2], (int)n, s);
     }
     cuda_check(cudaStreamSynchronize(s), "seed sync");
+    check_sort();
     recomputing_ = true;
     const int every = tape_.every;
     const int nseg = (T + every - 1) / every;
@@ -2360,6 +2380,7 @@ void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, 
                  "gradient read");
     cuda_check(cudaMemcpyAsync(pa, w.param_acc, sizeof(pa), cudaMemcpyDeviceToHost, s), "gradient read");
     cuda_check(cudaStreamSynchronize(s), "gradient sync");
+    check_sort();
     if (gparams) {
       gparams[0] = pa[0];
       gparams[1] = pa[1];

@@ -144,6 +144,10 @@ class FluidWorld {
   void set_stream(cudaStream_t s);
   cudaStream_t stream() const { return stream_; }
   void synchronize();
+  // Throws, once, when a step since the last report did not happen because a
+  // grid barrier of its sort gave up (the particles are those before it); to
+  // be called after a wait for the stream.
+  void check_sort();
   // Error bits of the last step (synchronises).
   uint32_t last_step_flags();
   // Candidates / pairs of the last step (synchronises); counting is enabled
@@ -266,6 +270,7 @@ class FluidWorld {
   struct HostWords {
     long long box[7];  // min xyz, max xyz, non-finite flag
     unsigned long long mask_demand;
+    uint32_t sort_lost;
   };
   HostWords* host_ = nullptr;
   uint32_t* sort_words_ = nullptr;  // cell_of, rank, tmp, perm, sorted_cell
@@ -312,6 +317,7 @@ class FluidWorld {
     std::vector<double> dts;
     std::vector<double*> ckpt;  // pool; the first nckpt are this tape's
     size_t nckpt = 0;
+    bool lost = false;  // a step of it did not happen
     int direct = -1;  // leading steps recorded as they ran; -1: none can be
     PhySphParams params;
   } tape_;

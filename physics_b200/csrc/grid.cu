@@ -812,6 +812,8 @@ struct SortArgs {
   uint32_t* large;
   uint32_t* large_count;
   uint32_t* barrier;      // arrivals, zeroed before the launch
+  int polls;              // of a barrier before the step is given up
+  uint32_t* lost;         // mapped host memory
   uint32_t* tile_of;
   uint32_t* tile_slot;
   uint32_t* num_tiles;
@@ -820,23 +822,25 @@ struct SortArgs {
   GatherArgs g;
 };
 
-// Waits until every block has arrived for the `phase`-th time; false (and the
-// error bit set) when the others do not arrive within the poll limit, which a
-// cooperative launch never lets happen.
-__device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t phase, uint32_t* flags) {
+// Waits until every block has arrived for the `phase`-th time; false (with the
+// error bit and the host's word set) when the others do not arrive within the
+// poll limit, seconds in a cooperative launch, whose blocks all run.
+__device__ __forceinline__ bool grid_barrier(const SortArgs& a, uint32_t phase) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(counter, 1u);
+    atomicAdd(a.barrier, 1u);
     const uint32_t want = phase * gridDim.x;
     uint32_t seen = 0;
-    int polls = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
-    } while (seen < want && ++polls < (1 << 22));
+    for (int polls = 0; seen < want && polls < a.polls; ++polls)
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.barrier) : "memory");
     s_ok = seen >= want;
-    if (seen < want) atomicOr(flags, kFlagSortLost);
+    if (seen < want) {
+      atomicOr(a.h.flags, kFlagSortLost);
+      *(volatile uint32_t*)a.lost = 1u;
+      __threadfence_system();
+    }
     __threadfence();
   }
   __syncthreads();
@@ -858,16 +862,16 @@ __global__ void __launch_bounds__(kThreads) k_sort_fused(StepConsts c, SortArgs 
   for (uint32_t k = (uint32_t)first + threadIdx.x; k < a.len / 4u; k += (uint32_t)step) zero[k] = make_uint4(0, 0, 0, 0);
   if (kCells == 0)
     for (uint32_t k = (uint32_t)first + threadIdx.x; k < blocks; k += (uint32_t)step) a.sums[k] = make_uint2(0u, 0u);
-  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (!grid_barrier(a, ++phase)) return;
   for (int i0 = first; i0 < n; i0 += step) cell_hist(c, a.h, i0 + (int)threadIdx.x);  // whole blocks
-  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (!grid_barrier(a, ++phase)) return;
   if (kCells != 0) {
     // (A tile's few counters would be contended if the histogram summed them.)
     for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
       tile_reduce(a.h.buckets, a.h.count, a.sums, b);
       __syncthreads();
     }
-    if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+    if (!grid_barrier(a, ++phase)) return;
   }
   for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
     if (kCells == 0) {
@@ -879,10 +883,10 @@ __global__ void __launch_bounds__(kThreads) k_sort_fused(StepConsts c, SortArgs 
       tile_scan(n, a.ncells, a.h.buckets, a.h.count, a.sums, a.cell_start, a.tile_of, a.tile_slot, a.num_tiles, b);
     }
   }
-  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (!grid_barrier(a, ++phase)) return;
   for (int i0 = first; i0 < n; i0 += step)
     scatter(n, a.h.bucket_shift, a.h.cell_of, a.h.rank, a.h.count, a.tmp, i0 + (int)threadIdx.x);
-  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (!grid_barrier(a, ++phase)) return;
   allow_next();
   auto list = [&](uint32_t slot, uint32_t i) { a.perm[slot] = i; };
   if (kCells == 0 && *a.h.crowded == 0u) {  // settled by the histogram: uniform across the grid
@@ -900,11 +904,11 @@ __global__ void __launch_bounds__(kThreads) k_sort_fused(StepConsts c, SortArgs 
                                          a.h.rank, a.out, a.cell_start, a.tile_slot, a.tile_crowd, a.dense_mean,
                                          a.large, a.large_count, tile_stage, list);
   }
-  if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+  if (!grid_barrier(a, ++phase)) return;
   if (*a.large_count != 0u) {  // uniform
     order_large<kThreads>(a.cell_start, kCells == 0 ? a.tmp : a.out, a.h.id, a.h.okey, a.large, a.large_count,
                           large_stage, list);
-    if (!grid_barrier(a.barrier, ++phase, a.h.flags)) return;
+    if (!grid_barrier(a, ++phase)) return;
   }
   for (int s0 = first; s0 < n; s0 += step)
     if (s0 + (int)threadIdx.x < n) move_particle(a.g, (uint32_t)(s0 + (int)threadIdx.x), a.perm[s0 + (int)threadIdx.x]);
@@ -1079,7 +1083,7 @@ static int fused_blocks() {
 }
 
 template <int kCells>
-static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g, cudaStream_t s) {
+static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g, int polls, cudaStream_t s) {
   SortArgs a;
   a.h = hist_args(c, b, c.tile ? b.okey : nullptr, b.flags);
   a.ncells = c.ncells;
@@ -1095,6 +1099,8 @@ static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g
   a.large = c.tile ? b.large_cells : b.rank;
   a.large_count = b.order_count;
   a.barrier = b.order_count + 1;
+  a.polls = polls;
+  a.lost = b.sort_lost;
   a.tile_of = b.tile_of;
   a.tile_slot = b.tile_slot;
   a.num_tiles = b.num_tiles;
@@ -1110,9 +1116,9 @@ static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g
                               dim3(kThreads), args, sizeof(LargeStage), s);
 }
 
-void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, int block) {
+void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, const LaunchTuning& t) {
   // Per-particle kernels take any warp multiple up to kThreads.
-  const int bs = block >= 32 && block <= kThreads ? block / 32 * 32 : kThreads;
+  const int bs = t.sort_block >= 32 && t.sort_block <= kThreads ? t.sort_block / 32 * 32 : kThreads;
   const int n = c.n;
   const ParticleConsts& src = b.pc[b.cur];
   const ParticleConsts& dst = b.pc[b.cur ^ 1];
@@ -1141,11 +1147,11 @@ void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, int block) 
   const int buckets = c.tile ? c.ncells >> (3 * c.tile_log2) : c.ncells;
   if (n < kFusedBelow && buckets < kFusedBuckets) {
     if (c.tile == 4)
-      launch_fused<64>(c, b, g, s);
+      launch_fused<64>(c, b, g, t.sort_polls, s);
     else if (c.tile == 2)
-      launch_fused<8>(c, b, g, s);
+      launch_fused<8>(c, b, g, t.sort_polls, s);
     else
-      launch_fused<0>(c, b, g, s);
+      launch_fused<0>(c, b, g, t.sort_polls, s);
   } else {
     build_cells(c, b, s, bs, c.tile ? b.okey : nullptr, b.flags);
     k_gather<<<grid_for(n, bs), bs, 0, s>>>(n, b.perm, g);

@@ -20,6 +20,17 @@ struct ParticleConsts {
   uint16_t* scene = nullptr;  // scene of a batched world, optional
 };
 
+// A step whose sort was lost keeps its particles: the passes' current
+// constants become those the sort started from again (pv1 was not written).
+__device__ __forceinline__ void keep_particle(const ParticleConsts& from, const ParticleConsts& to, int i) {
+  to.mass[i] = from.mass[i];
+  to.mat[i] = from.mat[i];
+  to.id[i] = from.id[i];
+  if (from.ba[0])
+    for (int k = 0; k < 3; ++k) to.ba[k][i] = from.ba[k][i];
+  if (from.scene) to.scene[i] = from.scene[i];
+}
+
 struct DevBuffers {
   int capacity = 0;        // particles
   int cell_capacity = 0;   // grid cells (excluding the overflow cell)
@@ -111,6 +122,7 @@ struct DevBuffers {
   // [2] the sort's large-cell count, [3] its barrier arrivals, [4] whether a
   // bucket is crowded, [6..7] mask_ctl; zeroed by one memset per step (device).
   uint32_t* flags = nullptr;
+  uint32_t* sort_lost = nullptr;  // mapped host memory, set when a sort was lost
   uint32_t* order_count = nullptr;  // sort: cells of more than kOrderSmall particles (flags + 2)
   unsigned long long* counters = nullptr;  // candidates, pairs (device)
   // Optional outputs of the f64 plain force pass for the adjoint's tape: the
@@ -120,7 +132,8 @@ struct DevBuffers {
 };
 
 // grid.cu
-void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, int block = 256);
+struct LaunchTuning;
+void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, const LaunchTuning& t);
 // The cells of the current positions without moving the state: cell_start
 // over the box and perm[s] = the particle at sorted slot s in (cell,
 // insertion index) order.  c.tile must be 0 (x-major cells).  The
@@ -221,6 +234,7 @@ struct LaunchTuning {
   int ctas_per_sm = 0;
   int queue = 0;
   int sort_block = 256;
+  int sort_polls = 1 << 22;  // polls of a grid barrier of the one-launch sort before the step is given up
   int dense_masks = 1;  // 1: the dense-cell force pass walks the density pass's masks
 };
 

@@ -54,7 +54,10 @@ constexpr int kStepWords = 8;
 enum : uint32_t {
   kFlagOutOfBox = 1u,    // a cell key fell outside the grid box
   kFlagNonFinite = 2u,   // a new position or velocity is NaN/Inf
-  kFlagSortLost = 8u,   // a grid barrier of the fused sort ran out of polls: the step did not happen
+  // A grid barrier of the fused sort ran out of polls.  The step does not
+  // happen: its passes write nothing but the constants of the old order
+  // (keep_particle), and the host reports it at the next wait.
+  kFlagSortLost = 8u,
   kFlagMaskTable = 4u,   // a dense-cell task's kept masks lie outside the mask buffer (filtered again)
 };
 

@@ -56,6 +56,7 @@ struct CompArgs {
   uint32_t* nbr_count;
   int stride;
   uint32_t* flags;
+  ParticleConsts before, now;  // constants the sort read and wrote
   unsigned long long* counters;
 };
 
@@ -63,6 +64,10 @@ struct CompArgs {
 __global__ void __launch_bounds__(kThreads) k_prep_comp(StepConsts c, CompArgs a) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.n) return;
+  if (a.flags[0] & kFlagSortLost) {
+    keep_particle(a.before, a.now, i);
+    return;
+  }
   const double x = a.px[i], y = a.py[i], z = a.pz[i];
   const long long kx = key_axis(x, c.inv_cell);
   const long long ky = key_axis(y, c.inv_cell);
@@ -83,7 +88,7 @@ template <bool kCount>
 __global__ void __launch_bounds__(kThreads) k_density_comp(StepConsts c, CompArgs a) {
   __shared__ uint32_t s_list[kStagedNeighbors][kThreads];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
+  if (i >= c.n || (a.flags[0] & kFlagSortLost)) return;
   const double xi = a.px[i], yi = a.py[i], zi = a.pz[i];
   const long long kx = key_axis(xi, c.inv_cell);
   const long long ky = key_axis(yi, c.inv_cell);
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(kThreads) k_force_comp(StepConsts c, CompArgs 
   }
   __syncthreads();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
+  if (i >= c.n || (a.flags[0] & kFlagSortLost)) return;
   const double xi = a.px[i], yi = a.py[i], zi = a.pz[i];
   const double vxi = a.vx[i], vyi = a.vy[i], vzi = a.vz[i];
   const double rho_i = a.rho[i];
@@ -305,6 +310,8 @@ __global__ void __launch_bounds__(kThreads) k_force_comp(StepConsts c, CompArgs 
 void launch_comp_passes(const StepConsts& c, DevBuffers& b, cudaStream_t s, const PassEvents& ev) {
   const ParticleConsts& pc = b.pc[b.cur];
   CompArgs a;
+  a.before = b.pc[b.cur ^ 1];
+  a.now = pc;
   a.px = b.pv0[0];
   a.py = b.pv0[1];
   a.pz = b.pv0[2];

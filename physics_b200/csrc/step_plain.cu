@@ -73,6 +73,7 @@ struct PlainArgs {
   uint32_t* cand;
   uint32_t* hits;
   uint2* group;
+  ParticleConsts before, now;       // constants the sort read and wrote
   double* rec0;                     // packed pair operands, three parts
   double* rec1;
   double2* rec2;
@@ -129,6 +130,7 @@ constexpr int kDensityCtas = 8;
 constexpr int kSms = 148;
 constexpr int kZSpan = 6;     // z cells a warp's query segment may span
 constexpr int kSlotBits = 27; // slot index bits of a candidate word; the z cell modulo 32 sits above
+constexpr uint32_t kLostGroup = 0xffffffffu;  // words of a group whose step does not happen
 // Queries whose 27 cells hold at most this many particles (spray, sparse
 // scenes) walk them one by one instead of sharing a staged segment.
 constexpr unsigned kWalkBelow = 40;
@@ -193,7 +195,7 @@ __device__ __forceinline__ void density_term(const StepConsts& c, const PlainArg
 // only lets in candidates that the density pass's f64 test then rejects, so
 // the result is the reference's bit for bit.  A group whose candidates exceed
 // its record, and queries in sparse surroundings, are left to the density
-// pass's own walk (PlainArgs::walkers).
+// pass's own walk (PlainArgs::group).
 __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_search_plain(StepConsts c, PlainArgs a) {
   after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
@@ -204,9 +206,15 @@ __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_search_plain
   const int i = min(group * 32 + lane, c.n - 1);
   const float4 own = a.fpos[i];
   const uint32_t cell = a.sorted_cell[i];
-  // Else the overflow cell (or a sort that did not finish).
-  const bool inside =
-      group * 32 + lane < c.n && cell < (uint32_t)c.ncells && (a.flags[0] & kFlagSortLost) == 0u;
+  if (a.flags[0] & kFlagSortLost) {
+    if (group * 32 + lane < c.n) {
+      keep_particle(a.before, a.now, i);
+      a.nbr_count[i] = 0;  // (a recorded step then has no lists to follow)
+    }
+    if (lane == 0) a.group[group] = make_uint2(kLostGroup, 0u);
+    return;
+  }
+  const bool inside = group * 32 + lane < c.n && cell < (uint32_t)c.ncells;  // else the overflow cell
   const int bz = __float_as_int(own.w);
   const int col = (int)cell - bz;  // first cell of the column
   uint32_t* slots = a.cand + (size_t)group * (kSearchWords * 32);
@@ -346,6 +354,7 @@ __global__ void __launch_bounds__(kDensityWarps * 32, kDensityCtas) k_density_pl
   const bool valid = i < c.n;
   const int ii = valid ? i : c.n - 1;
   const uint2 rec = a.group[group];
+  if (rec.x == kLostGroup) return;
   {
     const uint32_t* slots = a.cand + (size_t)group * (kSearchWords * 32) + lane;
     const uint32_t* hits = a.hits + ii;
@@ -460,7 +469,8 @@ __global__ void __launch_bounds__(kDensityWarps * 32, kDensityCtas) k_density_pl
 // a / b given y = 1/b rounded to nearest: q = a y is within an ulp of the
 // quotient, its remainder is exact in one FMA, and the corrected quotient is
 // the correctly rounded one (Markstein, IBM J. Res. Dev. 34(1), 1990),
-// provided nothing under- or overflows on the way (StepSafe below).  The sign
+// provided nothing under- or overflows on the way: the sort's gather
+// (plain_safe) and the density pass set flags[1] otherwise.  The sign
 // of a zero quotient may differ, which no sum starting at +0 can show.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   const double q = __dmul_rn(a, y);
@@ -764,7 +774,9 @@ __global__ void __launch_bounds__(kThreads, kForceCtas) k_force_plain(StepConsts
   if (kG == 1 && !valid) return;
   const int ii = valid ? i : c.n - 1;
   double* buf = s_buf[kG == 1 ? 0 : threadIdx.x >> 5];
-  const bool fast = a.flags[1] == 0u && c.h < 1e100;  // uniform
+  const uint2 flags = *reinterpret_cast<const uint2*>(a.flags);  // uniform
+  if (flags.x & kFlagSortLost) return;
+  const bool fast = flags.y == 0u && c.h < 1e100;
   const PlainAcc q = fast ? plain_sums<kG, kShear, true>(c, a, ii, valid, lane, buf)
                           : plain_sums<kG, kShear, false>(c, a, ii, valid, lane, buf);
   if (valid && (kG == 1 || lane % kG == 0)) finish_plain(c, a, i, q);
@@ -800,6 +812,8 @@ void launch_plain_passes(const StepConsts& c, DevBuffers& b, cudaStream_t s, con
   a.rec1 = b.rec + 4 * (size_t)b.capacity;
   a.rec2 = reinterpret_cast<double2*>(b.rec + 8 * (size_t)b.capacity);
   a.cull2 = plain_cull2(c);
+  a.before = b.pc[b.cur ^ 1];
+  a.now = pc;
   a.px = b.pv0[0];
   a.py = b.pv0[1];
   a.pz = b.pv0[2];

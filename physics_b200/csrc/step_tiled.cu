@@ -107,6 +107,7 @@ struct TiledArgs {
   int stride;
   uint32_t* flags;
   unsigned long long* counters;
+  ParticleConsts before, now;  // constants the sort read and wrote
 };
 
 // Packed f32x2 arithmetic (sm_100): two lanes of a 64-bit register pair per
@@ -173,14 +174,9 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* ws, uint32_
   return off + x - v;
 }
 
-// Tiles of the list: none when the sort did not finish.
-__device__ __forceinline__ uint32_t occupied_tiles(const TiledArgs& a) {
-  return (a.flags[0] & kFlagSortLost) ? 0u : *a.num_tiles;
-}
-// First slot of the overflow cell when no tile is occupied.
-__device__ __forceinline__ uint32_t first_outside(const TiledArgs& a) {
-  return (a.flags[0] & kFlagSortLost) ? 0u : a.tile_slot[0];
-}
+// Whether the sort was lost: then no pass of the step writes anything but the
+// kept constants.
+__device__ __forceinline__ bool sort_lost(const TiledArgs& a) { return (a.flags[0] & kFlagSortLost) != 0u; }
 
 // Work items per tile: a world of few tiles splits each into x-slabs (the
 // slabs a tile with a large halo runs in), so that its queries spread over
@@ -478,7 +474,12 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2), H0SQ = f2_pack(c.h0sqf, c.h0sqf);
   __shared__ uint32_t s_next;
-  const uint32_t ntiles = occupied_tiles(a);
+  if (sort_lost(a)) {
+    for (int i = (int)(blockIdx.x * kTT + threadIdx.x); i < c.n; i += (int)(gridDim.x * kTT))
+      keep_particle(a.before, a.now, i);
+    return;
+  }
+  const uint32_t ntiles = *a.num_tiles;
   unsigned cand = 0, pairs = 0;
   const uint32_t parts = tile_parts<TB>(ntiles);
   const int layers = T::B / (int)parts;
@@ -545,7 +546,7 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
     }  // slabs
   }
   // Particles of the overflow cell (outside the grid box): no neighbours.
-  const uint32_t end = ntiles ? a.tile_slot[ntiles] : first_outside(a);
+  const uint32_t end = a.tile_slot[ntiles];
   for (uint32_t qi = end + blockIdx.x * kTT + threadIdx.x; qi < (uint32_t)c.n; qi += gridDim.x * kTT) {
     write_density(c, a, (int)qi, 0.0);
     a.nbr_count[qi] = 0;
@@ -822,7 +823,8 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
   uint32_t* ws = s_off + T::NH + 1;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   __shared__ uint32_t s_next;
-  const uint32_t ntiles = occupied_tiles(a);
+  if (sort_lost(a)) return;
+  const uint32_t ntiles = *a.num_tiles;
   const uint32_t parts = tile_parts<TB>(ntiles);
   const int layers = T::B / (int)parts;
   for (uint32_t item = next_tile(a.queue, 1, blockIdx.x, &s_next); item < ntiles * parts;
@@ -901,7 +903,7 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
     __syncthreads();
     }  // slabs
   }
-  const uint32_t end = ntiles ? a.tile_slot[ntiles] : first_outside(a);
+  const uint32_t end = a.tile_slot[ntiles];
   for (uint32_t qi = end + blockIdx.x * kTT + threadIdx.x; qi < (uint32_t)c.n; qi += gridDim.x * kTT) {
     CompAcc q;
     finish_particle(c, a, (int)qi, q, c.boxes[a.scene ? (int)a.scene[qi] : 0], load_own(a, (int)qi));
@@ -1098,7 +1100,7 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
   const int lane = threadIdx.x & 31;
   float* sp = s_pp[threadIdx.x >> 5];
   const float4* sp4 = reinterpret_cast<const float4*>(sp);
-  const uint32_t ntasks = *a.dense_count;
+  const uint32_t ntasks = sort_lost(a) ? 0u : *a.dense_count;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2), H0SQ = f2_pack(c.h0sqf, c.h0sqf);
   unsigned cand = 0, pairs = 0;
@@ -1227,7 +1229,7 @@ template <int TB, bool kShear>
 __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs a) {
   after_previous();
   // The entries this step's tasks asked for, for the host's next sizing.
-  if (a.mask_demand && blockIdx.x == 0 && threadIdx.x == 0) *a.mask_demand = *a.mask_ctl;
+  if (a.mask_demand && blockIdx.x == 0 && threadIdx.x == 0 && !sort_lost(a)) *a.mask_demand = *a.mask_ctl;
   // The chunk's 32 candidates, and in slot 32 a weightless copy of its first
   // (mass and m/rho 0) that pads the two-candidate rounds.
   __shared__ float4 s_pos[kWarps][33];
@@ -1237,7 +1239,7 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float* sp = s_pp[w];
   const float4* sp4 = reinterpret_cast<const float4*>(sp);
-  const uint32_t ntasks = *a.dense_count;
+  const uint32_t ntasks = sort_lost(a) ? 0u : *a.dense_count;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2);
   DenseTask t;
@@ -1524,6 +1526,8 @@ void launch_comp_tiled(const StepConsts& c, DevBuffers& b, cudaStream_t s, const
   a.stride = b.capacity;
   a.flags = b.flags;
   a.counters = b.counters;
+  a.before = b.pc[b.cur ^ 1];
+  a.now = pc;
   // Persistent grids: SM count x resident CTAs per SM (the occupancy limit,
   // or the tuned count when smaller).
   const Occupancy& o = occupancy();

@@ -375,7 +375,7 @@ class FluidWorld:
 
     def set_tuning(self, **knobs: int) -> None:
         """Kernel configuration (phy_fluid_set_tuning): comp_tile, halo_cap, ctas_per_sm, queue,
-        sort_block, graph_chunk, dense_mean, dense_masks.  Results of the f64 form never
+        sort_block, graph_chunk, dense_mean, dense_masks, sort_polls.  Results of the f64 form never
         change; the launch knobs (ctas_per_sm, queue, sort_block, graph_chunk, dense_masks)
         change no result of either form."""
         for name, value in knobs.items():

@@ -166,3 +166,27 @@ def test_a_new_world_maps_few_blocks_of_memory(fake, form, most):
     w = _world(form, n=64000)
     w.step(DT)
     assert fake.fake_device_calls() <= most and fake.fake_pinned_calls() <= 1
+
+
+def test_a_lost_sort_is_reported_once_at_the_next_wait(fake):
+    """The word a kernel sets in mapped memory (after the box and the mask demand)."""
+    w = _world()
+    for wait in (w.synchronize, lambda: w.get(pb.FIELD_RHO), lambda: w.pos, lambda: w.total_momentum()):
+        w.step(DT)
+        fake.fake_poke_pinned(64, 1)
+        with pytest.raises(L.PhyError, match="did not happen"):
+            wait()
+        wait()
+    fake.fake_poke_pinned(64, 1)
+    with pytest.raises(L.PhyError, match="did not happen"):
+        w._world.step_checked(DT)
+    assert w._world.step_checked(DT) == 0
+    w.tape_begin(2)
+    w.step(DT, 3)
+    fake.fake_poke_pinned(64, 1)
+    for _ in range(2):
+        with pytest.raises(L.PhyError, match="did not happen"):
+            w.step_backward(np.ones((64, 3)), None)
+    w.tape_begin(2)
+    w.step(DT, 3)
+    w.step_backward(np.ones((64, 3)), None)
