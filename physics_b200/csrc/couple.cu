@@ -21,7 +21,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <stdexcept>
 #include <vector>
 
 #include "sph_buffers.h"
@@ -40,7 +39,7 @@ struct CoupleArgs {
   double* vz;
   const double* mass;
   double* pts;  // 10 doubles per point: pos xyz, vel xyz, mass, force xyz
-  int np;
+  uint32_t* err;  // set by a walk that gave up (zero before the first batch)
   double dt, drag, soft_density;
 };
 
@@ -103,9 +102,8 @@ constexpr int kWB = 32 * kPer;  // candidates per chunk of a warp
 constexpr int kPB = 4096;       // candidates a point may have for a list
 constexpr int kTabU = 56;       // u32 per point table: in, total, beg[27], cnt[27]
 
-// The walk's words: ticket, error flag (two words, kFlowHead in all), then a
-// done flag per point.
-constexpr int kFlowHead = 2;
+// The walk's words: the ticket, then a done flag per point.
+constexpr int kFlowHead = 1;
 
 // world.rs:704-711 (a NaN coordinate passes, as there).
 __device__ __forceinline__ bool point_in(const StepConsts& c, const double* q) {
@@ -116,7 +114,7 @@ __device__ __forceinline__ bool point_in(const StepConsts& c, const double* q) {
 // One warp per point w of the batch: in-bounds flag, candidate count and
 // cell ranges, and key[w]: the centre cell in box coordinates (clamped far
 // outside the box, where a false overlap only costs a wait) and the in-bounds
-// flag.  Also clears the walk's ticket, error and done words.
+// flag.  Also clears the walk's ticket and done words.
 __device__ __forceinline__ int box_coord(long long k, long long b0) {
   const long long d = k - b0, far = 1ll << 28;
   return (int)(d < -far ? -far : d > far ? far : d);
@@ -149,8 +147,7 @@ __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a
     totals[w] = in && total <= (uint32_t)kPB ? total : 0u;
     key[w] = make_int4(box_coord(kx, c.bx0), box_coord(ky, c.by0), box_coord(kz, c.bz0), in ? 1 : 0);
     done[kFlowHead + w] = 0u;
-    if (w == 0)
-      for (int h = 0; h < kFlowHead; ++h) done[h] = 0u;
+    if (w == 0) done[0] = 0u;
   }
 }
 
@@ -160,30 +157,34 @@ __global__ void __launch_bounds__(256) k_point_tables(StepConsts c, CoupleArgs a
 __global__ void __launch_bounds__(256) k_point_candidates(CoupleArgs a, int nb, const uint32_t* tab,
                                                           const uint32_t* off, uint32_t* idx, double* m,
                                                           double* msum) {
+  __shared__ double s_m[256 / 32][kWB];
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= nb) return;
   const uint32_t* t = tab + (size_t)w * kTabU;
   if (!t[0] || t[1] > (uint32_t)kPB) return;
-  uint32_t o = off[w];
+  const uint32_t total = t[1], first = off[w];
+  const bool held = total <= (uint32_t)kWB;
+  double* sm = s_m[threadIdx.x >> 5];
+  uint32_t o = first;
   for (int u = 0; u < 27; ++u) {
     const uint32_t beg = t[2 + u], cnt = t[29 + u];
     for (uint32_t e = lane; e < cnt; e += 32) {
       const uint32_t i = a.perm[beg + e];
+      const double mi = a.mass[i];
       idx[o + e] = i;
-      m[o + e] = a.mass[i];
+      m[o + e] = mi;
+      if (held) sm[o - first + e] = mi;
     }
     o += cnt;
   }
   // The masses' sum in visit order, for the points the walk holds in
-  // registers.
-  const uint32_t total = t[1];
-  if (total <= (uint32_t)kWB) {
+  // registers (from shared memory: one point's took 10 us from global).
+  if (held) {
     __syncwarp();
     if (lane == 0) {
-      const double* p = m + off[w];
       double sw = 0.0;
 #pragma unroll 8
-      for (uint32_t e = 0; e < total; ++e) sw = sw + p[e];
+      for (uint32_t e = 0; e < total; ++e) sw = sw + sm[e];
       msum[w] = sw;
     }
   }
@@ -196,7 +197,7 @@ struct PointLists {
   const double* m;
   const double* msum;
   const int4* key;
-  uint32_t* flow;  // ticket, error, done flags
+  uint32_t* flow;  // ticket, done flags
 };
 
 // Cell table of a point without a list (its warp's copy).
@@ -365,7 +366,7 @@ __device__ __forceinline__ void walk_held(const StepConsts& c, const CoupleArgs&
 // The walk over the nb points of a batch.  Warps take points by ticket, in
 // order, so the points a warp waits for are held by running warps (or done)
 // and the wait ends; it gives up after a poll limit all the same, with the
-// error word set and the remaining points unwalked.
+// error word set and the remaining points (of later batches too) unwalked.
 __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, CoupleArgs a, int nb, PointLists L) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ WarpTable s_tab[kFW];
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, C
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double2* pw = reinterpret_cast<double2*>(smem) + (size_t)warp * 2 * kWB;
   uint32_t* done = L.flow + kFlowHead;
+  if (__any_sync(0xffffffffu, *(volatile uint32_t*)a.err != 0u)) return;
   for (;;) {
     uint32_t k = 0;
     if (lane == 0) k = atomicAdd(L.flow, 1u);
@@ -393,12 +395,12 @@ __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, C
       for (int polls = 0; polls < (1 << 22); ++polls) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(done + j) : "memory");
         if (seen) break;
-        if ((polls & 255) == 255 && *(volatile uint32_t*)(L.flow + 1)) break;
+        if ((polls & 255) == 255 && *(volatile uint32_t*)a.err) break;
       }
       ok = ok && seen != 0u;
     }
     if (!__all_sync(0xffffffffu, ok)) {
-      if (lane == 0) atomicOr(L.flow + 1, 1u);
+      if (lane == 0) atomicOr(a.err, 1u);
       return;
     }
     __syncwarp();  // what a lane's acquire makes visible, every lane reads
@@ -1180,8 +1182,8 @@ void CouplePointsScratch::release() {
   cap_tab = cap_totals = cap_off = cap_idx = cap_m = cap_key = cap_flow = cap_msum = 0;
 }
 
-void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int np, double dt, double drag,
-                          double soft_density, cudaStream_t s, CouplePointsScratch& sc) {
+void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, uint32_t* d_err, int np, double dt,
+                          double drag, double soft_density, cudaStream_t s, CouplePointsScratch& sc) {
   CoupleArgs a;
   a.cell_start = b.cell_start;
   a.perm = b.perm;
@@ -1190,7 +1192,7 @@ void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int
   a.vz = b.pv1[5];
   a.mass = b.pc[b.cur].mass;
   a.pts = d_pts;
-  a.np = np;
+  a.err = d_err;
   a.dt = dt;
   a.drag = drag;
   a.soft_density = soft_density;
@@ -1237,11 +1239,8 @@ void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int
     PointLists L{sc.tab, sc.off, sc.idx, sc.m, sc.msum, sc.key, sc.flow};
     k_couple_points_flow<<<std::min(flow_blocks, (nb + kFW - 1) / kFW), kFW * 32, kFlowSmem, s>>>(c, ab, nb, L);
     cuda_check(cudaGetLastError(), "couple points");
-    uint32_t failed = 0;
-    cuda_check(cudaMemcpyAsync(&failed, sc.flow + 1, sizeof(failed), cudaMemcpyDeviceToHost, s), "couple points status");
     // The offsets' host copy must outlive the upload.
     cuda_check(cudaStreamSynchronize(s), "couple points sync");
-    if (failed) throw std::runtime_error("couple_points: a point's wait for an earlier one ran out of polls");
   }
 }
 

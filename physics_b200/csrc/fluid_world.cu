@@ -1826,7 +1826,9 @@ void FluidWorld::couple_points(size_t np, const double* pos, const double* vel, 
   c.tile_log2 = 0;
   const size_t need = 10 * np + 1;
   dreserve(d_couple_, couple_cap_, need);
-  std::vector<double> h(10 * np);
+  // The points, then two words: the cell index's flags and the walk's error,
+  // which comes back with the forces.
+  std::vector<double> h(need, 0.0);
   for (size_t k = 0; k < np; ++k) {
     double* r = h.data() + 10 * k;
     for (int a = 0; a < 3; ++a) {
@@ -1838,11 +1840,15 @@ void FluidWorld::couple_points(size_t np, const double* pos, const double* vel, 
   }
   const size_t bytes = h.size() * sizeof(double);
   cuda_check(cudaMemcpyAsync(d_couple_, h.data(), bytes, cudaMemcpyHostToDevice, stream_), "couple upload");
-  launch_cell_index(c, b_, reinterpret_cast<uint32_t*>(d_couple_ + 10 * np), stream_);
-  launch_couple_points(c, b_, d_couple_, (int)np, dt, drag, soft_density, stream_, couple_scratch_);
+  uint32_t* words = reinterpret_cast<uint32_t*>(d_couple_ + 10 * np);
+  launch_cell_index(c, b_, words, stream_);
+  launch_couple_points(c, b_, d_couple_, words + 1, (int)np, dt, drag, soft_density, stream_, couple_scratch_);
   cuda_check(cudaGetLastError(), "couple launch");
   cuda_check(cudaMemcpyAsync(h.data(), d_couple_, bytes, cudaMemcpyDeviceToHost, stream_), "couple download");
   cuda_check(cudaStreamSynchronize(stream_), "couple sync");
+  uint32_t back[2];
+  std::memcpy(back, h.data() + 10 * np, sizeof(back));
+  if (back[1]) throw std::runtime_error("couple_points: a point's wait for an earlier one ran out of polls");
   for (size_t k = 0; k < np; ++k)
     for (int a = 0; a < 3; ++a) force[3 * k + a] = h[10 * k + 7 + a];
 }

@@ -162,8 +162,9 @@ struct CouplePointsScratch {
   size_t cap_tab = 0, cap_totals = 0, cap_off = 0, cap_idx = 0, cap_m = 0, cap_key = 0, cap_flow = 0, cap_msum = 0;
   void release();
 };
-void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, int np, double dt, double drag,
-                          double soft_density, cudaStream_t s, CouplePointsScratch& scratch);
+// d_err (zero on entry) is set when a point's wait for an earlier one gave up.
+void launch_couple_points(const StepConsts& c, DevBuffers& b, double* d_pts, uint32_t* d_err, int np, double dt,
+                          double drag, double soft_density, cudaStream_t s, CouplePointsScratch& scratch);
 
 // couple.cu: FluidWorld::couple_heat against a heat grid of nx*ny*nz cells
 // (x fastest), origin and cell size.  The scratch arena (size from
