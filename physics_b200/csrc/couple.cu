@@ -102,6 +102,10 @@ constexpr int kWB = 32 * kPer;  // candidates per chunk of a warp
 constexpr int kPB = 4096;       // candidates a point may have for a list
 constexpr int kTabU = 56;       // u32 per point table: in, total, beg[27], cnt[27]
 
+// Polls of a wait without any point finished before it gives up: ~25 s, where
+// a point over the 2^27 particles that a world can hold would take 15 s.
+constexpr int kWalkPolls = 1 << 27;
+
 // The walk's words: the ticket, then a done flag per point.
 constexpr int kFlowHead = 1;
 
@@ -365,8 +369,9 @@ __device__ __forceinline__ void walk_held(const StepConsts& c, const CoupleArgs&
 
 // The walk over the nb points of a batch.  Warps take points by ticket, in
 // order, so the points a warp waits for are held by running warps (or done)
-// and the wait ends; it gives up after a poll limit all the same, with the
-// error word set and the remaining points (of later batches too) unwalked.
+// and the wait ends; it gives up after a poll limit (counted anew whenever a
+// point is finished, so a long chain of heavy points does not reach it) all
+// the same, with the error word set and the remaining points (of later batches too) unwalked.
 __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, CoupleArgs a, int nb, PointLists L) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ WarpTable s_tab[kFW];
@@ -391,11 +396,17 @@ __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, C
       const int4 p = L.key[j];
       const bool overlap = p.w && abs(p.x - own.x) <= 2 && abs(p.y - own.y) <= 2 && abs(p.z - own.z) <= 2;
       if (!overlap) continue;
-      uint32_t seen = 0;
-      for (int polls = 0; polls < (1 << 22); ++polls) {
+      uint32_t seen = 0, taken = 0;
+      for (int polls = 0; polls < kWalkPolls; ++polls) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(done + j) : "memory");
         if (seen) break;
-        if ((polls & 255) == 255 && *(volatile uint32_t*)a.err) break;
+        if ((polls & 255) == 255) {
+          if (*(volatile uint32_t*)a.err) break;
+          // A ticket was taken: some point was finished, so the walk goes on.
+          const uint32_t t = *(volatile uint32_t*)L.flow;
+          if (t != taken) polls = 0;
+          taken = t;
+        }
       }
       ok = ok && seen != 0u;
     }
