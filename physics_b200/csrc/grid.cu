@@ -542,6 +542,12 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(
 // memory, except in cells of kOrderTile < count <= kOrderLarge particles,
 // which go to `large` for k_order_large (the thread of the cell's first slot
 // appends it).  Particles of the overflow cell keep their slots.
+//
+// Many sparse tiles (more than two per CTA, under 16 particles each) are taken
+// eight at a time, one per warp, where they hold at most 32 particles: a CTA
+// spends ~2 us on a tile however few there are (70,000 particles in as many
+// tiles: the one-launch sort 180 us with CTAs alone, 141 as separate kernels,
+// whose CTAs are twice as many).
 constexpr int kTileCache = 4;                         // particles per thread held in registers
 constexpr int kTileOrder = kTileCache * kThreads;     // 1024
 template <int kCells>
@@ -565,7 +571,7 @@ __device__ __forceinline__ void tile_cells(
   int& s_small = stage.small;
   const uint32_t count = *num_tiles;
   const int lane = threadIdx.x & 31;
-  for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) {
+  auto cta_tile = [&](uint32_t k) {
     const uint32_t t = tile_of[k];
     const uint32_t ts = tstart[t], te = tstart[t + 1];
     const uint32_t cell0 = t * (uint32_t)kCells;
@@ -689,6 +695,57 @@ __device__ __forceinline__ void tile_cells(
       }
     }
     __syncthreads();  // the counters and keys are free for the next tile
+  };
+  // One warp: tile k with at most 32 particles, a lane each; false otherwise.
+  auto warp_tile = [&](uint32_t k) {
+    const uint32_t t = tile_of[k];
+    const uint32_t ts = tstart[t], te = tstart[t + 1], cnt = te - ts;
+    if (cnt > 32u) return false;
+    const uint32_t cell0 = t * (uint32_t)kCells;
+    uint32_t i = 0, cl = 0xffffffffu;
+    unsigned long long mine = 0;
+    if ((uint32_t)lane < cnt) {
+      i = tmp[ts + lane];
+      cl = cell_of[i] - cell0;
+      mine = okey[i];
+    }
+    uint32_t r = 0, less0 = 0, less1 = 0;
+    bool head = (uint32_t)lane < cnt;
+    for (uint32_t j = 0; j < cnt; ++j) {
+      const uint32_t cj = __shfl_sync(0xffffffffu, cl, j);
+      const unsigned long long kj = __shfl_sync(0xffffffffu, mine, j);
+      r += cj < cl || (cj == cl && kj < mine) ? 1u : 0u;
+      less0 += cj < (uint32_t)lane ? 1u : 0u;
+      less1 += cj < (uint32_t)lane + 32u ? 1u : 0u;
+      head = head && !(cj == cl && j < (uint32_t)lane);
+    }
+    const uint32_t occ = (uint32_t)__popc(__ballot_sync(0xffffffffu, head));
+    if (lane < kCells) cell_start[cell0 + lane] = ts + less0;
+    if (kCells > 32) cell_start[cell0 + lane + 32] = ts + less1;
+    if (lane == 0) {
+      cell_start[cell0 + kCells] = te;
+      tile_slot[k] = ts;
+      tile_crowd[k] = cnt > (uint32_t)dense_mean * occ ? 1 : 0;
+    }
+    if ((uint32_t)lane < cnt) place(ts + r, i);
+    return true;
+  };
+  if (count > 2u * gridDim.x && (uint32_t)n < 16u * count) {
+    constexpr uint32_t kWarps = kThreads / 32;
+    __shared__ uint32_t s_left[kWarps];
+    const uint32_t warp = threadIdx.x >> 5;
+    for (uint32_t k0 = blockIdx.x; k0 < count; k0 += kWarps * gridDim.x) {
+      const uint32_t k = k0 + warp * gridDim.x;
+      const bool left = k < count && !warp_tile(k);  // uniform in the warp
+      if (lane == 0) s_left[warp] = left ? 1u << warp : 0u;
+      __syncthreads();
+      uint32_t todo = 0;  // the warps' tiles that need the whole CTA
+      for (uint32_t q = 0; q < kWarps; ++q) todo |= s_left[q];
+      __syncthreads();
+      for (; todo; todo &= todo - 1u) cta_tile(k0 + (uint32_t)(__ffs(todo) - 1) * gridDim.x);
+    }
+  } else {
+    for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) cta_tile(k);
   }
   const uint32_t of = cell_start[ncells];
   for (uint32_t e = of + blockIdx.x * blockDim.x + threadIdx.x; e < (uint32_t)n; e += gridDim.x * blockDim.x) {
