@@ -931,12 +931,20 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
 // of filtering again, which gives the same pairs in the same order; a task
 // whose reservation did not fit filters as before.
 
-// A task runs in two halves (every other chunk), which are work items of
-// their own: the warp that finishes a task second adds the halves' sums (half
-// 0 + half 1, so the result does not depend on which that is), and no warp
-// waits.  A whole task in cells of 160 takes one warp ~100 us, and a world of
-// 100,000 has barely more tasks than the GPU has warps.  The sums pass through
-// the queries' unused list rows.
+// A task is summed in two halves (every other chunk), which in small worlds are
+// work items of their own: the warp that finishes a task second adds the
+// halves' sums (half 0 + half 1, so the result does not depend on which that
+// is), and no warp waits.  A whole task in cells of 160 takes one warp ~100 us,
+// and a world of 100,000 has barely more tasks than the GPU has warps.  The
+// sums pass through the queries' unused list rows.  In worlds of kWholeFrom
+// particles and more, where tasks are plentiful, one warp takes both halves
+// (kWhole), with the same sums: a second item per task costs its start and the
+// join.  (us of the density and force passes by halves and whole: sheets of
+// 120,000 at 100 per cell 97 + 189 and 100 + 213, 300,000 at 40 149 + 278 and
+// 136 + 264, 1,000,000 at 100 588 + 1,320 and 568 + 1,310, at 1,000 3,147 +
+// 7,967 and 3,264 + 8,173; 256 collapsed scenes of 12 million 7,120 + 16,120
+// and 6,710 + 15,850, where one chain per task took 6,590 + 15,750.)
+constexpr int kWholeFrom = 200000;
 constexpr int kWT = 256;  // threads per dense-task CTA
 constexpr int kHalfWords = 17;  // floats of a half's sums in a list row
 static_assert(2 * kHalfWords * sizeof(float) <= kMaxNeighbors * sizeof(uint16_t), "both halves fit a list row");
@@ -1011,22 +1019,22 @@ __device__ __forceinline__ CellGeom cell_geom(const StepConsts& c, const TiledAr
 // 27 neighbour ranges held by lanes 0..26 (empty when the neighbour cell's
 // box is out of reach of the queries' box).
 struct DenseTask {
-  uint32_t k, half;  // task and which of its halves
+  uint32_t k, half;  // task and which of its halves (0 for a warp with both)
   uint32_t q0, qn;
   CellGeom cg;
   uint32_t nb_s, nb_e;  // this lane's neighbour range (lane < 27)
 };
 
-template <int TB>
+template <int TB, bool kWhole>
 __device__ __forceinline__ bool next_task(const StepConsts& c, const TiledArgs& a, uint32_t* counter,
                                           uint32_t ntasks, DenseTask& t) {
   const int lane = threadIdx.x & 31;
   uint32_t k = 0;
   if (lane == 0) k = atomicAdd(counter, 1u);
   k = __shfl_sync(0xffffffffu, k, 0);
-  if (k >= 2u * ntasks) return false;
-  t.half = k & 1u;
-  k >>= 1;
+  t.half = kWhole ? 0u : k & 1u;
+  if (!kWhole) k >>= 1;
+  if (k >= ntasks) return false;
   t.k = k;
   t.q0 = a.dense_q0[k];
   const uint32_t cell = a.sorted_cell[t.q0];
@@ -1093,10 +1101,11 @@ __device__ __forceinline__ void neighbour_offset(const StepConsts& c, int nb, fl
 // Density of the dense-cell particles: per query the compensated sum of
 // m_j poly6(r) over the 27 cells (world.rs:219-238), candidates in pairs on
 // f32x2 arithmetic (the filter of the tiled pass without the list).
-template <int TB, bool kCount, bool kExact>
+template <int TB, bool kCount, bool kExact, bool kWhole>
 __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArgs a) {
   after_previous();
   __shared__ __align__(16) float s_pp[kWarps][32 * 4];  // 32 candidates, pair-interleaved
+  __shared__ float2 s_sum[kWhole ? kWarps : 1][2][32];  // both halves' sums
   const int lane = threadIdx.x & 31;
   float* sp = s_pp[threadIdx.x >> 5];
   const float4* sp4 = reinterpret_cast<const float4*>(sp);
@@ -1105,7 +1114,7 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
   const f2 HC2 = f2_pack(hc2, hc2), H0SQ = f2_pack(c.h0sqf, c.h0sqf);
   unsigned cand = 0, pairs = 0;
   DenseTask t;
-  while (next_task<TB>(c, a, a.dense_taken, ntasks, t)) {
+  while (next_task<TB, kWhole>(c, a, a.dense_taken, ntasks, t)) {
     const bool qv = (uint32_t)lane < t.qn;
     const uint32_t qi = t.q0 + (uint32_t)lane;
     const float4 q = qv ? a.cpos[qi] : make_float4(kFar, kFar, kFar, 0.f);
@@ -1114,25 +1123,35 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
     const f2 PX = f2_pack(q.x, q.x), PY = f2_pack(q.y, q.y), PZ = f2_pack(q.z, q.z);
     // Mask entries: reserve the task's upper bound (one entry per chunk of
     // every neighbour cell in reach).
-    uint32_t mbase = kNoMasks, mcount = 0;
+    uint32_t mbase = kNoMasks, mcount = 0, bound0 = 0;
     if (a.mask_ctl) {
       const uint32_t chunks = __reduce_add_sync(0xffffffffu, (t.nb_e - t.nb_s + 31u) >> 5);
-      const uint32_t bound = (chunks + 1u - t.half) >> 1;  // this half's
+      bound0 = (chunks + 1u) >> 1;
+      const uint32_t bound = kWhole ? chunks : (chunks + 1u - t.half) >> 1;  // this half's
       unsigned long long base = 0;
       if (lane == 0) base = atomicAdd(a.mask_ctl, (unsigned long long)bound);
       base = __shfl_sync(0xffffffffu, base, 0);
-      if (base + bound <= a.mask_cap) mbase = (uint32_t)base;
+      if (base + bound <= a.mask_cap && (!kWhole || bound0 <= 0xffffu)) mbase = (uint32_t)base;
     }
     float s = 0.f, comp = 0.f;
+    // A warp with both halves keeps their sums in shared memory (in registers,
+    // exchanged at every chunk, they cost 3%), and counts the second one's
+    // entries in the upper bits (a task of more than 131,070 chunks keeps none).
+    uint32_t half = 1u, counts = 0;
+    if (kWhole) s_sum[threadIdx.x >> 5][0][lane] = s_sum[threadIdx.x >> 5][1][lane] = make_float2(0.f, 0.f);
     uint32_t skip = t.half;  // chunks of the other half before this half's next
     for (int nb = 0; nb < 27; ++nb) {
       const uint32_t s0 = __shfl_sync(0xffffffffu, t.nb_s, nb), e0 = __shfl_sync(0xffffffffu, t.nb_e, nb);
       if (s0 >= e0) continue;
       float off[3];
       neighbour_offset(c, nb, off);
-      uint32_t cb = s0 + 32u * skip;
-      skip ^= ((e0 - s0 + 31u) >> 5) & 1u;
-      for (; cb < e0; cb += 64) {
+      uint32_t cb = s0;
+      if (!kWhole) {
+        cb += 32u * skip;
+        skip ^= ((e0 - s0 + 31u) >> 5) & 1u;
+      }
+      for (; cb < e0; cb += kWhole ? 32 : 64) {
+        if (kWhole) half ^= 1u;
         const uint32_t j = cb + (uint32_t)lane;
         const bool cv = j < e0;
         float4 p = cv ? a.cpos[j] : make_float4(kFar, kFar, kFar, 0.f);
@@ -1177,19 +1196,39 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
         }
         float p0, p1;
         f2_unpack(NPART, p0, p1);
-        kahan_add(s, comp, c.poly6_cf * -(p0 + p1));
+        if (kWhole) {
+          float2 v = s_sum[threadIdx.x >> 5][half][lane];
+          kahan_add(v.x, v.y, c.poly6_cf * -(p0 + p1));
+          s_sum[threadIdx.x >> 5][half][lane] = v;
+        } else {
+          kahan_add(s, comp, c.poly6_cf * -(p0 + p1));
+        }
         if (mbase != kNoMasks) {
           // 2 ceil(m / 2) bits were shifted in (at least 2); bit k = candidate k.
           const uint32_t used = (m + 1u) & ~1u;
           const uint32_t bits = qv ? __brev(used < 32u ? mask << (32u - used) : mask) : 0u;
           if (__any_sync(0xffffffffu, bits != 0u)) {
-            a.mask_bits[(size_t)(mbase + mcount) * 32u + (uint32_t)lane] = bits;
-            if (lane == 0) a.mask_hdr[mbase + mcount] = (cb << 5) | (uint32_t)nb;
-            ++mcount;
+            const uint32_t e = mbase + (!kWhole ? mcount : half ? bound0 + (counts >> 16) : counts & 0xffffu);
+            a.mask_bits[(size_t)e * 32u + (uint32_t)lane] = bits;
+            if (lane == 0) a.mask_hdr[e] = (cb << 5) | (uint32_t)nb;
+            if (kWhole) counts += half ? 0x10000u : 1u;
+            else ++mcount;
           }
         }
         __syncwarp();  // the chunk is consumed before the next one is staged
       }
+    }
+    if (kWhole) {
+      if (a.mask_ctl && lane < 2) {
+        a.task_mbase[2u * t.k + (uint32_t)lane] = mbase == kNoMasks ? kNoMasks : mbase + (lane ? bound0 : 0u);
+        a.task_mcount[2u * t.k + (uint32_t)lane] = lane ? counts >> 16 : counts & 0xffffu;
+      }
+      if (qv) {
+        const float2 h = s_sum[threadIdx.x >> 5][0][lane], g = s_sum[threadIdx.x >> 5][1][lane];
+        write_density(c, a, (int)qi, ((double)h.x - (double)h.y) + ((double)g.x - (double)g.y));
+        a.nbr_count[qi] = kNoList;
+      }
+      continue;
     }
     if (a.mask_ctl && lane == 0) {
       a.task_mbase[2u * t.k + t.half] = mbase;
@@ -1225,7 +1264,7 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
 // tiled pass.  The partial sums are folded into the compensated totals every
 // 16 rounds (every 8 with the shear sum, one candidate per round) and at the
 // end of the chunk, uniformly across the warp.
-template <int TB, bool kShear>
+template <int TB, bool kShear, bool kWhole>
 __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs a) {
   after_previous();
   // The entries this step's tasks asked for, for the host's next sizing.
@@ -1236,14 +1275,17 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
   __shared__ float4 s_vel[kWarps][33];
   __shared__ float s_mr[kWarps][33];
   __shared__ __align__(16) float s_pp[kWarps][32 * 4];  // the chunk's positions, pair-interleaved
+  // The first half's sums of a warp with both.
+  __shared__ float s_first[kWhole ? kWarps : 1][kWhole ? kHalfWords : 1][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float* sp = s_pp[w];
   const float4* sp4 = reinterpret_cast<const float4*>(sp);
   const uint32_t ntasks = sort_lost(a) ? 0u : *a.dense_count;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2);
+  constexpr int kSums = kShear ? 17 : 15;
   DenseTask t;
-  while (next_task<TB>(c, a, a.dense_taken + 1, ntasks, t)) {
+  while (next_task<TB, kWhole>(c, a, a.dense_taken + 1, ntasks, t)) {
     const bool qv = (uint32_t)lane < t.qn;
     const uint32_t qi = t.q0 + (uint32_t)lane;
     const float4 qp = qv ? a.cpos[qi] : make_float4(kFar, kFar, kFar, 0.f);
@@ -1296,26 +1338,45 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
         if (rounds & 7) fold<kShear>(acc, part, qp.w * c.spiky_cf, lapm);
       }
     };
+    // The sums so far, put aside at the border by a warp with both halves.
+    auto second_half = [&]() {
+      const float sums[kHalfWords] = {acc.fpx, acc.cpx, acc.fpy, acc.cpy, acc.fpz, acc.cpz, acc.fvx, acc.cvx, acc.fvy,
+                                      acc.cvy, acc.fvz, acc.cvz, acc.xsx, acc.xsy, acc.xsz, acc.shear, acc.csh};
+#pragma unroll
+      for (int k = 0; k < kSums; ++k) s_first[w][k][lane] = sums[k];
+      acc = CompAcc();
+    };
+    // This half's entries, or the first half's and, `gap` further on, the
+    // second's.
     uint32_t mbase = a.task_mbase ? a.task_mbase[2u * t.k + t.half] : kNoMasks;
-    const uint32_t mcount = mbase != kNoMasks ? a.task_mcount[2u * t.k + t.half] : 0u;
-    if (mbase != kNoMasks && ((unsigned long long)mbase + mcount > a.mask_cap || mcount > (1u << 20))) {
+    uint32_t mfirst = mbase != kNoMasks ? a.task_mcount[2u * t.k + t.half] : 0u, mcount = mfirst, gap = 0;
+    bool bad = (unsigned long long)mbase + mfirst > a.mask_cap || mfirst > (1u << 20);
+    if (kWhole && mbase != kNoMasks) {
+      const uint32_t mbase2 = a.task_mbase[2u * t.k + 1u], mcount2 = a.task_mcount[2u * t.k + 1u];
+      bad = bad || (unsigned long long)mbase2 + mcount2 > a.mask_cap || mcount2 > (1u << 20);
+      gap = mbase2 - mbase - mfirst;
+      mcount += mcount2;
+    }
+    if (mbase != kNoMasks && bad) {
       if (lane == 0) atomicOr(a.flags, kFlagMaskTable);
       mbase = kNoMasks;
     }
     if (mbase != kNoMasks) {
+      auto entry = [&](uint32_t e) { return mbase + e + (kWhole && e >= mfirst ? gap : 0u); };
       // The density pass's chunks, in its order; the next entry's header and
       // mask are loaded while the current chunk is walked.
       uint32_t hdr = 0, bits = 0;
       if (mcount) {
-        hdr = a.mask_hdr[mbase];
-        bits = a.mask_bits[(size_t)mbase * 32u + (uint32_t)lane];
+        hdr = a.mask_hdr[entry(0)];
+        bits = a.mask_bits[(size_t)entry(0) * 32u + (uint32_t)lane];
       }
       for (uint32_t e = 0; e < mcount; ++e) {
         const uint32_t h = hdr, mask = bits;
         if (e + 1 < mcount) {
-          hdr = a.mask_hdr[mbase + e + 1];
-          bits = a.mask_bits[(size_t)(mbase + e + 1) * 32u + (uint32_t)lane];
+          hdr = a.mask_hdr[entry(e + 1)];
+          bits = a.mask_bits[(size_t)entry(e + 1) * 32u + (uint32_t)lane];
         }
+        if (kWhole && e == mfirst) second_half();
         // Only candidates some lane has in range are loaded, and the chunk's
         // first (always a particle), which pads the two-candidate rounds as in
         // the filtering walk; the other slots hold far dummies, never walked.
@@ -1333,11 +1394,18 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
         walk(mask);
         __syncwarp();  // the chunk is consumed before the next one is staged
       }
+      if (kWhole && mcount == mfirst) second_half();
     } else {
       const Box3 qb = warp_box(qp.x, qp.y, qp.z, qv);
       task_neighbours<TB>(c, a, t, qb, hc2);
       uint32_t skip = t.half;  // chunks of the other half before this half's next
-      for (int nb = 0; nb < 27; ++nb) {
+      // (Both halves: twice over the cells.)
+      for (int n2 = 0; n2 < (kWhole ? 54 : 27); ++n2) {
+        const int nb = kWhole && n2 >= 27 ? n2 - 27 : n2;
+        if (kWhole && n2 == 27) {
+          second_half();
+          skip = 1u;
+        }
         const uint32_t s0 = __shfl_sync(0xffffffffu, t.nb_s, nb), e0 = __shfl_sync(0xffffffffu, t.nb_e, nb);
         if (s0 >= e0) continue;
         float off[3];
@@ -1380,16 +1448,16 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
     }
     const float sums[kHalfWords] = {acc.fpx, acc.cpx, acc.fpy, acc.cpy, acc.fpz, acc.cpz, acc.fvx, acc.cvx, acc.fvy,
                                     acc.cvy, acc.fvz, acc.cvz, acc.xsx, acc.xsy, acc.xsz, acc.shear, acc.csh};
-    if (qv) {
+    if (!kWhole && qv) {
 #pragma unroll
-      for (int k = 0; k < (kShear ? 17 : 15); ++k) *half_sum(a, t, t.half, k) = sums[k];
+      for (int k = 0; k < kSums; ++k) *half_sum(a, t, t.half, k) = sums[k];
     }
-    if (finishes_task(a, t.k, 1) && qv) {
+    if ((kWhole || finishes_task(a, t.k, 1)) && qv) {
       float v[kHalfWords], o[kHalfWords];
 #pragma unroll
       for (int k = 0; k < kHalfWords; ++k) {
-        v[k] = k < (kShear ? 17 : 15) ? __ldcg(half_sum(a, t, 0, k)) : 0.f;
-        o[k] = k < (kShear ? 17 : 15) ? __ldcg(half_sum(a, t, 1, k)) : 0.f;
+        v[k] = k >= kSums ? 0.f : kWhole ? s_first[w][k][lane] : __ldcg(half_sum(a, t, 0, k));
+        o[k] = k >= kSums ? 0.f : kWhole ? sums[k] : __ldcg(half_sum(a, t, 1, k));
       }
 #pragma unroll
       for (int k = 0; k < 17; k += 2) {
@@ -1439,8 +1507,8 @@ const Occupancy& occupancy() {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_density_tiled<4, false, true>, kTT, kDensitySmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, k_force_tiled<4, true>, kTT, kForceSmem);
     int dd = 0, df = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dd, k_density_dense<4, false, true>, kWT, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&df, k_force_dense<4, true>, kWT, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dd, k_density_dense<4, false, true, false>, kWT, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&df, k_force_dense<4, true, false>, kWT, 0);
     r.dense_density = std::max(dd, 1);
     r.dense_force = std::max(df, 1);
     r.sms = std::max(r.sms, 1);
@@ -1449,6 +1517,22 @@ const Occupancy& occupancy() {
     return r;
   }();
   return o;
+}
+
+// The dense-cell passes for tile edge TB; kWhole: a warp takes both halves of a
+// task.
+template <int TB, bool kWhole>
+void launch_dense(const StepConsts& c, const TiledArgs& a, cudaStream_t s, bool force, bool exact, int blocks) {
+  const bool overlap = c.n < kOverlapBelow;
+  if (!force) {
+    auto f = a.counters
+                 ? (exact ? k_density_dense<TB, true, true, kWhole> : k_density_dense<TB, true, false, kWhole>)
+                 : (exact ? k_density_dense<TB, false, true, kWhole> : k_density_dense<TB, false, false, kWhole>);
+    launch_after(overlap, f, blocks, kWT, 0, s, c, a);
+  } else {
+    launch_after(overlap, c.shear_live ? k_force_dense<TB, true, kWhole> : k_force_dense<TB, false, kWhole>, blocks,
+                 kWT, 0, s, c, a);
+  }
 }
 
 // The four passes of a tiled step (staged and dense-cell density, staged and
@@ -1460,12 +1544,11 @@ void launch_passes(const StepConsts& c, const TiledArgs& a, cudaStream_t s, cons
   auto density = a.counters ? (exact ? k_density_tiled<TB, true, true> : k_density_tiled<TB, true, false>)
                             : (exact ? k_density_tiled<TB, false, true> : k_density_tiled<TB, false, false>);
   launch_after(overlap, density, density_blocks, kTT, kDensitySmem, s, c, a);
-  auto dense = a.counters ? (exact ? k_density_dense<TB, true, true> : k_density_dense<TB, true, false>)
-                          : (exact ? k_density_dense<TB, false, true> : k_density_dense<TB, false, false>);
-  launch_after(overlap, dense, dense_d_blocks, kWT, 0, s, c, a);
+  auto dense = c.n >= kWholeFrom ? launch_dense<TB, true> : launch_dense<TB, false>;
+  dense(c, a, s, false, exact, dense_d_blocks);
   if (ev.after_density) cudaEventRecord(ev.after_density, s);
   launch_after(overlap, c.shear_live ? k_force_tiled<TB, true> : k_force_tiled<TB, false>, force_blocks, kTT, kForceSmem, s, c, a);
-  launch_after(overlap, c.shear_live ? k_force_dense<TB, true> : k_force_dense<TB, false>, dense_f_blocks, kWT, 0, s, c, a);
+  dense(c, a, s, true, exact, dense_f_blocks);
 }
 
 }  // namespace
