@@ -360,7 +360,7 @@ int32_t phy_fluid_autotune_horizon(PhyWorldHandle *w, uint32_t sub, double dt, u
  * reverse sweep over all recorded steps, re-running each segment forward
  * from its checkpoint (the f64 plain step repeats bit-exactly; the first
  * steps of an f64 tape, up to 512 MiB of them, are recorded as they run and
- * not run again): given
+ * not run again, unless device memory runs out): given
  * dL/dpos_T and dL/dvel_T (3n doubles each, insertion order, xyz
  * interleaved; NULL = zero) it writes dL/dpos_0, dL/dvel_0 (3n each) and
  * grad_params2 = {dL/d stiffness, dL/d visc_k[0]} (any output may be NULL).
@@ -372,7 +372,10 @@ int32_t phy_fluid_autotune_horizon(PhyWorldHandle *w, uint32_t sub, double dt, u
  * recorded end state and the tape is kept for further sweeps until
  * phy_fluid_tape_clear or the next phy_fluid_tape_begin.  Particles added
  * after phy_fluid_tape_begin are stepped, but the tape's checkpoints lack
- * them: phy_fluid_step_backward then fails.  The reference has
+ * them: phy_fluid_step_backward then fails.  phy_fluid_tape_clear keeps up to
+ * 1 GiB of device memory for the next tape; it is freed when the world's
+ * particle count changes, when the world runs out of memory, or with the
+ * world.  The reference has
  * no adjoint; these calls replace nothing in phy_ffi.h. */
 int32_t phy_fluid_tape_begin(PhyWorldHandle *w, uint32_t sub, uint32_t checkpoint_every);
 int32_t phy_fluid_tape_clear(PhyWorldHandle *w, uint32_t sub);

@@ -360,17 +360,37 @@ void dfree(T*& p) {
   p = nullptr;
 }
 
+}  // namespace
+
+void cuda_check(cudaError_t e, const char* what) {
+  if (e == cudaSuccess) return;
+  // The error goes to the caller; a non-sticky API error must not stay in the
+  // runtime's last-error slot and fail the next, unrelated call's check.
+  (void)cudaGetLastError();
+  throw CudaError(std::string(what) + ": " + cudaGetErrorString(e), e);
+}
+
+void* FluidWorld::dmalloc(size_t bytes) {
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && release_spare()) {
+    (void)cudaGetLastError();
+    e = cudaMalloc(&p, bytes);
+  }
+  cuda_check(e, "cudaMalloc");
+  return p;
+}
+
 template <class T>
-void dalloc(T*& p, size_t count) {
+void FluidWorld::dalloc(T*& p, size_t count) {
   dfree(p);
-  if (count == 0) count = 1;
-  cuda_check(cudaMalloc((void**)&p, count * sizeof(T)), "cudaMalloc");
+  p = static_cast<T*>(dmalloc(std::max<size_t>(count, 1) * sizeof(T)));
 }
 
 // Makes a device array of at least `need` elements out of one of `cap`; after a
 // failure it has none.
 template <class T, class C>
-void dreserve(T*& p, C& cap, size_t need) {
+void FluidWorld::dreserve(T*& p, C& cap, size_t need) {
   if (p && (size_t)cap >= need) return;
   cap = 0;
   dalloc(p, need);
@@ -379,9 +399,8 @@ void dreserve(T*& p, C& cap, size_t need) {
 
 // Grows a device array to `cap` elements, keeping the first `keep`.
 template <class T>
-void dgrow(T*& p, size_t keep, size_t cap, cudaStream_t s) {
-  T* q = nullptr;
-  cuda_check(cudaMalloc((void**)&q, std::max<size_t>(cap, 1) * sizeof(T)), "cudaMalloc");
+void FluidWorld::dgrow(T*& p, size_t keep, size_t cap, cudaStream_t s) {
+  T* q = static_cast<T*>(dmalloc(std::max<size_t>(cap, 1) * sizeof(T)));
   if (p && keep) cuda_check(cudaMemcpyAsync(q, p, keep * sizeof(T), cudaMemcpyDeviceToDevice, s), "grow copy");
   if (p) {
     cuda_check(cudaStreamSynchronize(s), "grow sync");
@@ -390,14 +409,32 @@ void dgrow(T*& p, size_t keep, size_t cap, cudaStream_t s) {
   p = q;
 }
 
-}  // namespace
-
-void cuda_check(cudaError_t e, const char* what) {
-  if (e == cudaSuccess) return;
-  // The error goes to the caller; a non-sticky API error must not stay in the
-  // runtime's last-error slot and fail the next, unrelated call's check.
-  (void)cudaGetLastError();
-  throw CudaError(std::string(what) + ": " + cudaGetErrorString(e));
+// Gives up what the adjoint could do without; false when that is nothing.
+// (The vectors keep their sizes: a caller may hold one of their elements.)
+bool FluidWorld::release_spare() {
+  if (spare_busy_) return false;
+  bool any = adj_work_ != nullptr;
+  dfree(adj_work_);
+  adj_work_n_ = 0;
+  for (size_t k = 0; k < adj_slot_f_.size(); ++k) {
+    any = any || adj_slot_f_[k] || adj_slot_u_[k];
+    dfree(adj_slot_f_[k]);
+    dfree(adj_slot_u_[k]);
+    adj_slot_ucount_[k] = 0;
+  }
+  tape_.direct = -1;
+  if (tape_.on) return any;
+  for (auto& p : tape_.ckpt) {
+    any = any || p;
+    dfree(p);
+  }
+  for (int q = 0; q < kSnapSlots; ++q)
+    if (snap_count_[q] == 0) {
+      any = any || snap_arena_[q];
+      dfree(snap_arena_[q]);
+      snap_bytes_[q] = 0;
+    }
+  return any;
 }
 
 // ---- SphParams -------------------------------------------------------------
@@ -2026,7 +2063,8 @@ static constexpr size_t kAdjWorkArrays = kAdjRec + 4 * 3 + 4 + 4;
 // Ends the tape.  Its buffers stay for the next tape of the same size while
 // they are small (an optimisation loop clears and begins a tape every
 // iteration; allocating and freeing them took two thirds of it at 65,536
-// particles); they go with the world or when its particle count changes.
+// particles); they go with the world, when its particle count changes, or
+// where memory runs out for the world (release_spare).
 void FluidWorld::tape_clear() {
   constexpr size_t kKeepBytes = size_t(1) << 30;
   tape_.nckpt = 0;
@@ -2089,8 +2127,13 @@ void FluidWorld::tape_begin(int every) {
   tape_.lost = false;
   tape_.every = every;
   tape_.params = params.to_c();
-  save_checkpoint();
   tape_.on = true;
+  try {
+    save_checkpoint();
+  } catch (...) {
+    tape_.on = false;
+    throw;
+  }
 }
 
 namespace {
@@ -2170,14 +2213,17 @@ bool FluidWorld::direct_slot(const StepConsts& c) {
   if (prec_ != Precision::F64Plain || tape_.direct != (int)tape_.dts.size() - 1) return false;
   const size_t slot = 22 * n_ * sizeof(double) + tape_ucount(c) * sizeof(uint32_t);
   if ((size_t)(tape_.direct + 1) * slot > kDirectBytes) return false;
+  spare_busy_ = true;
+  bool ok = true;
   try {
     ensure_adj_work();
     ensure_slot(c, tape_.direct);
   } catch (const std::exception&) {
     (void)cudaGetLastError();
-    return false;
+    ok = false;
   }
-  return true;
+  spare_busy_ = false;
+  return ok;
 }
 
 // Copies the step just enqueued (constants c) to slot `si`.
@@ -2224,7 +2270,28 @@ AdjTape FluidWorld::record_step(const StepConsts& c, int si, uint32_t* slot_of) 
   return v;
 }
 
+// The sweep, again without the steps recorded as they ran where memory runs
+// out beside them.
 void FluidWorld::step_backward(const double* gx, const double* gv, double* gx0, double* gv0, double* gparams) {
+  spare_busy_ = true;
+  try {
+    try {
+      sweep(gx, gv, gx0, gv0, gparams);
+    } catch (const CudaError& e) {
+      if (e.code != cudaErrorMemoryAllocation || tape_.direct <= 0) throw;
+      spare_busy_ = false;
+      release_spare();
+      spare_busy_ = true;
+      sweep(gx, gv, gx0, gv0, gparams);
+    }
+  } catch (...) {
+    spare_busy_ = false;
+    throw;
+  }
+  spare_busy_ = false;
+}
+
+void FluidWorld::sweep(const double* gx, const double* gv, double* gx0, double* gv0, double* gparams) {
   const size_t n = n_;
   const int T = (int)tape_.dts.size();
   if (!tape_.on) throw std::invalid_argument("step_backward: no adjoint tape (call tape_begin before stepping)");

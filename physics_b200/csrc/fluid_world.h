@@ -45,7 +45,8 @@ enum class Precision : int { F64Plain = 0, F32Comp = 1 };
 
 class CudaError : public std::runtime_error {
  public:
-  using std::runtime_error::runtime_error;
+  CudaError(const std::string& what, cudaError_t e) : std::runtime_error(what), code(e) {}
+  cudaError_t code;
 };
 
 void cuda_check(cudaError_t e, const char* what);
@@ -212,6 +213,18 @@ class FluidWorld {
   StepConsts make_consts(double dt) const;
 
  private:
+  // Device memory for this world.  An allocation that fails is tried again
+  // after the adjoint's spare buffers were given up: steps recorded as they
+  // ran, which a sweep can re-run, and what tape_clear kept.
+  void* dmalloc(size_t bytes);
+  template <class T>
+  void dalloc(T*& p, size_t count);
+  template <class T, class C>
+  void dreserve(T*& p, C& cap, size_t need);
+  template <class T>
+  void dgrow(T*& p, size_t keep, size_t cap, cudaStream_t s);
+  bool release_spare();
+  bool spare_busy_ = false;  // the spare buffers are being made or used
   void ensure_capacity(size_t n);
   void ensure_mode_buffers();
   bool mode_ready_ = true;  // the buffers of ensure_mode_buffers are those of the capacity
@@ -322,6 +335,7 @@ class FluidWorld {
     PhySphParams params;
   } tape_;
   void tape_free();
+  void sweep(const double* gx, const double* gv, double* gx0, double* gv0, double* gparams);
   void ensure_slot(const StepConsts& c, int si);
   void ensure_adj_work();
   void set_tape_outputs(bool on);

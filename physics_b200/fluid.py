@@ -416,6 +416,8 @@ class FluidWorld:
         L.check(self._lib.phy_fluid_tape_begin(self._h, self._sub, checkpoint_every), "phy_fluid_tape_begin")
 
     def tape_clear(self) -> None:
+        """Ends the tape (phy_fluid_tape_clear), keeping up to 1 GiB of its device memory for the
+        next one until the particle count changes or the world goes."""
         L.check(self._lib.phy_fluid_tape_clear(self._h, self._sub), "phy_fluid_tape_clear")
 
     @property

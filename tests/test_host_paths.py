@@ -190,3 +190,47 @@ def test_a_lost_sort_is_reported_once_at_the_next_wait(fake):
     w.tape_begin(2)
     w.step(DT, 3)
     w.step_backward(np.ones((64, 3)), None)
+
+
+def _tape_world(n=4000):
+    return _world(n=n), (22 * 8 + 99 * 4) * n, 48 * n  # one recorded step, one checkpoint
+
+
+def test_recorded_steps_make_room_for_checkpoints(fake):
+    """Steps recorded as they run fill the device; the checkpoints that the sweep cannot do
+    without still find room, as they did while nothing was recorded."""
+    w, slot, ckpt = _tape_world()
+    w.step(DT)
+    fake.fake_set_budget(int(fake.fake_live() + 4 * slot + 8 * ckpt))
+    w.tape_begin(1)
+    w.step(DT, 30)
+    assert fake.fake_refused() > 0
+    fake.fake_set_budget(1 << 40)
+    w.step_backward(np.ones((4000, 3)), None)
+
+
+def test_recorded_steps_make_room_for_the_sweep(fake):
+    w, slot, ckpt = _tape_world()
+    w.step(DT)
+    fake.fake_set_budget(int(fake.fake_live() + 6.5 * slot))
+    w.tape_begin(4)
+    w.step(DT, 16)
+    recorded = fake.fake_launches(b"k_tape_copy")
+    w.step_backward(np.ones((4000, 3)), None)
+    assert 0 < recorded < 16 and fake.fake_launches(b"k_tape_copy") >= recorded + 16
+
+
+def test_a_cleared_tape_makes_room_for_the_world(fake):
+    w, slot, ckpt = _tape_world()
+    w.step(DT)
+    before = fake.fake_live()
+    w.tape_begin(5)
+    w.step(DT, 10)
+    w.step_backward(np.ones((4000, 3)), None)
+    w.tape_clear()
+    kept = fake.fake_live() - before
+    assert kept > 8 * slot
+    fake.fake_set_budget(fake.fake_live())
+    w.set(pb.FIELD_BODY_ACC, np.ones((4000, 3)))
+    assert fake.fake_live() < before + kept // 2
+    fake.fake_set_budget(1 << 40)
