@@ -8,6 +8,7 @@
 #include <cstring>
 #include <climits>
 #include <limits>
+#include <mutex>
 
 namespace phy {
 
@@ -502,6 +503,66 @@ SphParams SphParams::from_c(const PhySphParams& c) {
   return p;
 }
 
+// Mapped host memory for the worlds' words.  Page-locking memory takes up to
+// milliseconds, so worlds share pages of 64 slots; a page that empties is given
+// back unless it is the last empty one.  Not freed at exit: the runtime may be
+// gone by then.
+namespace {
+
+struct HostPage {
+  unsigned char* base;
+  uint64_t used;  // bit per slot
+};
+constexpr size_t kHostSlot = 128;
+struct HostPages {
+  std::mutex lock;
+  std::vector<HostPage> pages;
+};
+HostPages& host_pages() {
+  static HostPages* p = new HostPages;
+  return *p;
+}
+
+void* take_host_slot() {
+  HostPages& h = host_pages();
+  std::lock_guard<std::mutex> l(h.lock);
+  HostPage* page = nullptr;
+  for (auto& p : h.pages)
+    if (~p.used) page = &p;
+  if (!page) {
+    HostPage p{nullptr, 0};
+    cuda_check(cudaMallocHost((void**)&p.base, 64 * kHostSlot), "cudaMallocHost");
+    h.pages.push_back(p);
+    page = &h.pages.back();
+  }
+  int k = 0;
+  while ((page->used >> k) & 1u) ++k;
+  page->used |= uint64_t(1) << k;
+  std::memset(page->base + k * kHostSlot, 0, kHostSlot);
+  return page->base + k * kHostSlot;
+}
+
+void give_host_slot(void* slot) {
+  HostPages& h = host_pages();
+  std::lock_guard<std::mutex> l(h.lock);
+  size_t empty = 0, at = 0;
+  for (size_t q = 0; q < h.pages.size(); ++q) {
+    HostPage& p = h.pages[q];
+    const size_t off = (size_t)(static_cast<unsigned char*>(slot) - p.base);
+    if (slot >= p.base && off < 64 * kHostSlot) p.used &= ~(uint64_t(1) << (off / kHostSlot));
+    if (p.used == 0) {
+      ++empty;
+      at = q;
+    }
+  }
+  if (empty > 1) {
+    cudaFreeHost(h.pages[at].base);
+    h.pages.erase(h.pages.begin() + (ptrdiff_t)at);
+  }
+}
+
+}  // namespace
+
 // ---- FluidWorld --------------------------------------------------------------
 
 FluidWorld::FluidWorld(const SphParams& p, Precision prec) : params(p), prec_(prec), h0_(p.h) {
@@ -514,8 +575,8 @@ FluidWorld::FluidWorld(const SphParams& p, Precision prec) : params(p), prec_(pr
   b_.flags = reinterpret_cast<uint32_t*>(d_words_);
   b_.order_count = b_.flags + 2;
   b_.counters = reinterpret_cast<unsigned long long*>(d_words_ + 256);
-  cuda_check(cudaMallocHost((void**)&host_, sizeof(HostWords)), "cudaMallocHost");
-  std::memset(host_, 0, sizeof(HostWords));
+  static_assert(sizeof(HostWords) <= kHostSlot, "one slot per world");
+  host_ = static_cast<HostWords*>(take_host_slot());
   b_.sort_lost = &host_->sort_lost;
 }
 
@@ -524,7 +585,7 @@ FluidWorld::~FluidWorld() {
   drop_graphs();
   free_all();
   dfree(d_words_);
-  if (host_) cudaFreeHost(host_);
+  if (host_) give_host_slot(host_);
   dfree(d_couple_);
   couple_scratch_.release();
   dfree(d_heat_);

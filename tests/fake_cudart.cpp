@@ -104,11 +104,12 @@ int fake_launches(const char* part) {
     if (k.first.find(part) != std::string::npos) n += k.second;
   return n;
 }
-// Fills every page-locked allocation's bytes [offset, offset + 4) with `v`.
-void fake_poke_pinned(unsigned long long offset, uint32_t v) {
+// Fills bytes [offset, offset + 4) of every `stride` bytes of page-locked memory with `v`.
+void fake_poke_pinned(unsigned long long offset, unsigned long long stride, uint32_t v) {
   Lock l(g_mu);
   for (auto& p : g_pinned)
-    if (offset + 4 <= p.second) std::memcpy(reinterpret_cast<void*>(p.first + offset), &v, 4);
+    for (size_t at = offset; at + 4 <= p.second; at += stride)
+      std::memcpy(reinterpret_cast<void*>(p.first + at), &v, 4);
 }
 
 // ---- the runtime's side ----

@@ -36,7 +36,7 @@ def fake_library(tmp_path_factory):
         fn.restype, fn.argtypes = res, args
     lib.fake_live.restype = C.c_ulonglong
     lib.fake_set_budget.argtypes = [C.c_ulonglong]
-    lib.fake_poke_pinned.argtypes = [C.c_ulonglong, C.c_uint32]
+    lib.fake_poke_pinned.argtypes = [C.c_ulonglong, C.c_ulonglong, C.c_uint32]
     lib.fake_launches.argtypes = [C.c_char_p]
     return lib
 
@@ -173,17 +173,17 @@ def test_a_lost_sort_is_reported_once_at_the_next_wait(fake):
     w = _world()
     for wait in (w.synchronize, lambda: w.get(pb.FIELD_RHO), lambda: w.pos, lambda: w.total_momentum()):
         w.step(DT)
-        fake.fake_poke_pinned(64, 1)
+        fake.fake_poke_pinned(64, 128, 1)
         with pytest.raises(L.PhyError, match="did not happen"):
             wait()
         wait()
-    fake.fake_poke_pinned(64, 1)
+    fake.fake_poke_pinned(64, 128, 1)
     with pytest.raises(L.PhyError, match="did not happen"):
         w._world.step_checked(DT)
     assert w._world.step_checked(DT) == 0
     w.tape_begin(2)
     w.step(DT, 3)
-    fake.fake_poke_pinned(64, 1)
+    fake.fake_poke_pinned(64, 128, 1)
     for _ in range(2):
         with pytest.raises(L.PhyError, match="did not happen"):
             w.step_backward(np.ones((64, 3)), None)
@@ -234,3 +234,14 @@ def test_a_cleared_tape_makes_room_for_the_world(fake):
     w.set(pb.FIELD_BODY_ACC, np.ones((4000, 3)))
     assert fake.fake_live() < before + kept // 2
     fake.fake_set_budget(1 << 40)
+
+
+def test_worlds_share_page_locked_memory(fake):
+    """64 worlds a page; worlds made and dropped one after another lock no page each."""
+    worlds = [_world() for _ in range(130)]
+    assert fake.fake_pinned_calls() <= 3
+    for w in worlds:
+        w._world.close()
+    for _ in range(5):
+        _world()._world.close()
+    assert fake.fake_pinned_calls() <= 3
