@@ -273,7 +273,8 @@ int32_t phy_fluid_phase_times(PhyWorldHandle *w, uint32_t sub, double *out5, int
  *                         persistent grids (0 = occupancy limit, default);
  *   PHY_TUNE_QUEUE        0 = static tile stride, 1 = device work queue;
  *   PHY_TUNE_SORT_BLOCK   threads per block of the sort's per-particle
- *                         kernels (32..256, default 256);
+ *                         kernels (32..256, default 256; no effect where the
+ *                         sort is one launch, below 80,000 particles);
  *   PHY_TUNE_GRAPH_CHUNK  0 = launch every step (default); k > 0 = capture
  *                         runs of k steps of phy_fluid_step into a CUDA graph
  *                         once and replay it (re-captured when parameters,

@@ -1749,7 +1749,7 @@ double FluidWorld::time_tuning(const LaunchTuning& t, int comp_tile, double dt, 
   return total / nslots;
 }
 
-// Candidates: sort block 128/256, static tile stride or work queue, 1..the
+// Candidates: sort block 128/256 (256 where the sort is one launch), static tile stride or work queue, 1..the
 // occupancy limit of CTAs per SM, and (tiled worlds) 4 or 2 cells per tile
 // edge.  With horizon > 0 the states the run will meet are sampled first:
 // the current state, and the states after horizon/2 and horizon steps of the
@@ -1768,8 +1768,12 @@ std::vector<TuneTrial> FluidWorld::autotune(double dt, int steps, int horizon) {
   const int max_per_sm = tiled ? tiled_max_ctas_per_sm() : 1;
   std::vector<std::pair<LaunchTuning, int>> cands;
   const std::vector<int> tiles = tiled ? std::vector<int>{4, 2} : std::vector<int>{comp_tile_};
-  for (int tile : tiles)
-    for (int sort_block : {128, 256})
+  ensure_cells();
+  for (int tile : tiles) {
+    // (A one-launch sort has blocks of its own: both values time the same step.)
+    const int cells = tiled ? tile * tile * tile : 1;
+    const bool one = sort_in_one_launch((int)n_, ncells_ / cells);
+    for (int sort_block : one ? std::vector<int>{256} : std::vector<int>{128, 256})
       for (int queue = 0; queue <= (tiled ? 1 : 0); ++queue)
         for (int per = 1; per <= max_per_sm; ++per) {
           LaunchTuning t;
@@ -1779,6 +1783,7 @@ std::vector<TuneTrial> FluidWorld::autotune(double dt, int steps, int horizon) {
           t.sort_polls = tuning_.sort_polls;
           cands.push_back({t, tile});
         }
+  }
   const LaunchTuning saved = tuning_;
   const int saved_tile = comp_tile_;
   snapshot(false, 0);

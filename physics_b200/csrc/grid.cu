@@ -1173,6 +1173,8 @@ static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g
                               dim3(kThreads), args, sizeof(LargeStage), s);
 }
 
+bool sort_in_one_launch(int n, int buckets) { return n < kFusedBelow && buckets < kFusedBuckets; }
+
 void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, const LaunchTuning& t) {
   // Per-particle kernels take any warp multiple up to kThreads.
   const int bs = t.sort_block >= 32 && t.sort_block <= kThreads ? t.sort_block / 32 * 32 : kThreads;
@@ -1202,7 +1204,7 @@ void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, const Launc
   g.origin[2] = (double)c.bz0 * c.h0;
   g.bz0 = c.bz0;
   const int buckets = c.tile ? c.ncells >> (3 * c.tile_log2) : c.ncells;
-  if (n < kFusedBelow && buckets < kFusedBuckets) {
+  if (sort_in_one_launch(n, buckets)) {
     if (c.tile == 4)
       launch_fused<64>(c, b, g, t.sort_polls, s);
     else if (c.tile == 2)

@@ -134,6 +134,9 @@ struct DevBuffers {
 // grid.cu
 struct LaunchTuning;
 void launch_sort(const StepConsts& c, DevBuffers& b, cudaStream_t s, const LaunchTuning& t);
+// Whether launch_sort takes one launch (in which LaunchTuning::sort_block means
+// nothing) for n particles in `buckets` cells, or tiles of a tiled world.
+bool sort_in_one_launch(int n, int buckets);
 // The cells of the current positions without moving the state: cell_start
 // over the box and perm[s] = the particle at sorted slot s in (cell,
 // insertion index) order.  c.tile must be 0 (x-major cells).  The

@@ -245,3 +245,14 @@ def test_worlds_share_page_locked_memory(fake):
     for _ in range(5):
         _world()._world.close()
     assert fake.fake_pinned_calls() <= 3
+
+
+@pytest.mark.parametrize("n,blocks", [(2000, {256}), (90000, {128, 256})])
+@pytest.mark.parametrize("form", ["f64", "comp"])
+def test_autotune_tries_the_sort_block_where_it_matters(fake, form, n, blocks):
+    """Below 80,000 particles the sort is one launch without the knob: its values would time the
+    same step twice."""
+    trials = _world(form, n=n).autotune(DT, 1)
+    assert {t["sort_block"] for t in trials} == blocks
+    keys = [(t["comp_tile"], t["queue"], t["ctas_per_sm"], t["sort_block"]) for t in trials]
+    assert len(set(keys)) == len(keys) >= len(blocks)
