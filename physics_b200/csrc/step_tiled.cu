@@ -175,7 +175,9 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* ws, uint32_
 }
 
 // Whether the sort was lost: then no pass of the step writes anything but the
-// kept constants.
+// kept constants.  (The dense-cell passes find no tasks: a second word to wait
+// for before the tasks are counted made the nearer SMs take them all, and
+// their density pass 40% slower in worlds of few tasks.)
 __device__ __forceinline__ bool sort_lost(const TiledArgs& a) { return (a.flags[0] & kFlagSortLost) != 0u; }
 
 // Work items per tile: a world of few tiles splits each into x-slabs (the
@@ -477,6 +479,7 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
   if (sort_lost(a)) {
     for (int i = (int)(blockIdx.x * kTT + threadIdx.x); i < c.n; i += (int)(gridDim.x * kTT))
       keep_particle(a.before, a.now, i);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.dense_count = 0u;
     return;
   }
   const uint32_t ntiles = *a.num_tiles;
@@ -1109,7 +1112,7 @@ __global__ void __launch_bounds__(kWT, 4) k_density_dense(StepConsts c, TiledArg
   const int lane = threadIdx.x & 31;
   float* sp = s_pp[threadIdx.x >> 5];
   const float4* sp4 = reinterpret_cast<const float4*>(sp);
-  const uint32_t ntasks = sort_lost(a) ? 0u : *a.dense_count;
+  const uint32_t ntasks = *a.dense_count;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2), H0SQ = f2_pack(c.h0sqf, c.h0sqf);
   unsigned cand = 0, pairs = 0;
@@ -1268,7 +1271,7 @@ template <int TB, bool kShear, bool kWhole>
 __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs a) {
   after_previous();
   // The entries this step's tasks asked for, for the host's next sizing.
-  if (a.mask_demand && blockIdx.x == 0 && threadIdx.x == 0 && !sort_lost(a)) *a.mask_demand = *a.mask_ctl;
+  if (a.mask_demand && blockIdx.x == 0 && threadIdx.x == 0) *a.mask_demand = *a.mask_ctl;
   // The chunk's 32 candidates, and in slot 32 a weightless copy of its first
   // (mass and m/rho 0) that pads the two-candidate rounds.
   __shared__ float4 s_pos[kWarps][33];
@@ -1280,7 +1283,7 @@ __global__ void __launch_bounds__(kWT, 2) k_force_dense(StepConsts c, TiledArgs 
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float* sp = s_pp[w];
   const float4* sp4 = reinterpret_cast<const float4*>(sp);
-  const uint32_t ntasks = sort_lost(a) ? 0u : *a.dense_count;
+  const uint32_t ntasks = *a.dense_count;
   const float hc2 = fminf(c.h2f, c.h0sqf);
   const f2 HC2 = f2_pack(hc2, hc2);
   constexpr int kSums = kShear ? 17 : 15;
