@@ -188,10 +188,19 @@ __device__ __forceinline__ bool sort_lost(const TiledArgs& a) { return (a.flags[
 // (us of the density and force passes with 1, 2 and 4 parts: 76,800
 // particles in ~250 tiles 46 + 41, 39 + 43, 40 + 40; 147,456 in ~440 60 + 51,
 // 50 + 47, -; 524,288 in ~1,200 119 + 116, 124 + 127, -.)
-constexpr uint32_t kSplit4Below = 150, kSplit2Below = 600;
+// From 222 tiles on, two parts of each no longer run at once (the force pass
+// has 444 CTAs), and tiles are split only where they have 384 queries on
+// average (in one and two parts: 300 tiles of 200 particles 34 + 36 and 33 + 44,
+// 500 of them 41 + 48 and 46 + 61, 480 of 60 23 + 29 and 30 + 38, 480 of 250 46 +
+// 51 and 47 + 48, 512 of 390 62 + 56 and 57 + 55).
+// Parts of one index are dealt before those of the next: dealt tile by tile,
+// CTAs of one parity took all first parts, which in scenes that end inside a
+// tile hold most particles (80,000 in 16 scenes 90 + 220 us, now 97 + 147).
+constexpr uint32_t kSplit4Below = 150, kSplitFew = 222, kSplit2Below = 600, kSplitMean = kTT / 2 * 3;
 template <int TB>
-__device__ __forceinline__ uint32_t tile_parts(uint32_t ntiles) {
-  return ntiles < kSplit4Below ? (uint32_t)TB : (TB == 4 && ntiles < kSplit2Below) ? 2u : 1u;
+__device__ __forceinline__ uint32_t tile_parts(uint32_t ntiles, int n) {
+  if (ntiles < kSplit4Below) return (uint32_t)TB;
+  return TB == 4 && ntiles < kSplit2Below && (ntiles < kSplitFew || (uint32_t)n > ntiles * kSplitMean) ? 2u : 1u;
 }
 
 struct TileGeom {
@@ -484,12 +493,12 @@ __global__ void __launch_bounds__(kTT, 6) k_density_tiled(StepConsts c, TiledArg
   }
   const uint32_t ntiles = *a.num_tiles;
   unsigned cand = 0, pairs = 0;
-  const uint32_t parts = tile_parts<TB>(ntiles);
+  const uint32_t parts = tile_parts<TB>(ntiles, c.n);
   const int layers = T::B / (int)parts;
   for (uint32_t item = next_tile(a.queue, 0, blockIdx.x, &s_next); item < ntiles * parts;
        item = next_tile(a.queue, 0, item + gridDim.x, &s_next)) {
-    const uint32_t k = item / parts;
-    const int xa = (int)(item % parts) * layers;
+    const uint32_t k = item % ntiles;
+    const int xa = (int)(item / ntiles) * layers;
     const TileGeom g = tile_geom<TB>(c, a, k);
     halo_table<TB>(c, a, g, s_src, s_end, s_off, ws);
     const int fit = a.tile_crowd[k] ? 0 : pick_slab<TB>(s_off, (uint32_t)min(c.halo_cap, kHaloCap));
@@ -828,12 +837,12 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
   __shared__ uint32_t s_next;
   if (sort_lost(a)) return;
   const uint32_t ntiles = *a.num_tiles;
-  const uint32_t parts = tile_parts<TB>(ntiles);
+  const uint32_t parts = tile_parts<TB>(ntiles, c.n);
   const int layers = T::B / (int)parts;
   for (uint32_t item = next_tile(a.queue, 1, blockIdx.x, &s_next); item < ntiles * parts;
        item = next_tile(a.queue, 1, item + gridDim.x, &s_next)) {
-    const uint32_t k = item / parts;
-    const int xa = (int)(item % parts) * layers;
+    const uint32_t k = item % ntiles;
+    const int xa = (int)(item / ntiles) * layers;
     const TileGeom g = tile_geom<TB>(c, a, k);
     halo_table<TB>(c, a, g, s_src, s_end, s_off, ws);
     const int fit = a.tile_crowd[k] ? 0 : pick_slab<TB>(s_off, (uint32_t)min(c.halo_cap, kHaloCap));

@@ -36,6 +36,43 @@ def test_few_particles_in_a_wide_box(gpu, form, tile, wide, n):
         assert_bits_equal(getattr(a, k), getattr(b, k), k)
 
 
+@pytest.mark.parametrize("dims", [(7, 8, 9), (16, 16, 16), (24, 30, 24)])
+def test_split_of_small_tiles(gpu, dims):
+    """2x2x2 tiles: alone (under 150 and under 600 of them) and beside a scene of thousands."""
+    rng = np.random.default_rng(sum(dims))
+    pos, other = scenes.dam_break_positions(*dims), scenes.dam_break_positions(40, 60, 40)
+    vel = rng.normal(0.0, 0.3, pos.shape)
+    top = 0.2 * max(dims)
+    a = _world(gpu, "comp", 2, top, pos, vel)
+    b = _world(gpu, "comp", 2, top, np.concatenate([pos, other]), np.concatenate([vel, np.zeros_like(other)]))
+    b.set_scenes([len(pos), len(other)], [(0.0,) * 3] * 2, [(top,) * 3, (20.0,) * 3])
+    for w in (a, b):
+        w.step(0.005, 3)
+    for k in FIELDS:
+        assert_bits_equal(getattr(a, k), getattr(b, k)[:len(pos)], k)
+
+
+@pytest.mark.parametrize("ns,per,flat", [(20, 3000, 0.1), (290, 200, 0.05), (290, 500, 1.0)])
+def test_split_of_scenes_that_end_inside_a_tile(gpu, ns, per, flat):
+    """Batches on both sides of the split's rules, the first and the last scene against a world of
+    their own."""
+    rng = np.random.default_rng(ns + per)
+    m = int(np.ceil(per ** (1.0 / 3.0)))
+    i = np.arange(per)
+    one = (np.stack([i // (m * m), (i // m) % m, i % m], axis=1) + 0.5) * [0.1, 0.1 * flat, 0.1]
+    pos = np.concatenate([one + rng.uniform(-0.002, 0.002, one.shape) for _ in range(ns)])
+    vel = rng.normal(0.0, 0.1, pos.shape)
+    both = _world(gpu, "comp", 4, 4.0, pos, vel)
+    both.set_scenes([per] * ns, [(0.0,) * 3] * ns, [(4.0,) * 3] * ns)
+    both.step(0.001, 2)
+    for k in (0, ns - 1):
+        part = slice(k * per, (k + 1) * per)
+        alone = _world(gpu, "comp", 4, 4.0, pos[part], vel[part])
+        alone.step(0.001, 2)
+        for f in FIELDS:
+            assert_bits_equal(getattr(alone, f), getattr(both, f)[part], f)
+
+
 @pytest.mark.parametrize("n", [33, 5000, 70001])
 @pytest.mark.parametrize("shuffled", [False, True])
 def test_one_particle_per_cell(gpu, oracle_mod, n, shuffled):
