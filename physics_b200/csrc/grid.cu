@@ -30,9 +30,10 @@ constexpr int kScanTile = kThreads * kScanItems;  // 4096 cells per scan block
 
 // Particles and buckets below which the sort is one cooperative launch.  The
 // separate kernels take ~40 us up to 100,000 particles (launches), the fused
-// one 22 us at 343, 21 us at 4,275, 32 us at 65,536 and 46 us at 111,777 (its
-// grid of resident blocks moves less at once); tiled, 30 against 41 us at
-// 8,303 and 66 against 59 us at 379,603.
+// one 19 us at 300 and 4,000 and 23 us at 79,000 (with the scan sums contended
+// 46 us at 111,777, where the separate ones were taken); tiled, 27 against 41 us
+// at 8,000, 30 against 43 at 76,800 and 66 against 59 us at 379,603 (its grid of
+// resident blocks moves less at once).
 constexpr int kFusedBelow = 80000;
 constexpr int kFusedBuckets = 1 << 22;
 
@@ -1124,6 +1125,8 @@ void launch_cell_index(const StepConsts& c, DevBuffers& b, uint32_t* flags, cuda
   build_cells(c, b, s, kThreads, nullptr, flags);
 }
 
+constexpr int kSms = 148;
+
 // Blocks of the fused sort: resident, at most four per SM (the barrier takes
 // 1.3 us with 35 blocks and 1.6 us with 296).  Per device: the shared-memory
 // limit belongs to the device's context, and the grid to its size.
@@ -1168,9 +1171,14 @@ static void launch_fused(const StepConsts& c, DevBuffers& b, const GatherArgs& g
   a.out = b.sorted_cell;
   a.tile_crowd = b.tile_crowd;
   a.g = g;
-  // Enough blocks for the particles and the scanned entries, at most the resident ones
-  // (all of those when tiled: crowded cells are ordered a block each).
-  const int want = c.tile ? INT_MAX : std::max(grid_for(c.n), (int)(a.len / kScanTile));
+  // Enough blocks for the particles, the scanned entries and, up to one per SM,
+  // sparse tiles (a block each), at most the resident ones.  Not all of those:
+  // a cooperative launch starts when all its blocks fit, so worlds on streams
+  // of their own would wait for each other (a round of 16 worlds of 10,000
+  // particles 591 -> 239 us, of 70,000 1,101 -> 774; one world 72 -> 66 and 93 ->
+  // 91).
+  int want = std::max(grid_for(c.n), (int)(a.len / kScanTile));
+  if (c.tile) want = std::max(want, std::min({(int)a.h.buckets, c.n / 8, kSms}));
   StepConsts cc = c;
   void* args[] = {&cc, &a};
   cudaLaunchCooperativeKernel((const void*)k_sort_fused<kCells>, dim3((unsigned)std::min(want, fused_blocks<kCells>())),

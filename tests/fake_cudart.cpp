@@ -20,6 +20,7 @@ namespace {
 std::recursive_mutex g_mu;
 std::map<uintptr_t, size_t> g_dev, g_pinned;  // base -> bytes
 size_t g_live = 0, g_budget = SIZE_MAX;
+unsigned g_coop_blocks = 0;  // of the last cooperative launch
 int g_refused = 0, g_violations = 0, g_device = 0, g_pinned_calls = 0, g_dev_calls = 0;
 std::map<const void*, std::string> g_name;
 std::map<std::string, int> g_launches;
@@ -96,6 +97,7 @@ int fake_refused() { return g_refused; }
 int fake_violations() { return g_violations; }
 int fake_pinned_calls() { return g_pinned_calls; }
 int fake_device_calls() { return g_dev_calls; }
+unsigned fake_cooperative_blocks() { return g_coop_blocks; }
 void fake_set_device(int d) { g_device = d; }
 int fake_launches(const char* part) {
   Lock l(g_mu);
@@ -135,7 +137,8 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
   return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launch(f, smem); }
-cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) {
+cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 grid, dim3, void**, size_t smem, cudaStream_t) {
+  g_coop_blocks = grid.x;
   return launch(f, smem);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {

@@ -256,3 +256,13 @@ def test_autotune_tries_the_sort_block_where_it_matters(fake, form, n, blocks):
     assert {t["sort_block"] for t in trials} == blocks
     keys = [(t["comp_tile"], t["queue"], t["ctas_per_sm"], t["sort_block"]) for t in trials]
     assert len(set(keys)) == len(keys) >= len(blocks)
+
+
+@pytest.mark.parametrize("form", ["f64", "comp"])
+@pytest.mark.parametrize("n", [1, 300, 2000, 10000, 70000])
+def test_the_one_launch_sort_leaves_room_for_other_worlds(fake, form, n):
+    """A cooperative launch starts when all its blocks fit: one per 256 particles, or per SM where
+    sparse tiles need them, not every one that the GPU (296 here) holds."""
+    w = _world(form, n=n)
+    w.step(DT)
+    assert 1 <= fake.fake_cooperative_blocks() <= max(148, (n + 255) // 256)
