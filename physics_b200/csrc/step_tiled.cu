@@ -189,14 +189,15 @@ __device__ __forceinline__ bool sort_lost(const TiledArgs& a) { return (a.flags[
 // particles in ~250 tiles 46 + 41, 39 + 43, 40 + 40; 147,456 in ~440 60 + 51,
 // 50 + 47, -; 524,288 in ~1,200 119 + 116, 124 + 127, -.)
 // From 222 tiles on, two parts of each no longer run at once (the force pass
-// has 444 CTAs), and tiles are split only where they have 384 queries on
-// average (in one and two parts: 300 tiles of 200 particles 34 + 36 and 33 + 44,
-// 500 of them 41 + 48 and 46 + 61, 480 of 60 23 + 29 and 30 + 38, 480 of 250 46 +
-// 51 and 47 + 48, 512 of 390 62 + 56 and 57 + 55).
+// has 444 CTAs), and tiles are split only where they have about as many queries
+// on average as a CTA has threads (in one and two parts: 480 tiles of 60
+// particles 23 + 29 and 30 + 38, 300 of 200 34 + 36 and 33 + 44, 500 of 200 41 +
+// 48 and 46 + 61; 225 of 311 55 + 54 and 43 + 54, 343 of 290 48 + 40 and 42 + 43, 512
+// of 390 62 + 56 and 57 + 55).
 // Parts of one index are dealt before those of the next: dealt tile by tile,
 // CTAs of one parity took all first parts, which in scenes that end inside a
 // tile hold most particles (80,000 in 16 scenes 90 + 220 us, now 97 + 147).
-constexpr uint32_t kSplit4Below = 150, kSplitFew = 222, kSplit2Below = 600, kSplitMean = kTT / 2 * 3;
+constexpr uint32_t kSplit4Below = 150, kSplitFew = 222, kSplit2Below = 600, kSplitMean = kTT / 8 * 7;
 template <int TB>
 __device__ __forceinline__ uint32_t tile_parts(uint32_t ntiles, int n) {
   if (ntiles < kSplit4Below) return (uint32_t)TB;
