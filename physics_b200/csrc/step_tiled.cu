@@ -951,13 +951,17 @@ __global__ void __launch_bounds__(kTT, 3) k_force_tiled(StepConsts c, TiledArgs 
 // and a world of 100,000 has barely more tasks than the GPU has warps.  The
 // sums pass through the queries' unused list rows.  In worlds of kWholeFrom
 // particles and more, where tasks are plentiful, one warp takes both halves
-// (kWhole), with the same sums: a second item per task costs its start and the
-// join.  (us of the density and force passes by halves and whole: sheets of
-// 120,000 at 100 per cell 97 + 189 and 100 + 213, 300,000 at 40 149 + 278 and
-// 136 + 264, 1,000,000 at 100 588 + 1,320 and 568 + 1,310, at 1,000 3,147 +
-// 7,967 and 3,264 + 8,173; 256 collapsed scenes of 12 million 7,120 + 16,120
-// and 6,710 + 15,850, where one chain per task took 6,590 + 15,750.)
+// (kWhole), with the same sums, while tasks are short: a second item per task
+// costs its start and the join, and a warp with both adds to two sums by turns.
+// Long tasks are those of a step that reserved kLongTasks mask entries per
+// particle (the last one that the host knows of; ~150 particles per cell).  (us
+// of the density and force passes by halves and whole: sheets of 120,000 at 100
+// per cell 97 + 189 and 100 + 213; 1,000,000 at 50 421 + 878 and 388 + 852, at 160 832
+// + 1,887 and 838 + 1,919, at 1,000 3,100 + 7,802 and 3,309 + 8,133; 256 scenes of 12
+// million at 130 7,638 + 17,901 and 7,422 + 17,849, where one chain per task took
+// 7,144 + 17,537.)
 constexpr int kWholeFrom = 200000;
+constexpr double kLongTasks = 1.5;
 constexpr int kWT = 256;  // threads per dense-task CTA
 constexpr int kHalfWords = 17;  // floats of a half's sums in a list row
 static_assert(2 * kHalfWords * sizeof(float) <= kMaxNeighbors * sizeof(uint16_t), "both halves fit a list row");
@@ -1557,7 +1561,9 @@ void launch_passes(const StepConsts& c, const TiledArgs& a, cudaStream_t s, cons
   auto density = a.counters ? (exact ? k_density_tiled<TB, true, true> : k_density_tiled<TB, true, false>)
                             : (exact ? k_density_tiled<TB, false, true> : k_density_tiled<TB, false, false>);
   launch_after(overlap, density, density_blocks, kTT, kDensitySmem, s, c, a);
-  auto dense = c.n >= kWholeFrom ? launch_dense<TB, true> : launch_dense<TB, false>;
+  const bool is_long =
+      a.mask_demand && (double)*(const volatile unsigned long long*)a.mask_demand >= kLongTasks * (double)c.n;
+  auto dense = c.n >= kWholeFrom && !is_long ? launch_dense<TB, true> : launch_dense<TB, false>;
   dense(c, a, s, false, exact, dense_d_blocks);
   if (ev.after_density) cudaEventRecord(ev.after_density, s);
   launch_after(overlap, c.shear_live ? k_force_tiled<TB, true> : k_force_tiled<TB, false>, force_blocks, kTT, kForceSmem, s, c, a);

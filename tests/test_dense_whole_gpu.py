@@ -101,3 +101,24 @@ def test_dense_sums_against_the_terms(gpu, n, per_cell, whole):
     acc = ((d * fp[..., None]).sum(1) + (dv * fv[..., None]).sum(1) * mu) / rho[:, None]
     size = ((d.abs() * fp.abs()[..., None]).sum(1) + (dv.abs() * fv[..., None]).sum(1) * mu) / rho[:, None]
     assert ((got["acc"] - acc).abs() <= 1e-5 * size + 1e-9).all()
+
+
+def test_long_tasks_of_a_large_world(gpu):
+    """300 particles per cell: whole tasks until the reservations are known, halves from then on."""
+    n = 200003
+    rng = np.random.default_rng(n)
+    pos, top = _sheet(rng, n, 300)
+    vel = rng.normal(0.0, 0.1, pos.shape)
+    w = gpu.FluidWorld(_params(gpu, top, 1), "comp")
+    w.add_particles(pos, scenes.lattice_mass(0.1), vel=vel)
+    outs = []
+    for start in range(3):
+        if start:
+            w.set(gpu.FIELD_POS, pos)
+            w.set(gpu.FIELD_VEL, vel)
+        w.step(0.001)
+        outs.append({k: getattr(w, k).copy() for k in FIELDS})
+        assert w.dense_mask_info()["demand"] > 1.5 * n
+    for o in outs[1:]:
+        for k in FIELDS:
+            assert_bits_equal(o[k], outs[0][k], k)
