@@ -972,6 +972,23 @@ void FluidWorld::ensure_cells() {
   }
 }
 
+// A new world's cell tables, with the load of its first particles: mapping the
+// block that they take, 0.3 ms, is then not the first step's.  (Tables of large
+// boxes are left to the step, as scenes of their own may still replace the box;
+// so is an allocation that fails, which the step tries again and reports.)
+void FluidWorld::first_cells() {
+  constexpr long double kSmallBox = 1 << 21;
+  if (b_.cell_capacity > 0 || !box_valid_) return;
+  long double cells = 1;
+  for (int a = 0; a < 3; ++a) cells *= (long double)(kmax_[a] - kmin_[a] + 3);
+  if (cells > kSmallBox) return;
+  try {
+    ensure_cells();
+  } catch (const std::exception&) {
+    (void)cudaGetLastError();
+  }
+}
+
 StepConsts FluidWorld::make_consts(double dt) const {
   StepConsts c;
   std::memset(&c, 0, sizeof(c));
@@ -1114,6 +1131,7 @@ void FluidWorld::add_particles(size_t m, const double* pos, const double* vel, c
   n_ += m;
   // The staging vector must outlive the copy.
   cuda_check(cudaStreamSynchronize(stream_), "append sync");
+  first_cells();
 }
 
 // Loads a caller's device particles (set_particles_device) in one pass: the
@@ -1182,6 +1200,7 @@ void FluidWorld::set_particles_device(size_t m, const double* pos, const double*
   // The positions may widen the grid box (a failure leaves the world empty).
   merge_box(host_->box, host_->box + 3, host_->box[6] != 0);
   n_ = m;
+  first_cells();
 }
 
 void FluidWorld::get_field_device(int field, double* out) {
@@ -1749,9 +1768,9 @@ double FluidWorld::time_tuning(const LaunchTuning& t, int comp_tile, double dt, 
   return total / nslots;
 }
 
-// Candidates: sort block 128/256 (256 where the sort is one launch), static tile stride or work queue, 1..the
-// occupancy limit of CTAs per SM, and (tiled worlds) 4 or 2 cells per tile
-// edge.  With horizon > 0 the states the run will meet are sampled first:
+// Candidates: sort block 128/256 (256 where the sort is one launch), static
+// tile stride or work queue, 1..the occupancy limit of CTAs per SM, and (tiled
+// worlds) 4 or 2 cells per tile edge.  With horizon > 0 the states the run will meet are sampled first:
 // the current state, and the states after horizon/2 and horizon steps of the
 // current configuration.  Every candidate runs `steps` steps from the first
 // sample; the kKeep fastest then also run from the other samples, and the

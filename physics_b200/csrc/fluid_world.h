@@ -230,6 +230,7 @@ class FluidWorld {
   bool mode_ready_ = true;  // the buffers of ensure_mode_buffers are those of the capacity
   void ensure_masks();
   void ensure_cells();
+  void first_cells();
   void grow_box_with_bounds();
   void grow_box_with_positions(size_t n, const double* pos3);
   void merge_box(const long long* mn, const long long* mx, bool any_nonfinite);

@@ -266,3 +266,11 @@ def test_the_one_launch_sort_leaves_room_for_other_worlds(fake, form, n):
     w = _world(form, n=n)
     w.step(DT)
     assert 1 <= fake.fake_cooperative_blocks() <= max(148, (n + 255) // 256)
+
+
+@pytest.mark.parametrize("form", ["f64", "comp"])
+def test_the_first_step_of_a_loaded_world_allocates_nothing(fake, form):
+    w = _world(form, n=64000)
+    calls = fake.fake_device_calls()
+    w.step(DT)
+    assert fake.fake_device_calls() == calls
