@@ -286,9 +286,10 @@ int32_t phy_fluid_phase_times(PhyWorldHandle *w, uint32_t sub, double *out5, int
  *                         the candidates again.
  *   PHY_TUNE_SORT_POLLS   polls after which a grid barrier of the one-launch
  *                         sort (small worlds) gives up (default 2^22, seconds);
- *                         that step does not happen, and the next call that
- *                         waits for the world fails once (0: every such step,
- *                         for tests of the caller's handling).
+ *                         that step does not happen, and the next readback,
+ *                         synchronisation, checked step or adjoint sweep of
+ *                         the world fails once (0: every such step, for tests
+ *                         of the caller's handling).
  * phy_fluid_get_tuning reads the same parameters. */
 enum {
   PHY_TUNE_COMP_TILE = 0,

@@ -371,7 +371,8 @@ __device__ __forceinline__ void walk_held(const StepConsts& c, const CoupleArgs&
 // order, so the points a warp waits for are held by running warps (or done)
 // and the wait ends; it gives up after a poll limit (counted anew whenever a
 // point is finished, so a long chain of heavy points does not reach it) all
-// the same, with the error word set and the remaining points (of later batches too) unwalked.
+// the same, with the error word set and the remaining points (of later batches
+// too) unwalked.
 __global__ void __launch_bounds__(kFW * 32) k_couple_points_flow(StepConsts c, CoupleArgs a, int nb, PointLists L) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ WarpTable s_tab[kFW];

@@ -1770,9 +1770,9 @@ double FluidWorld::time_tuning(const LaunchTuning& t, int comp_tile, double dt, 
 
 // Candidates: sort block 128/256 (256 where the sort is one launch), static
 // tile stride or work queue, 1..the occupancy limit of CTAs per SM, and (tiled
-// worlds) 4 or 2 cells per tile edge.  With horizon > 0 the states the run will meet are sampled first:
-// the current state, and the states after horizon/2 and horizon steps of the
-// current configuration.  Every candidate runs `steps` steps from the first
+// worlds) 4 or 2 cells per tile edge.  With horizon > 0 the states the run will
+// meet are sampled first: the current state, and the states after horizon/2 and
+// horizon steps of the current configuration.  Every candidate runs `steps` steps from the first
 // sample; the kKeep fastest then also run from the other samples, and the
 // fastest mean over all samples wins (successive halving keeps the tuning
 // time near one pass over the candidates).  The world returns to its
